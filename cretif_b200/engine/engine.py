@@ -23,6 +23,8 @@ from __future__ import annotations
 
 import array
 import collections
+import contextlib
+import gc
 from typing import Dict, Optional, Sequence, Tuple, Union
 
 import numpy as np
@@ -93,6 +95,22 @@ class _PinnedRing:
         if self.events[i] is None:
             self.events[i] = torch.cuda.Event()
         self.events[i].record()
+
+
+@contextlib.contextmanager
+def capturing(graph, pool, stream):
+    """Capture into ``graph`` on ``stream``, which is current, with the garbage collector held
+    off: an engine that is in a reference cycle holds graphs, and destroying one of them while a
+    capture runs is an unsafe call that ends the capture (``cudaErrorStreamCaptureInvalidated``).
+    """
+    collects = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.graph(graph, pool=pool, stream=stream):
+            yield
+    finally:
+        if collects:
+            gc.enable()
 
 
 def parse_dtype(dtype) -> torch.dtype:
@@ -326,7 +344,7 @@ class Engine:
         cur = torch.cuda.current_stream()
         self._graph_stream.wait_stream(cur)
         with torch.cuda.stream(self._graph_stream):
-            with torch.cuda.graph(graph, pool=self._graph_pool, stream=self._graph_stream):
+            with capturing(graph, self._graph_pool, self._graph_stream):
                 logits = self.model.forward(ctx, self.cache, None if all_rows else want_rows)
         cur.wait_stream(self._graph_stream)
         self._graphs[key] = {"graph": graph, "meta": meta, "logits": logits}

@@ -24,6 +24,7 @@ import torch
 
 from ..csrc import ops
 from ..sampling import Sampler, SamplingParams
+from .engine import capturing
 
 
 @dataclass
@@ -207,7 +208,7 @@ class DecodeRunner:
                 if states is not None:
                     cache.restore_states(slots, states)
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, pool=self.pool, stream=self.stream):
+                with capturing(g, self.pool, self.stream):
                     self._body(b, B, context)
             cur.wait_stream(self.stream)
             b["ints"].copy_(saved)
