@@ -257,6 +257,14 @@ int cretif_gemm_tc_qkv_rope(const void* A, const void* Wqkv, void* Q, int ldq, c
                             int write_cache, int M, int K, int lda, int ldw, unsigned int* fault,
                             void* stream);
 
+// The 32-bit path's attention for heads of 64 (attn_f32.cu): float rows and caches, without a bias
+// by distance or pooled entries.  rows: 0 every sequence brings one token, 1 each brings eight or
+// more, 2 a mixture.
+int cretif_attn_f32(const float* q, int ldq, float* out, int ldo, const float* kc, const float* vc,
+                    const int* table, int table_stride, const int* tok_pos, const int* tok_seq,
+                    const int* seq_slot, int nh, int nkv, int hd, float scale, int window, int bt,
+                    int T, const float* sink, const float* slope, int rows, void* stream);
+
 // Causal grouped-query attention over the block cache, any step shape.  sink (may be null):
 // one float per query head, exp(sink) joins the softmax's denominator without a key or value.
 // vd: size of a value head (the cache's values are [blocks, nkv, bt, vd], out rows nh * vd).

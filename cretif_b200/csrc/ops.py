@@ -1273,7 +1273,7 @@ def moe_combine(rows, place, top: int, y, wts=None, identity=None, plus=None, ad
 # ------------------------------------------------------------------ attention
 def attn_simt(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv: int, hd: int,
               scale: float, window: int, block_tokens: int, sink=None, vd: int = 0, bias=None,
-              bias_edges=None, slope=None, pool=None) -> None:
+              bias_edges=None, slope=None, pool=None, news=None) -> None:
     """``window`` > 0: a sliding window of that many keys; < 0: chunks of ``-window`` positions
     counted from 0, a query sees the keys of its own chunk; 0: every earlier key.  ``slope``
     (float32 [heads], optional): the key n positions back has ``slope[h] * n`` taken off its
@@ -1282,7 +1282,10 @@ def attn_simt(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv: i
     (float32 [rows, heads]) with ``bias_edges`` (int32 [rows], ascending from 0): the key n
     positions back adds ``bias[r, h]`` to its scaled score, r the last row with edge <= n.  ``pool``
     (a PoolView; with a sliding window): the entries whose last token lies ``window`` or more
-    positions back join the softmax, without bias or slope."""
+    positions back join the softmax, without bias or slope.  ``news``: how many tokens each
+    sequence of the step brings, where the caller knows; 32-bit heads of 64 channels then take the
+    faster kernels of attn_f32.cu (a prompt's rows share their keys' reads there, which single
+    tokens of many sequences cannot)."""
     _need(q, "q", dim=2); _need(out, "out", q.dtype, 2)
     _need(kc, "k cache", q.dtype, 4); _need(vc, "v cache", q.dtype, 4)
     T = q.shape[0]
@@ -1313,6 +1316,17 @@ def attn_simt(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv: i
         if slope.numel() != nh or not slope.is_contiguous():
             raise KernelError("attention: the slope has one number per query head")
     _need_window_pool(pool, kc, vc, window)
+    if (news and q.dtype == torch.float32 and hd == vd == block_tokens == 64 and bias is None and pool is None
+            and kc.shape[0] * nkv * 64 < 2 ** 31
+            and T and not (q.stride(0) % 4 or out.stride(0) % 4 or nh > 65535
+                           or (q.data_ptr() | out.data_ptr() | kc.data_ptr() | vc.data_ptr()) % 16)):
+        rows = 0 if max(news) == 1 else 1 if min(news) >= 8 else 2
+        _check(lib().cretif_attn_f32(
+            _p(q), _rows(q, "q"), _p(out), _rows(out, "out"), _p(kc), _p(vc), _p(table),
+            table.stride(0), _p(tok_pos), _p(tok_seq), _p(seq_slot), nh, nkv, hd,
+            ctypes.c_float(scale), window, block_tokens, T, _p(sink), _p(slope), rows, _stream()),
+            "attn_f32", 2 if rows == 2 else 1)
+        return
     _check(lib().cretif_attn_simt_pooled(
         _p(q), _rows(q, "q"), _p(out), _rows(out, "out"), _dt(q), _p(kc), _p(vc), _p(table),
         table.stride(0), _p(tok_pos), _p(tok_seq), _p(seq_slot), nh, nkv, hd,

@@ -174,7 +174,8 @@ def run_attention(q, o, ctx, kv, nh, nkv, hd, scale, window, dtype, sink=None, v
             return
     ops.attn_simt(q, o, kv.k, kv.v, kv.table, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot,
                   nh, nkv, hd, scale, window, kv.block_tokens, sink=sink, vd=vd, bias=bias,
-                  bias_edges=bias_edges, slope=slope, pool=pool)
+                  bias_edges=bias_edges, slope=slope, pool=pool,
+                  news=None if _force_plain else (1,) if ctx.is_decode else ctx.seq_new_host)
 
 
 @register_part("mixer", "attention")
