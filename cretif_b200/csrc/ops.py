@@ -34,6 +34,7 @@ def lib():
     if _lib is None:
         L = load_library()
         L.cretif_uniform01.restype = ctypes.c_float
+        L.cretif_delta_chunk_row.restype = ctypes.c_longlong
         L.cretif_uniform01.argtypes = [ctypes.c_ulonglong, ctypes.c_longlong, ctypes.c_int]
         _lib = L
     return _lib
@@ -392,11 +393,37 @@ def delta_conv_state(proj, conv_state, taps: int, C: int, cu_seqlens, seq_slot, 
         taps, C, _p(cu_seqlens), _p(seq_slot), B, _stream()), "delta_conv_state")
 
 
+# The delta rules take chunks of tokens (delta_chunk.cu) from this many tokens of a step's longest
+# sequence on (48 tokens: 26 us token by token and 19 in chunks at 9 heads of 64, 43 and 39 for the
+# general rule at 16 of 128) ...
+DELTA_CHUNKS_FROM = 64
+# ... and, for heads of 64, up to this many heads in flight (sequences of the longest's length
+# times heads): beyond, the walk fills the chip as well and has no workspace to write and read
+# (9 heads of 64 by 256 tokens, walk and chunks: 16 sequences 122 and 100 us, 32 161 and 170, 64
+# 261 and 329).
+DELTA_CHUNKS_HEADS64 = 256
+
+
+def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: bool, state, rows):
+    """The workspace of a step whose delta rule goes in chunks, or None where it walks token by
+    token: few tokens, or sizes and strides that the chunk kernels' 16-byte accesses do not take."""
+    if longest < DELTA_CHUNKS_FROM or (d == 64 and T * H > DELTA_CHUNKS_HEADS64 * longest):
+        return None
+    if any(r.stride(0) % 4 or r.data_ptr() % 16 for r in rows):
+        return None
+    row = int(lib().cretif_delta_chunk_row(H, d, e, int(general)))
+    if not row or state.stride(0) % 4 or state.data_ptr() % 16 or H > 65535:
+        return None
+    return torch.empty(T * row, dtype=torch.float32, device=state.device)
+
+
 def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G: int, d: int,
-                     e: int, norm_w, eps: float, out, write_state: bool = True) -> None:
+                     e: int, norm_w, eps: float, out, write_state: bool = True,
+                     longest: int = 0) -> None:
     """The recurrence over the step's tokens of every (sequence, head), from and to ``state``
     (view [slots, H·d·e] float32), then the per-head RMS norm times ``norm_w`` times
-    SiLU(``gate``) → ``out`` [T, H·e]."""
+    SiLU(``gate``) → ``out`` [T, H·e].  ``longest``: the most tokens a sequence brings (0: not
+    known), by which the step goes token by token or in chunks."""
     _need(prep, "prep", torch.float32, 2); _need(gate, "gate", torch.float32, 2)
     _need(state, "state", torch.float32, 2); _need(out, "out", dim=2)
     _need(norm_w, "norm_w", torch.float32, 1)
@@ -404,6 +431,13 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
         raise KernelError("delta_recurrence: the state's sizes do not fit")
     T = prep.shape[0]
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=prep.device)
+    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,))
+    if ws is not None:
+        _check(lib().cretif_delta_chunks(
+            _p(prep), _rows(prep, "prep"), _p(state), ctypes.c_longlong(state.stride(0)),
+            _p(cu_seqlens), _p(seq_slot), B, H, G, d, e, _p(ws), _p(o_raw), int(write_state), T,
+            _stream()), "delta_chunks", kernels=2)
+        return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
     _check(lib().cretif_delta_recurrence(
         _p(prep), _rows(prep, "prep"), _p(gate), _rows(gate, "gate"), _p(state),
         ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, G, d, e,
@@ -979,10 +1013,11 @@ def general_delta_prepare(proj, prep, a_bias, z, w0, H: int, d: int, e: int, uni
 
 def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, d: int,
                              e: int, norm_w, eps: float, out, per_head_weight: bool = True,
-                             gate_sigmoid: bool = True, write_state: bool = True) -> None:
+                             gate_sigmoid: bool = True, write_state: bool = True,
+                             longest: int = 0) -> None:
     """The generalized delta rule over the step's tokens of every (sequence, head), from and to
     ``state`` (view [slots, H·d·e] float32), then the per-head RMS norm times ``norm_w`` times
-    the gate -> ``out`` [T, H·e]."""
+    the gate -> ``out`` [T, H·e].  ``longest``: see ``delta_recurrence``."""
     _need(proj, "proj", torch.float32, 2); _need(prep, "prep", torch.float32, 2)
     _need(gate, "gate", torch.float32, 2); _need(state, "state", torch.float32, 2)
     _need(out, "out", dim=2); _need(norm_w, "norm_w", torch.float32, 1)
@@ -991,6 +1026,13 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
             or out.shape[1] < H * e or norm_w.numel() != (H * e if per_head_weight else e)):
         raise KernelError("general_delta_recurrence: sizes do not fit")
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=proj.device)
+    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep))
+    if ws is not None:
+        _check(lib().cretif_general_delta_chunks(
+            _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(state),
+            ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, d, e, _p(ws),
+            _p(o_raw), int(write_state), T, _stream()), "general_delta_chunks", kernels=2)
+        return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
     _check(lib().cretif_general_delta_recurrence(
         _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(gate),
         _rows(gate, "gate"), _p(state), ctypes.c_longlong(state.stride(0)), _p(cu_seqlens),

@@ -91,13 +91,15 @@ class GatedDeltaRule(Part):
         proj = linear(x, self.w_in, out_dtype=torch.float32)          # [T, C + H e + 2 H]
         matrices = cache.state[:, :self.matrix_floats]
         inputs = cache.state[:, self.matrix_floats:]
-        prep = torch.empty((T, C + 2 * H), dtype=torch.float32, device=x.device)
+        # rows of whole 16 bytes, whatever the number of heads
+        prep = torch.empty((T, -(-(C + 2 * H) // 4) * 4), dtype=torch.float32,
+                           device=x.device)[:, :C + 2 * H]
         ops.delta_prepare(proj, prep, self.conv_w, inputs, self.a_log, self.dt_bias, ctx.tok_pos,
                           ctx.tok_seq, ctx.seq_slot, ctx.seq_start, H, G, d, e, self.unit_eps)
         out = torch.empty((T, H * e), dtype=self.dtype, device=x.device)
         ops.delta_recurrence(prep, proj[:, C:C + H * e], matrices, ctx.cu_seqlens, ctx.seq_slot,
                              ctx.B, H, G, d, e, self.norm_w, self.eps, out,
-                             write_state=cache.writes)
+                             write_state=cache.writes, longest=ctx.max_new)
         if cache.writes:
             ops.delta_conv_state(proj, inputs, self.taps, C, ctx.cu_seqlens, ctx.seq_slot, ctx.B)
         return linear(out, self.w_o, out_dtype=torch.float32)
@@ -198,7 +200,8 @@ class GeneralDeltaRule(Part):
         gate = proj[:, 2 * H * d + H * e:2 * H * d + 2 * H * e]
         ops.general_delta_recurrence(proj, prep, gate, cache.state, ctx.cu_seqlens, ctx.seq_slot,
                                      ctx.B, H, d, e, self.norm_w, self.eps, out,
-                                     per_head_weight=True, gate_sigmoid=True, write_state=True)
+                                     per_head_weight=True, gate_sigmoid=True, write_state=True,
+                                     longest=ctx.max_new)
         return linear(out, self.w_o, out_dtype=torch.float32)
 
     def weight_bytes(self):

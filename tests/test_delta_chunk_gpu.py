@@ -1,0 +1,128 @@
+"""The delta rules in chunks of 32 tokens against the token-by-token formula in 64 bits, at the
+edges of a chunk, beside the kernels that walk token by token."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [(1, 31, 32, 33, 0, 95), (200,), (64, 2, 129)]
+
+
+def _gated(prep, state, lens, slots, H, G, d, e):
+    """[T, H e] read-outs and the new states, in float64."""
+    P, M = prep.double(), state.double().clone()
+    out, at = [], 0
+    for n, slot in zip(lens, slots):
+        S = M[slot].view(H, d, e)
+        for t in range(at, at + n):
+            q = P[t, :G * d].view(G, d).repeat_interleave(H // G, 0)
+            k = P[t, G * d:2 * G * d].view(G, d).repeat_interleave(H // G, 0)
+            v = P[t, 2 * G * d:2 * G * d + H * e].view(H, e)
+            beta, g = P[t, -2 * H:-H], P[t, -H:]
+            S.mul_(g[:, None, None])
+            u = beta[:, None] * (v - torch.einsum("hde,hd->he", S, k))
+            S.add_(torch.einsum("hd,he->hde", k, u))
+            out.append(torch.einsum("hde,hd->he", S, q).reshape(-1))
+        at += n
+    return torch.stack(out), M
+
+
+def _general(proj, prep, state, lens, slots, H, d, e):
+    P, Q, M = proj.double(), prep.double(), state.double().clone()
+    out, at = [], 0
+    for n, slot in zip(lens, slots):
+        S = M[slot].view(H, d, e)
+        for t in range(at, at + n):
+            r, k = P[t, :H * d].view(H, d), P[t, H * d:2 * H * d].view(H, d)
+            v = P[t, 2 * H * d:2 * H * d + H * e].view(H, e)
+            u, nb, w = (Q[t, i * H * d:(i + 1) * H * d].view(H, d) for i in range(3))
+            x = torch.einsum("hde,hd->he", S, u)
+            S.mul_(w[..., None]).add_(torch.einsum("hd,he->hde", nb, x)
+                                      + torch.einsum("hd,he->hde", k, v))
+            out.append(torch.einsum("hde,hd->he", S, r).reshape(-1))
+        at += n
+    return torch.stack(out), M
+
+
+def _off(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("lens", LENGTHS)
+@pytest.mark.parametrize("general,H,G,d,e", [(False, 4, 2, 64, 16), (False, 2, 2, 128, 48),
+                                             (False, 40, 8, 64, 128), (True, 2, 2, 64, 48),
+                                             (True, 3, 3, 128, 16), (True, 40, 40, 64, 64)])
+def test_chunks_against_the_formula(general, H, G, d, e, lens):
+    """Both ways are 32-bit sums of the same terms: the chunks' result may be no further from the
+    64-bit one than 1e-6 (16 times 2^-24), and than four times the walk's.  Some decays are 0 or
+    tiny (a quotient of cumulated decays would not survive them)."""
+    from cretif_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    T, B = sum(lens), len(lens)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+
+    def unit(x, heads, width):
+        x = x.view(T, heads, width)
+        return (x / x.norm(dim=2, keepdim=True)).reshape(T, heads * width)
+    decays = torch.rand(T, H * d if general else H, generator=gen, device="cuda") * 0.5 + 0.5
+    decays[5::7] = 0.999
+    decays[11::23] = 1e-30
+    decays[17::29] = 0.0
+    slots = list(range(B, 0, -1))
+    state = torch.randn(B + 2, H * d * e, generator=gen, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    seq_slot = torch.tensor(slots, **i32)
+    gate, norm_w = rand(T, H * e), torch.ones(e, device="cuda")
+    if general:
+        key = unit(rand(T, H * d), H, d)
+        proj = torch.cat([rand(T, H * d), key, rand(T, H * e)], 1)
+        prep = torch.cat([key, -torch.rand(T, H * d, generator=gen, device="cuda") * key, decays], 1)
+        want, want_state = _general(proj, prep, state, lens, slots, H, d, e)
+    else:
+        beta = torch.rand(T, H, generator=gen, device="cuda")
+        prep = torch.cat([unit(rand(T, G * d), G, d), unit(rand(T, G * d), G, d), rand(T, H * e),
+                          beta, decays], 1)
+        prep = torch.nn.functional.pad(prep, (0, -prep.shape[1] % 4))[:, :prep.shape[1]]
+        want, want_state = _gated(prep, state, lens, slots, H, G, d, e)
+    # the gate and the norm after the recurrence are the same kernel on both ways
+    w64 = want.view(T, H, e)
+    w64 = (w64 / torch.sqrt((w64 * w64).mean(2, keepdim=True) + 1e-5)).reshape(T, H * e)
+    w64 = w64 * (torch.sigmoid(gate.double()) if general else
+                 gate.double() * torch.sigmoid(gate.double()))
+    off = {}
+    for longest in (0, 1 << 20):
+        mine, out = state.clone(), torch.empty(T, H * e, device="cuda")
+        if general:
+            ops.general_delta_recurrence(proj, prep, gate, mine, cu, seq_slot, B, H, d, e, norm_w,
+                                         1e-5, out, per_head_weight=False, longest=longest)
+        else:
+            ops.delta_recurrence(prep, gate, mine, cu, seq_slot, B, H, G, d, e, norm_w, 1e-5, out,
+                                 longest=longest)
+        off[longest] = _off(out, w64), _off(mine, want_state)
+        assert torch.equal(mine[0], state[0]) and torch.equal(mine[B + 1], state[B + 1])
+    for chunks, walk in zip(off[1 << 20], off[0]):
+        assert chunks <= 1e-6 and chunks <= 4 * walk, off
+    frozen, out = state.clone(), torch.empty(T, H * e, device="cuda")
+    if not general:
+        ops.delta_recurrence(prep, gate, frozen, cu, seq_slot, B, H, G, d, e, norm_w, 1e-5, out,
+                             write_state=False, longest=1 << 20)
+        assert torch.equal(frozen, state) and _off(out, w64) <= 1e-6
+
+
+def test_small_or_odd_sizes_walk():
+    from cretif_b200.csrc import ops
+    state = torch.zeros(2, 2 * 64 * 16, device="cuda")
+    prep = torch.zeros(70, 2 * 128, device="cuda")
+    room = ops._delta_chunk_room
+    assert room(70, 70, 2, 64, 16, False, state, (prep,)) is not None
+    assert room(ops.DELTA_CHUNKS_FROM - 1, 70, 2, 64, 16, False, state, (prep,)) is None
+    assert room(70, 70 * 129, 2, 64, 16, False, state, (prep,)) is None
+    assert room(70, 70 * 128, 2, 64, 16, False, state, (prep,)) is not None
+    assert room(70, 70, 2, 64, 24, False, state, (prep,)) is None
+    assert room(70, 70, 2, 96, 16, False, state, (prep,)) is None
+    assert room(70, 70, 2, 64, 16, False, state, (prep[:, 1:],)) is None
+    assert room(70, 70, 2, 64, 16, False, state, (torch.zeros(70, 257, device="cuda"),)) is None
+    assert room(70, 70, 2, 64, 16, False, state[:, 2:], (prep,)) is None
