@@ -55,6 +55,7 @@ __device__ __forceinline__ void run_of(const AttnF32& a, int t, int& lo, int& hi
 
 __global__ void __launch_bounds__(kRowWarps * 32)
 attn_f32_row_kernel(const AttnF32 a, int only_short) {
+  dependent_begin();
   __shared__ float part_acc[kRowWarps][kHd];
   __shared__ float part_m[kRowWarps], part_l[kRowWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -394,7 +395,7 @@ extern "C" int cretif_attn_f32(const float* q, int ldq, float* out, int ldo, con
     if (const int r = launch_status()) return r;
   }
   if (rows != 1) {
-    attn_f32_row_kernel<<<(unsigned)T * nh, kRowWarps * 32, 0, st>>>(a, rows == 2);
+    launch_dependent(attn_f32_row_kernel, (unsigned)T * nh, kRowWarps * 32, 0, st, a, rows == 2);
     return launch_status();
   }
   return kOk;

@@ -189,9 +189,48 @@ enum Variant : int {
 };
 void count_variant(int v);
 
+// A kernel of a step's chain of small launches begins with dependent_begin(): the kernel behind it
+// may be launched (its own beginning, and the weights that it asks for ahead, then run under this
+// one), and nothing of the kernels before it is read before they are done.  Every thread goes
+// through the wait, so that "the kernel before is done" holds for all kernels before that one as
+// well; the embedding is launched plainly, so that nothing starts before the step before has
+// ended.  dependent_wait() alone: the kernel behind may not start early (it reads ahead what this
+// one writes, or would find the SMs taken).
+__device__ __forceinline__ void dependent_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void dependent_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  dependent_wait();
+}
+
 // Whether kernels that support it are launched as programmatic dependents of the kernel
 // before them (decode_fused.cu owns the switch).
 int dependent_launch_enabled();
+
+// Launch a kernel that begins with dependent_begin() or dependent_wait(), as a programmatic
+// dependent of the kernel before it where it has few CTAs (a decode step's).  CTAs that start
+// early go where SMs are free at that moment, several to one of them: for a short kernel that is
+// made up for by the launch and the drain it hides (0.7 us each), for a recurrence's or a
+// streaming product's CTAs it is not (delta_recurrence 5.4 -> 11.2 us, memory_carry 109 -> 140),
+// so those are launched plainly.  The status is the runtime's last error, as after <<< >>>.
+constexpr int kSmCount = 148;             // of a B200
+template <typename... Params, typename... Args>
+inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed =
+      (long long)grid.x * grid.y * grid.z <= kSmCount ? dependent_launch_enabled() : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 
 // Activations of a feed-forward without a gate: 0 relu(z)^2, 1 gelu (tanh form), 2 silu,
 // 3 gelu (the exact form, with the error function).

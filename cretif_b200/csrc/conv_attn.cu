@@ -37,6 +37,7 @@ conv_headnorm_kv_append_kernel(const float* __restrict__ proj, int ldp,
                                const int* __restrict__ table, int table_stride,
                                T* __restrict__ kc, T* __restrict__ vc, int bt, int write_cache,
                                unsigned int* __restrict__ fault) {
+  dependent_wait();
   if (TAPS > 0) taps = TAPS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x;
@@ -145,10 +146,10 @@ extern "C" int cretif_conv_headnorm_kv_append(
   cudaStream_t st = (cudaStream_t)stream;
   const int widest = nkv > 0 && vd > hd ? vd : hd;
 #define CRETIF_CONV_K(TT, NCH, TAPS)                                                            \
-  conv_headnorm_kv_append_kernel<TT, NCH, TAPS><<<grid, kCvWarps * 32, 0, st>>>(                 \
-      proj, ldp, conv_w, taps, conv_state, (size_t)state_stride, tok_pos, tok_seq, seq_slot,     \
-      seq_start, nh, nkv, hd, vd, eps, gain_coef, gain_every, (TT*)q_out, ldq, table,            \
-      table_stride, (TT*)kc, (TT*)vc, bt, write_cache, fault)
+  launch_dependent(conv_headnorm_kv_append_kernel<TT, NCH, TAPS>, grid, kCvWarps * 32, 0, st,     \
+                   proj, ldp, conv_w, taps, conv_state, (size_t)state_stride, tok_pos, tok_seq,   \
+                   seq_slot, seq_start, nh, nkv, hd, vd, eps, gain_coef, gain_every, (TT*)q_out,  \
+                   ldq, table, table_stride, (TT*)kc, (TT*)vc, bt, write_cache, fault)
 #define CRETIF_CONV(TT, NCH)                                                                    \
   do {                                                                                          \
     if (taps == 4) CRETIF_CONV_K(TT, NCH, 4);                                                    \

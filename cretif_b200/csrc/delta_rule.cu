@@ -45,6 +45,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int ldp, float* __restrict_
                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                      const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int H,
                      int G, int d, int e, float unit_eps) {
+  dependent_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x;
   const int unit = blockIdx.y * kPrepWarps + warp;
@@ -102,6 +103,13 @@ __global__ void delta_conv_state_kernel(const float* __restrict__ proj, int ldp,
                                         float* __restrict__ conv_state, size_t state_stride,
                                         int taps, int C, const int* __restrict__ cu_seqlens,
                                         const int* __restrict__ seq_slot) {
+  // Few CTAs let the kernel behind start early (an output product's weights).  With more, the CTAs
+  // of a decode attention that starts early find the SMs taken and run in two waves (four
+  // sequences, 48 CTAs here: 10.5 -> 15.1 us).
+  if (gridDim.x * gridDim.y <= 32)
+    dependent_begin();
+  else
+    dependent_wait();
   const int b = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -132,6 +140,7 @@ delta_recurrence_kernel(const float* __restrict__ prep, int ldp, float* __restri
                         const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
                         int H, int G, int d, int e, int P, int ecols, float* __restrict__ o_raw,
                         int write_state, int vec) {
+  dependent_begin();
   extern __shared__ __align__(16) float sm[];
   // with at most 512 threads a lane also keeps the token's key slice in registers between
   // the two passes over its rows
@@ -284,6 +293,7 @@ __global__ void __launch_bounds__(256)
 delta_out_norm_kernel(const float* __restrict__ o_raw, const float* __restrict__ gate, int ldg,
                       const float* __restrict__ norm_w, float eps, TO* __restrict__ out, int ldo,
                       int H, int e, long long items, int w_stride, int gate_sigmoid) {
+  dependent_begin();
   const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (item >= items) return;
   const int lane = threadIdx.x & 31;
@@ -373,8 +383,8 @@ extern "C" int cretif_delta_conv_state(const float* proj, int ldp, float* conv_s
                                        void* stream) {
   if (B <= 0 || taps <= 1) return kOk;
   if (C <= 0 || ldp < C) return kBadArgument;
-  delta_conv_state_kernel<<<dim3(B, (C + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      proj, ldp, conv_state, (size_t)state_stride, taps, C, cu_seqlens, seq_slot);
+  launch_dependent(delta_conv_state_kernel, dim3(B, (C + 255) / 256), 256, 0, (cudaStream_t)stream,
+                   proj, ldp, conv_state, (size_t)state_stride, taps, C, cu_seqlens, seq_slot);
   return launch_status();
 }
 
@@ -430,11 +440,11 @@ extern "C" int cretif_delta_recurrence(const float* prep, int ldp, const float* 
   const long long items = (long long)T * H;
   const unsigned blocks = (unsigned)((items + 7) / 8);
   if (out_dt == kF32)
-    delta_out_norm_kernel<float><<<blocks, 256, 0, st>>>(o_raw, gate, ldg, norm_w, eps,
-                                                         (float*)out, ldo, H, e, items, 0, 0);
+    launch_dependent(delta_out_norm_kernel<float>, blocks, 256, 0, st, o_raw, gate, ldg, norm_w,
+                     eps, (float*)out, ldo, H, e, items, 0, 0);
   else
-    delta_out_norm_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(
-        o_raw, gate, ldg, norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items, 0, 0);
+    launch_dependent(delta_out_norm_kernel<__nv_bfloat16>, blocks, 256, 0, st, o_raw, gate, ldg,
+                     norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items, 0, 0);
   return launch_status();
 }
 
@@ -450,13 +460,12 @@ extern "C" int cretif_heads_out_norm(const float* o_raw, const float* gate, int 
   const unsigned blocks = (unsigned)((items + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
   if (out_dt == kF32)
-    delta_out_norm_kernel<float><<<blocks, 256, 0, st>>>(o_raw, gate, ldg, norm_w, eps,
-                                                         (float*)out, ldo, H, e, items,
-                                                         per_head_weight ? e : 0, gate_sigmoid);
+    launch_dependent(delta_out_norm_kernel<float>, blocks, 256, 0, st, o_raw, gate, ldg, norm_w,
+                     eps, (float*)out, ldo, H, e, items, per_head_weight ? e : 0, gate_sigmoid);
   else if (out_dt == kBF16)
-    delta_out_norm_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(
-        o_raw, gate, ldg, norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items,
-        per_head_weight ? e : 0, gate_sigmoid);
+    launch_dependent(delta_out_norm_kernel<__nv_bfloat16>, blocks, 256, 0, st, o_raw, gate, ldg,
+                     norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items, per_head_weight ? e : 0,
+                     gate_sigmoid);
   else
     return kBadDType;
   return launch_status();
@@ -493,6 +502,7 @@ general_delta_prepare_kernel(const float* __restrict__ proj, int ldp, float* __r
                              int ldo, const float* __restrict__ a_bias,
                              const float* __restrict__ z, int ldz, const float* __restrict__ w0,
                              int H, int d, int e, float unit_eps, float decay_scale) {
+  dependent_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x;
   const float* row = proj + (size_t)t * ldp;
@@ -533,6 +543,7 @@ general_delta_prepare_kernel(const float* __restrict__ proj, int ldp, float* __r
 template <typename TO>
 __global__ void tanh_cols_kernel(const float* __restrict__ in, int ld, TO* __restrict__ out,
                                  int R, long long total) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const long long t = idx / R;
@@ -548,6 +559,7 @@ general_delta_recurrence_kernel(const float* __restrict__ proj, int ldp,
                                 const int* __restrict__ cu_seqlens,
                                 const int* __restrict__ seq_slot, int H, int d, int e, int P,
                                 int ecols, float* __restrict__ o_raw, int write_state, int vec) {
+  dependent_begin();
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.x, h = blockIdx.y;
   constexpr int kSlice = DREG + 4;               // see delta_recurrence_kernel
@@ -715,8 +727,8 @@ extern "C" int cretif_general_delta_prepare(const float* proj, int ldp, float* p
   if (ldp < 3 * H * d + 2 * H * e || ldo < 3 * H * d || ldz < H * d) return kBadArgument;
   dim3 grid(T, (H + kPrepWarps - 1) / kPrepWarps);
   if (grid.y > 65535) return kBadArgument;
-  general_delta_prepare_kernel<<<grid, kPrepWarps * 32, 0, (cudaStream_t)stream>>>(
-      proj, ldp, prep, ldo, a_bias, z, ldz, w0, H, d, e, unit_eps, decay_scale);
+  launch_dependent(general_delta_prepare_kernel, grid, kPrepWarps * 32, 0, (cudaStream_t)stream,
+                   proj, ldp, prep, ldo, a_bias, z, ldz, w0, H, d, e, unit_eps, decay_scale);
   return launch_status();
 }
 
@@ -728,9 +740,10 @@ extern "C" int cretif_tanh_cols(const float* in, int ld, void* out, int out_dt, 
   const unsigned blocks = (unsigned)((total + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (out_dt == kF32)
-    tanh_cols_kernel<float><<<blocks, 256, 0, st>>>(in, ld, (float*)out, R, total);
+    launch_dependent(tanh_cols_kernel<float>, blocks, 256, 0, st, in, ld, (float*)out, R, total);
   else if (out_dt == kBF16)
-    tanh_cols_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(in, ld, (__nv_bfloat16*)out, R, total);
+    launch_dependent(tanh_cols_kernel<__nv_bfloat16>, blocks, 256, 0, st, in, ld,
+                     (__nv_bfloat16*)out, R, total);
   else
     return kBadDType;
   return launch_status();
@@ -807,12 +820,10 @@ extern "C" int cretif_general_delta_recurrence(
   const unsigned blocks = (unsigned)((items + 7) / 8);
   const int w_stride = per_head_weight ? e : 0;
   if (out_dt == kF32)
-    delta_out_norm_kernel<float><<<blocks, 256, 0, st>>>(o_raw, gate, ldg, norm_w, eps,
-                                                         (float*)out, ldo, H, e, items, w_stride,
-                                                         gate_sigmoid);
+    launch_dependent(delta_out_norm_kernel<float>, blocks, 256, 0, st, o_raw, gate, ldg, norm_w,
+                     eps, (float*)out, ldo, H, e, items, w_stride, gate_sigmoid);
   else
-    delta_out_norm_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(
-        o_raw, gate, ldg, norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items, w_stride,
-        gate_sigmoid);
+    launch_dependent(delta_out_norm_kernel<__nv_bfloat16>, blocks, 256, 0, st, o_raw, gate, ldg,
+                     norm_w, eps, (__nv_bfloat16*)out, ldo, H, e, items, w_stride, gate_sigmoid);
   return launch_status();
 }

@@ -210,6 +210,7 @@ add_rmsnorm_rows_kernel(float* __restrict__ h, const TD* __restrict__ delta,
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ act, int I, int block,
                                 GateRule gate, size_t total) {
+  dependent_begin();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const size_t t = idx / I;
@@ -236,6 +237,7 @@ __global__ void rope_kv_append_kernel(T* __restrict__ qkv, int ld, const float* 
                                       const int* __restrict__ table, int table_stride,
                                       T* __restrict__ kc, T* __restrict__ vc, int bt,
                                       int write_cache, unsigned int* __restrict__ fault) {
+  dependent_begin();
   const int t = blockIdx.x;
   const int pos = tok_pos[t];
   T* row = qkv + (size_t)t * ld;
@@ -421,11 +423,11 @@ extern "C" int cretif_silu_mul(const void* gu, void* act, int dt, int T, int I, 
   const size_t total = (size_t)T * I;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (dt == kF32)
-    silu_mul_kernel<float><<<blocks, 256, 0, st>>>((const float*)gu, (float*)act, I, block, gate,
-                                                  total);
+    launch_dependent(silu_mul_kernel<float>, blocks, 256, 0, st, (const float*)gu, (float*)act, I,
+                     block, gate, total);
   else if (dt == kBF16)
-    silu_mul_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)gu,
-                                                          (__nv_bfloat16*)act, I, block, gate, total);
+    launch_dependent(silu_mul_kernel<__nv_bfloat16>, blocks, 256, 0, st, (const __nv_bfloat16*)gu,
+                     (__nv_bfloat16*)act, I, block, gate, total);
   else
     return kBadDType;
   return launch_status();
@@ -444,14 +446,14 @@ extern "C" int cretif_rope_kv_append(void* qkv, int ld, int dt, const float* cos
   cudaStream_t st = (cudaStream_t)stream;
   const int threads = 128;
   if (dt == kF32)
-    rope_kv_append_kernel<float><<<T, threads, 0, st>>>(
-        (float*)qkv, ld, cos_t, sin_t, pairing, rot_dim, nh, nkv, hd, tok_pos, tok_seq, seq_slot,
-        table, table_stride, (float*)kc, (float*)vc, bt, write_cache, fault);
+    launch_dependent(rope_kv_append_kernel<float>, T, threads, 0, st, (float*)qkv, ld, cos_t, sin_t,
+                     pairing, rot_dim, nh, nkv, hd, tok_pos, tok_seq, seq_slot, table, table_stride,
+                     (float*)kc, (float*)vc, bt, write_cache, fault);
   else if (dt == kBF16)
-    rope_kv_append_kernel<__nv_bfloat16><<<T, threads, 0, st>>>(
-        (__nv_bfloat16*)qkv, ld, cos_t, sin_t, pairing, rot_dim, nh, nkv, hd, tok_pos, tok_seq,
-        seq_slot, table, table_stride, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, bt, write_cache,
-        fault);
+    launch_dependent(rope_kv_append_kernel<__nv_bfloat16>, T, threads, 0, st, (__nv_bfloat16*)qkv,
+                     ld, cos_t, sin_t, pairing, rot_dim, nh, nkv, hd, tok_pos, tok_seq, seq_slot,
+                     table, table_stride, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, bt, write_cache,
+                     fault);
   else
     return kBadDType;
   return launch_status();

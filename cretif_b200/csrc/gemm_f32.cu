@@ -59,6 +59,7 @@ template <int MT>
 __global__ void __launch_bounds__(kFewWarps * 32)
 gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                     int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int WK) {
+  dependent_begin();
   constexpr int NV = kR * MT;
   __shared__ float part[kFewWarps][NV];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -235,8 +236,8 @@ static int launch_few(const float* A, const float* W, float* C, int M, int N, in
                       int ldc, int accumulate, int WK, cudaStream_t st) {
   const int rows = kR * (kFewWarps / WK);               // of W, a CTA
   const dim3 grid((M + MT - 1) / MT, (N + rows - 1) / rows);
-  gemm_f32_few_kernel<MT><<<grid, kFewWarps * 32, 0, st>>>(A, W, C, M, N, K, lda, ldw, ldc,
-                                                           accumulate, WK);
+  launch_dependent(gemm_f32_few_kernel<MT>, grid, kFewWarps * 32, 0, st, A, W, C, M, N, K, lda, ldw,
+                   ldc, accumulate, WK);
   return launch_status();
 }
 

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(128)
 gemm_heads_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W,
                   __nv_bfloat16* __restrict__ C, int M, int N, int K, int lda, int ldc,
                   long long sa, long long sw, long long sc, int a_vec, int w_vec) {
+  dependent_begin();
   using namespace nvcuda;
   __shared__ __align__(32) __nv_bfloat16 As[kHM][kHK + kHPad];
   __shared__ __align__(32) __nv_bfloat16 Ws[kHN][kHK + kHPad];
@@ -119,8 +120,8 @@ extern "C" int cretif_gemm_heads(const void* A, const void* W, void* C, int M, i
   const int a_vec = ((uintptr_t)A % 16 == 0) && lda % 8 == 0 && sa % 8 == 0;
   const int w_vec = ((uintptr_t)W % 16 == 0) && K % 8 == 0;
   dim3 grid((N + kHN - 1) / kHN, (M + kHM - 1) / kHM, batch);
-  gemm_heads_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, (__nv_bfloat16*)C, M, N, K, lda, ldc, sa,
-      (long long)N * K, sc, a_vec, w_vec);
+  launch_dependent(gemm_heads_kernel, grid, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)A,
+                   (const __nv_bfloat16*)W, (__nv_bfloat16*)C, M, N, K, lda, ldc, sa,
+                   (long long)N * K, sc, a_vec, w_vec);
   return launch_status();
 }

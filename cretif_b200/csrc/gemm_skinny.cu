@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(kSkWarps * 32)
 gemm_skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W,
                    TC* __restrict__ C, int M, int N, int K, int ldx, int ldw, int ldc,
                    int accumulate) {
+  dependent_begin();
   __shared__ float red[kSkWarps][kSkRows][8 * NT + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = lane >> 2, c = lane & 3;
@@ -96,9 +97,9 @@ static int launch_skinny(const void* X, const void* W, void* C, int M, int N, in
   const int blocks = (N + kSkRows - 1) / kSkRows;
   const int nt = (M + 7) / 8;
 #define CRETIF_SK(NT)                                                                        \
-  gemm_skinny_kernel<NT, TC><<<blocks, kSkWarps * 32, 0, st>>>(                              \
-      (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, (TC*)C, M, N, K, ldx, ldw, ldc,      \
-      accumulate)
+  launch_dependent(gemm_skinny_kernel<NT, TC>, blocks, kSkWarps * 32, 0, st,                      \
+                   (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, (TC*)C, M, N, K, ldx, ldw,   \
+                   ldc, accumulate)
   switch (nt) {
     case 1: CRETIF_SK(1); break;
     case 2: CRETIF_SK(2); break;

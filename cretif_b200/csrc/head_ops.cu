@@ -46,6 +46,7 @@ headnorm_rope_kv_append_kernel(const TI* __restrict__ proj, int ldp,
                                const int* __restrict__ table, int table_stride,
                                T* __restrict__ kc, T* __restrict__ vc, int bt, int write_cache,
                                unsigned int* __restrict__ fault) {
+  dependent_begin();
   __shared__ float normed[kHnWarps][kHnMaxD];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x;
@@ -266,6 +267,7 @@ projnorm_rope_kv_append_kernel(const float* __restrict__ proj, int ldp,
                                int table_stride, T* kc, T* vc, int bt, int write_cache, T* pk, T* pv,
                                const int* __restrict__ pool_table, int pool_stride, int pool,
                                const ProjConv conv, unsigned int* __restrict__ fault) {
+  dependent_wait();
   extern __shared__ __align__(16) float row_s[];       // q | k with the bias
   __shared__ float sums[NT / 32][2];
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -474,6 +476,7 @@ projnorm_rope_kv_append_kernel(const float* __restrict__ proj, int ldp,
 template <typename T>
 __global__ void gate_heads_kernel(T* __restrict__ o, int ldo, const float* __restrict__ g, int ldg,
                                   int nh, int vd, long long total) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int w = nh * vd;
@@ -490,6 +493,7 @@ __global__ void gate_heads_kernel(T* __restrict__ o, int ldo, const float* __res
 __global__ void gate_heads8_kernel(__nv_bfloat16* __restrict__ o, int ldo,
                                    const float* __restrict__ g, int ldg, int nh, int vd,
                                    long long groups) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= groups) return;
   const int per_row = nh * vd / 8;
@@ -513,6 +517,7 @@ __global__ void gate_heads8_kernel(__nv_bfloat16* __restrict__ o, int ldo,
 __global__ void gate_channels8_kernel(__nv_bfloat16* __restrict__ o, int ldo,
                                       const float* __restrict__ g, int ldg, int width,
                                       long long groups) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= groups) return;
   const int per_row = width / 8;
@@ -535,6 +540,7 @@ template <typename TI, typename TO>
 __global__ void activation_kernel(const TI* __restrict__ in, int ldi, TO* __restrict__ out, int ldo,
                                   int width, long long total, int kind, const TO* __restrict__ mul,
                                   int mul_ld, int mul_rows, const int* __restrict__ mul_ids) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const long long t = idx / width;
@@ -549,11 +555,13 @@ __global__ void activation_kernel(const TI* __restrict__ in, int ldi, TO* __rest
 
 // z <- cap * tanh(z / cap), in place, 32-bit.
 __global__ void softcap_kernel(float* __restrict__ z, long long total, float cap) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < total) z[idx] = cap * tanhf(z[idx] / cap);
 }
 
 __global__ void scale_kernel(float* __restrict__ z, long long total, float factor) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < total) z[idx] *= factor;
 }
@@ -562,6 +570,7 @@ __global__ void scale_kernel(float* __restrict__ z, long long total, float facto
 template <typename TY>
 __global__ void axpy_rows_kernel(float* __restrict__ h, const TY* __restrict__ y, float alpha,
                                  long long total) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < total) h[idx] = fmaf(alpha, to_float(y[idx]), h[idx]);
 }
@@ -590,10 +599,10 @@ extern "C" int cretif_headnorm_rope_kv_append(
   cudaStream_t st = (cudaStream_t)stream;
   const int widest = vd > hd ? vd : hd;
 #define CRETIF_HN(TI, TT, NCH)                                                                   \
-  headnorm_rope_kv_append_kernel<TI, TT, NCH><<<grid, kHnWarps * 32, 0, st>>>(                    \
-      (const TI*)proj, ldp, bias, wq, wk, eps, cos_t, sin_t, pairing, rot_dim, tok_pos, tok_seq,  \
-      seq_slot, nh, nkv, hd, vd, (TT*)q_out, ldq, table, table_stride, (TT*)kc, (TT*)vc, bt,      \
-      write_cache, fault)
+  launch_dependent(headnorm_rope_kv_append_kernel<TI, TT, NCH>, grid, kHnWarps * 32, 0, st,       \
+                   (const TI*)proj, ldp, bias, wq, wk, eps, cos_t, sin_t, pairing, rot_dim,       \
+                   tok_pos, tok_seq, seq_slot, nh, nkv, hd, vd, (TT*)q_out, ldq, table,           \
+                   table_stride, (TT*)kc, (TT*)vc, bt, write_cache, fault)
 #define CRETIF_HN_T(TI, TT)                                                                      \
   do {                                                                                           \
     if (widest <= 64) CRETIF_HN(TI, TT, 2);                                                       \
@@ -670,10 +679,11 @@ extern "C" int cretif_projnorm_rope_kv_append(
                                              (int)smem);                                          \
       if (err != cudaSuccess) return (int)err;                                                    \
     }                                                                                             \
-    projnorm_rope_kv_append_kernel<TT, VEC, NT, TAPS><<<T, NT, smem, st>>>(                       \
-        proj, ldp, bias, wq, wk, eps, cos_t, sin_t, pairing, rot_dim, tok_pos, tok_seq, seq_slot, \
-        nh, nkv, hd, vd, v_scale, (TT*)q_out, ldq, table, table_stride, (TT*)kc, (TT*)vc, bt,     \
-        write_cache, (TT*)pool_k, (TT*)pool_v, pool_table, pool_stride, pool, conv, fault);       \
+    launch_dependent(projnorm_rope_kv_append_kernel<TT, VEC, NT, TAPS>, T, NT, smem, st, proj,    \
+                     ldp, bias, wq, wk, eps, cos_t, sin_t, pairing, rot_dim, tok_pos, tok_seq,    \
+                     seq_slot, nh, nkv, hd, vd, v_scale, (TT*)q_out, ldq, table, table_stride,    \
+                     (TT*)kc, (TT*)vc, bt, write_cache, (TT*)pool_k, (TT*)pool_v, pool_table,     \
+                     pool_stride, pool, conv, fault);                                             \
   } while (0)
   if (dt == kF32) {
     CRETIF_PN_T(float);
@@ -722,7 +732,8 @@ extern "C" int cretif_pool_kv(const void* kc, const void* vc, int dt, const int*
 
 extern "C" int cretif_scale(float* z, long long total, float factor, void* stream) {
   if (total <= 0) return kOk;
-  scale_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, total, factor);
+  launch_dependent(scale_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream, z,
+                   total, factor);
   return launch_status();
 }
 
@@ -734,16 +745,17 @@ extern "C" int cretif_gate_heads(void* o, int ldo, int dt, const float* g, int l
   const unsigned blocks = (unsigned)((total + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (dt == kF32)
-    gate_heads_kernel<float><<<blocks, 256, 0, st>>>((float*)o, ldo, g, ldg, nh, vd, total);
+    launch_dependent(gate_heads_kernel<float>, blocks, 256, 0, st, (float*)o, ldo, g, ldg, nh, vd,
+                     total);
   else if (dt == kBF16 && vd == 1 && nh % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)o & 15) == 0)
-    gate_channels8_kernel<<<(unsigned)((total / 8 + 255) / 256), 256, 0, st>>>(
-        (__nv_bfloat16*)o, ldo, g, ldg, nh, total / 8);
+    launch_dependent(gate_channels8_kernel, (unsigned)((total / 8 + 255) / 256), 256, 0, st,
+                     (__nv_bfloat16*)o, ldo, g, ldg, nh, total / 8);
   else if (dt == kBF16 && vd % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)o & 15) == 0)
-    gate_heads8_kernel<<<(unsigned)((total / 8 + 255) / 256), 256, 0, st>>>(
-        (__nv_bfloat16*)o, ldo, g, ldg, nh, vd, total / 8);
+    launch_dependent(gate_heads8_kernel, (unsigned)((total / 8 + 255) / 256), 256, 0, st,
+                     (__nv_bfloat16*)o, ldo, g, ldg, nh, vd, total / 8);
   else if (dt == kBF16)
-    gate_heads_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((__nv_bfloat16*)o, ldo, g, ldg, nh,
-                                                            vd, total);
+    launch_dependent(gate_heads_kernel<__nv_bfloat16>, blocks, 256, 0, st, (__nv_bfloat16*)o, ldo,
+                     g, ldg, nh, vd, total);
   else
     return kBadDType;
   return launch_status();
@@ -759,17 +771,17 @@ extern "C" int cretif_activation(const void* in, int ldi, int in_dt, void* out, 
   const unsigned blocks = (unsigned)((total + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (in_dt == kF32 && out_dt == kF32)
-    activation_kernel<float, float><<<blocks, 256, 0, st>>>((const float*)in, ldi, (float*)out,
-                                                            ldo, width, total, kind,
-                                                            (const float*)mul, mul_ld, mul_rows, mul_ids);
+    launch_dependent(activation_kernel<float, float>, blocks, 256, 0, st, (const float*)in, ldi,
+                     (float*)out, ldo, width, total, kind, (const float*)mul, mul_ld, mul_rows,
+                     mul_ids);
   else if (in_dt == kF32 && out_dt == kBF16)
-    activation_kernel<float, __nv_bfloat16><<<blocks, 256, 0, st>>>(
-        (const float*)in, ldi, (__nv_bfloat16*)out, ldo, width, total, kind,
-        (const __nv_bfloat16*)mul, mul_ld, mul_rows, mul_ids);
+    launch_dependent(activation_kernel<float, __nv_bfloat16>, blocks, 256, 0, st, (const float*)in,
+                     ldi, (__nv_bfloat16*)out, ldo, width, total, kind, (const __nv_bfloat16*)mul,
+                     mul_ld, mul_rows, mul_ids);
   else if (in_dt == kBF16 && out_dt == kBF16)
-    activation_kernel<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, st>>>(
-        (const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo, width, total, kind,
-        (const __nv_bfloat16*)mul, mul_ld, mul_rows, mul_ids);
+    launch_dependent(activation_kernel<__nv_bfloat16, __nv_bfloat16>, blocks, 256, 0, st,
+                     (const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo, width, total, kind,
+                     (const __nv_bfloat16*)mul, mul_ld, mul_rows, mul_ids);
   else
     return kBadDType;
   return launch_status();
@@ -778,7 +790,8 @@ extern "C" int cretif_activation(const void* in, int ldi, int in_dt, void* out, 
 extern "C" int cretif_softcap(float* z, long long total, float cap, void* stream) {
   if (total <= 0) return kOk;
   if (!(cap > 0.f)) return kBadArgument;
-  softcap_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, total, cap);
+  launch_dependent(softcap_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream, z,
+                   total, cap);
   return launch_status();
 }
 
@@ -788,10 +801,10 @@ extern "C" int cretif_axpy_rows(float* h, const void* y, int y_dt, float alpha, 
   const unsigned blocks = (unsigned)((total + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (y_dt == kF32)
-    axpy_rows_kernel<float><<<blocks, 256, 0, st>>>(h, (const float*)y, alpha, total);
+    launch_dependent(axpy_rows_kernel<float>, blocks, 256, 0, st, h, (const float*)y, alpha, total);
   else if (y_dt == kBF16)
-    axpy_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(h, (const __nv_bfloat16*)y, alpha,
-                                                           total);
+    launch_dependent(axpy_rows_kernel<__nv_bfloat16>, blocks, 256, 0, st, h,
+                     (const __nv_bfloat16*)y, alpha, total);
   else
     return kBadDType;
   return launch_status();

@@ -45,6 +45,7 @@ latent_in_kernel(const TI* __restrict__ proj, int ldp, int q_rank, int rank, int
                  const int* __restrict__ seq_slot, T* __restrict__ cq_out, int ldq,
                  const int* __restrict__ table, int table_stride, T* __restrict__ kc, int bt,
                  int write_cache, unsigned int* __restrict__ fault) {
+  dependent_begin();
   __shared__ float sums[2][8];
   __shared__ float kr[kLatMaxRot];
   const int t = blockIdx.x;
@@ -106,6 +107,7 @@ latent_in_rows_kernel(const TI* __restrict__ proj, int ldp, int q_rank, int rank
                       T* __restrict__ cq_out, int ldq, const int* __restrict__ table,
                       int table_stride, T* __restrict__ kc, int bt, int write_cache, int T_tokens,
                       unsigned int* __restrict__ fault) {
+  dependent_begin();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T_tokens) return;
@@ -166,6 +168,7 @@ rope_pairs_kernel(const TI* __restrict__ q, int ldq, int nh, int d, int rot, int
                   const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pairing,
                   const int* __restrict__ tok_pos, T* __restrict__ out, int ldo, int ldh, int off,
                   long long total) {
+  dependent_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int slots = rot >> 1, half = rdims >> 1;
@@ -196,6 +199,7 @@ rope_heads_kernel(const TI* __restrict__ q, int ldq, int nh, int d, int rot, int
                   const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pairing,
                   const int* __restrict__ tok_pos, T* __restrict__ out, int ldo, int ldh, int off,
                   long long items) {
+  dependent_begin();
   __shared__ float part[8][kLatMaxRot];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * 8 + warp;
@@ -217,6 +221,7 @@ rope_heads_kernel(const TI* __restrict__ q, int ldq, int nh, int d, int rot, int
 __global__ void __launch_bounds__(256)
 rmsnorm_row_block_kernel(float* __restrict__ x, int ld, const float* __restrict__ w, int H,
                          float eps) {
+  dependent_begin();
   __shared__ float scratch[33];
   float* row = x + (size_t)blockIdx.x * ld;
   float ss = 0.f;
@@ -230,6 +235,7 @@ rmsnorm_row_block_kernel(float* __restrict__ x, int ld, const float* __restrict_
 __global__ void __launch_bounds__(256)
 rmsnorm_rows_kernel(float* __restrict__ x, int ld, const float* __restrict__ w, int R, int H,
                     float eps) {
+  dependent_begin();
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= R) return;
   float* row = x + (size_t)r * ld;
@@ -267,15 +273,15 @@ extern "C" int cretif_latent_in(const void* proj, int ldp, int proj_dt, int q_ra
 #define CRETIF_LAT(TI, TT)                                                                      \
   do {                                                                                          \
     if (T < 256)                                                                                \
-      latent_in_kernel<TI, TT><<<T, 256, 0, st>>>(                                              \
-          (const TI*)proj, ldp, q_rank, rank, rot, rdims, wq, wc, eps, cos_t, sin_t, pairing,    \
-          tok_pos, tok_seq, seq_slot, (TT*)cq_out, ldq, table, table_stride, (TT*)kc, bt,        \
-          write_cache, fault);                                                                    \
+      launch_dependent(latent_in_kernel<TI, TT>, T, 256, 0, st, (const TI*)proj, ldp, q_rank,     \
+                       rank, rot, rdims, wq, wc, eps, cos_t, sin_t, pairing, tok_pos, tok_seq,    \
+                       seq_slot, (TT*)cq_out, ldq, table, table_stride, (TT*)kc, bt, write_cache, \
+                       fault);                                                                    \
     else                                                                                        \
-      latent_in_rows_kernel<TI, TT><<<(unsigned)((T + 7) / 8), 256, 0, st>>>(                    \
-          (const TI*)proj, ldp, q_rank, rank, rot, rdims, wq, wc, eps, cos_t, sin_t, pairing,    \
-          tok_pos, tok_seq, seq_slot, (TT*)cq_out, ldq, table, table_stride, (TT*)kc, bt,        \
-          write_cache, T, fault);                                                                 \
+      launch_dependent(latent_in_rows_kernel<TI, TT>, (unsigned)((T + 7) / 8), 256, 0, st,        \
+                       (const TI*)proj, ldp, q_rank, rank, rot, rdims, wq, wc, eps, cos_t, sin_t, \
+                       pairing, tok_pos, tok_seq, seq_slot, (TT*)cq_out, ldq, table, table_stride,\
+                       (TT*)kc, bt, write_cache, T, fault);                                       \
   } while (0)
   if (proj_dt == kF32 && dt == kF32) CRETIF_LAT(float, float);
   else if (proj_dt == kF32 && dt == kBF16) CRETIF_LAT(float, __nv_bfloat16);
@@ -301,13 +307,13 @@ extern "C" int cretif_rope_heads(const void* q, int ldq, int q_dt, int nh, int d
 #define CRETIF_RH(TI, TT)                                                                       \
   do {                                                                                          \
     if (T < 256)                                                                                \
-      rope_heads_kernel<TI, TT><<<blocks, 256, 0, st>>>((const TI*)q, ldq, nh, d, rot, rdims,   \
-                                                        cos_t, sin_t, pairing, tok_pos,         \
-                                                        (TT*)out, ldo, ldh, off, items);        \
+      launch_dependent(rope_heads_kernel<TI, TT>, blocks, 256, 0, st, (const TI*)q, ldq, nh, d,   \
+                       rot, rdims, cos_t, sin_t, pairing, tok_pos, (TT*)out, ldo, ldh, off,       \
+                       items);                                                                    \
     else                                                                                        \
-      rope_pairs_kernel<TI, TT><<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(               \
-          (const TI*)q, ldq, nh, d, rot, rdims, cos_t, sin_t, pairing, tok_pos, (TT*)out, ldo,  \
-          ldh, off, pairs);                                                                        \
+      launch_dependent(rope_pairs_kernel<TI, TT>, (unsigned)((pairs + 255) / 256), 256, 0, st,    \
+                       (const TI*)q, ldq, nh, d, rot, rdims, cos_t, sin_t, pairing, tok_pos,      \
+                       (TT*)out, ldo, ldh, off, pairs);                                           \
   } while (0)
   if (q_dt == kF32 && dt == kF32) CRETIF_RH(float, float);
   else if (q_dt == kF32 && dt == kBF16) CRETIF_RH(float, __nv_bfloat16);
@@ -322,9 +328,9 @@ extern "C" int cretif_rmsnorm_rows(float* x, int ld, const float* w, int R, int 
   if (R <= 0) return kOk;
   if (H <= 0 || ld < H || !w) return kBadArgument;
   if (R <= 64)
-    rmsnorm_row_block_kernel<<<R, 256, 0, (cudaStream_t)stream>>>(x, ld, w, H, eps);
+    launch_dependent(rmsnorm_row_block_kernel, R, 256, 0, (cudaStream_t)stream, x, ld, w, H, eps);
   else
-    rmsnorm_rows_kernel<<<(unsigned)((R + 7) / 8), 256, 0, (cudaStream_t)stream>>>(x, ld, w, R, H,
-                                                                                   eps);
+    launch_dependent(rmsnorm_rows_kernel, (unsigned)((R + 7) / 8), 256, 0, (cudaStream_t)stream, x,
+                     ld, w, R, H, eps);
   return launch_status();
 }

@@ -79,6 +79,7 @@ constexpr int kMemChunk = 16;
 template <int R>
 __global__ void __launch_bounds__(256)
 memory_token_kernel(const MemArgs a, int P, int ecols) {
+  dependent_begin();
   extern __shared__ __align__(16) float smem[];
   const int b = blockIdx.x, h = blockIdx.y, H = a.H, d = a.d, e = a.e;
   const int col0 = blockIdx.z * ecols;
@@ -682,6 +683,7 @@ template <typename TO>
 __global__ void __launch_bounds__(256)
 memory_out_kernel(const MemArgs a, const int* __restrict__ tok_seq, const float* __restrict__ norm_w,
                   float eps, TO* __restrict__ out, int ldo, long long items) {
+  dependent_begin();
   const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (item >= items) return;
@@ -800,10 +802,11 @@ extern "C" int cretif_matrix_memory(const float* proj, int ldp, const float* bia
   const long long items = (long long)T * H;
   const unsigned blocks = (unsigned)((items + 7) / 8);
   if (out_dt == kF32)
-    memory_out_kernel<float><<<blocks, 256, 0, st>>>(a, tok_seq, norm_w, eps, (float*)out, ldo, items);
+    launch_dependent(memory_out_kernel<float>, blocks, 256, 0, st, a, tok_seq, norm_w, eps,
+                     (float*)out, ldo, items);
   else if (out_dt == kBF16)
-    memory_out_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(a, tok_seq, norm_w, eps,
-                                                             (__nv_bfloat16*)out, ldo, items);
+    launch_dependent(memory_out_kernel<__nv_bfloat16>, blocks, 256, 0, st, a, tok_seq, norm_w, eps,
+                     (__nv_bfloat16*)out, ldo, items);
   else
     return kBadDType;
   return launch_status();

@@ -225,6 +225,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRouteWarps * 32)
 moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr, int E, int H,
                  const RouteRule rule, int* __restrict__ ids, float* __restrict__ wts, int vec) {
+  dependent_begin();
   __shared__ float logits[kMaxExperts];
   __shared__ float scratch[2 * kMaxExperts];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,6 +258,7 @@ moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr,
 __global__ void __launch_bounds__(256)
 moe_topk_kernel(const float* __restrict__ logits, int ld, int E, const RouteRule rule,
                 int* __restrict__ ids, float* __restrict__ wts, int T) {
+  dependent_begin();
   __shared__ float scratch[8][2 * kMaxExperts];
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -565,6 +567,7 @@ __global__ void __launch_bounds__(256)
 moe_gemv_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, void* Cv, int ldc, int N,
                 int K, int top, int mode, int scale_at, const int* __restrict__ ids,
                 const float* __restrict__ wts, int vec, int experts, const GateRule gate) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char gemv_smem[];
   T* xs = reinterpret_cast<T*>(gemv_smem);
   const int p = blockIdx.y;
@@ -646,6 +649,7 @@ moe_combine_kernel(const float* __restrict__ rows, int ld, const int* __restrict
                    const int* __restrict__ ids, int experts, const float* __restrict__ id_wts,
                    const TX* __restrict__ x, int ldx, const float* __restrict__ plus, int add,
                    __nv_bfloat16* __restrict__ x_out) {
+  dependent_begin();
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (idx >= (long long)T * H) return;
   const int t = (int)(idx / H), c = (int)(idx - (long long)t * H);
@@ -720,11 +724,11 @@ extern "C" int cretif_moe_route(const void* x, int x_dt, int ldx, const float* r
   cudaStream_t st = (cudaStream_t)stream;
   const int vec = H % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)router_w) & 15) == 0;
   if (x_dt == kF32)
-    moe_route_kernel<float><<<T, kRouteWarps * 32, 0, st>>>((const float*)x, ldx, router_w, E, H,
-                                                            rule, ids, wts, vec);
+    launch_dependent(moe_route_kernel<float>, T, kRouteWarps * 32, 0, st, (const float*)x, ldx,
+                     router_w, E, H, rule, ids, wts, vec);
   else if (x_dt == kBF16)
-    moe_route_kernel<__nv_bfloat16><<<T, kRouteWarps * 32, 0, st>>>(
-        (const __nv_bfloat16*)x, ldx, router_w, E, H, rule, ids, wts, vec);
+    launch_dependent(moe_route_kernel<__nv_bfloat16>, T, kRouteWarps * 32, 0, st,
+                     (const __nv_bfloat16*)x, ldx, router_w, E, H, rule, ids, wts, vec);
   else
     return kBadDType;
   return launch_status();
@@ -739,8 +743,8 @@ extern "C" int cretif_moe_topk(const float* logits, int ld, int E, int top, int 
   if (E <= 0 || E > kMaxExperts || top <= 0 || top > E || ld < E) return kBadArgument;
   if (!route_rule_ok(E, top, groups, keep)) return kBadArgument;
   const RouteRule rule{top, renorm, groups, keep, sum_eps, softmax, group_best, correction, bias};
-  moe_topk_kernel<<<(unsigned)((T + 7) / 8), 256, 0, (cudaStream_t)stream>>>(logits, ld, E, rule,
-                                                                             ids, wts, T);
+  launch_dependent(moe_topk_kernel, (unsigned)((T + 7) / 8), 256, 0, (cudaStream_t)stream, logits,
+                   ld, E, rule, ids, wts, T);
   return launch_status();
 }
 
@@ -886,13 +890,13 @@ extern "C" int cretif_moe_combine(const float* rows, int ld, const int* place, i
 #define CRETIF_COMBINE(TX)                                                                          \
   do {                                                                                              \
     if (vec)                                                                                        \
-      moe_combine_kernel<TX, 4><<<blocks, 256, 0, st>>>(rows, ld, place, top, wts, y, T, H, ids,    \
-                                                        experts, id_wts, (const TX*)x, ldx, plus,     \
-                                                        add, (__nv_bfloat16*)x_out);  \
+      launch_dependent(moe_combine_kernel<TX, 4>, blocks, 256, 0, st, rows, ld, place, top, wts,  \
+                       y, T, H, ids, experts, id_wts, (const TX*)x, ldx, plus, add,               \
+                       (__nv_bfloat16*)x_out);                                                    \
     else                                                                                            \
-      moe_combine_kernel<TX, 1><<<blocks, 256, 0, st>>>(rows, ld, place, top, wts, y, T, H, ids,    \
-                                                        experts, id_wts, (const TX*)x, ldx, plus,     \
-                                                        add, (__nv_bfloat16*)x_out);  \
+      launch_dependent(moe_combine_kernel<TX, 1>, blocks, 256, 0, st, rows, ld, place, top, wts,  \
+                       y, T, H, ids, experts, id_wts, (const TX*)x, ldx, plus, add,               \
+                       (__nv_bfloat16*)x_out);                                                    \
   } while (0)
   if (x_dt == kF32) CRETIF_COMBINE(float);
   else if (x_dt == kBF16) CRETIF_COMBINE(__nv_bfloat16);

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_add_kernel(float* __restrict__ h, const TY* __restrict__ y, int ldy,
                    const float* __restrict__ weight, int R, int H, float eps,
                    __nv_bfloat16* __restrict__ x_out) {
+  dependent_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x * 8 + warp;
   if (r >= R) return;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_add_row_block_kernel(float* __restrict__ h, const TY* __restrict__ y, int ldy,
                              const float* __restrict__ weight, int H, float eps,
                              __nv_bfloat16* __restrict__ x_out) {
+  dependent_begin();
   __shared__ float sums[8];
   const int r = blockIdx.x, tid = threadIdx.x, n4 = H >> 2;
   const TY* yrow = y + (size_t)r * ldy;
@@ -284,6 +286,7 @@ static int launch_layernorm(float* h, const TD* delta, const float* w, const flo
 template <typename TO>
 __global__ void convert_rows_kernel(const float* __restrict__ h, TO* __restrict__ out,
                                     size_t total) {
+  dependent_begin();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total) out[i] = from_float<TO>(h[i]);
 }
@@ -292,6 +295,7 @@ __global__ void convert_rows_kernel(const float* __restrict__ h, TO* __restrict_
 template <typename TO, int V>
 __global__ void __launch_bounds__(256)
 convert_into_kernel(const float* __restrict__ h, TO* __restrict__ out, int ldo, int H, long long total) {
+  dependent_begin();
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (idx >= total) return;
   const long long r = idx / H;
@@ -313,6 +317,7 @@ proj_norm_kv_append_kernel(T* __restrict__ row0, int ld, int q_dim, const float*
                            const int* __restrict__ seq_slot, const int* __restrict__ table,
                            int table_stride, T* __restrict__ kc, T* __restrict__ vc, int bt,
                            int write_cache, unsigned int* __restrict__ fault) {
+  dependent_begin();
   __shared__ float scratch[33];
   const int t = blockIdx.x;
   T* row = row0 + (size_t)t * ld;
@@ -373,21 +378,26 @@ extern "C" int cretif_rmsnorm_add(float* h, const void* y, int y_dt, int ldy, co
   __nv_bfloat16* xo = (__nv_bfloat16*)x_out;
   if (vec && R < 256 && H >= 512) {
     if (y_dt == kF32)
-      rmsnorm_add_row_block_kernel<float><<<R, 256, 0, st>>>(h, (const float*)y, ldy, weight, H, eps, xo);
+      launch_dependent(rmsnorm_add_row_block_kernel<float>, R, 256, 0, st, h, (const float*)y, ldy,
+                       weight, H, eps, xo);
     else if (y_dt == kBF16)
-      rmsnorm_add_row_block_kernel<__nv_bfloat16><<<R, 256, 0, st>>>(h, (const __nv_bfloat16*)y, ldy,
-                                                                     weight, H, eps, xo);
+      launch_dependent(rmsnorm_add_row_block_kernel<__nv_bfloat16>, R, 256, 0, st, h,
+                       (const __nv_bfloat16*)y, ldy, weight, H, eps, xo);
     else
       return kBadDType;
     return launch_status();
   }
   if (y_dt == kF32) {
-    if (vec) rmsnorm_add_kernel<float, true><<<blocks, 256, 0, st>>>(h, (const float*)y, ldy, weight, R, H, eps, xo);
-    else rmsnorm_add_kernel<float, false><<<blocks, 256, 0, st>>>(h, (const float*)y, ldy, weight, R, H, eps, xo);
+    if (vec) launch_dependent(rmsnorm_add_kernel<float, true>, blocks, 256, 0, st, h,
+                              (const float*)y, ldy, weight, R, H, eps, xo);
+    else launch_dependent(rmsnorm_add_kernel<float, false>, blocks, 256, 0, st, h, (const float*)y,
+                          ldy, weight, R, H, eps, xo);
   } else if (y_dt == kBF16) {
     typedef __nv_bfloat16 bf16;
-    if (vec) rmsnorm_add_kernel<bf16, true><<<blocks, 256, 0, st>>>(h, (const bf16*)y, ldy, weight, R, H, eps, xo);
-    else rmsnorm_add_kernel<bf16, false><<<blocks, 256, 0, st>>>(h, (const bf16*)y, ldy, weight, R, H, eps, xo);
+    if (vec) launch_dependent(rmsnorm_add_kernel<bf16, true>, blocks, 256, 0, st, h, (const bf16*)y,
+                              ldy, weight, R, H, eps, xo);
+    else launch_dependent(rmsnorm_add_kernel<bf16, false>, blocks, 256, 0, st, h, (const bf16*)y,
+                          ldy, weight, R, H, eps, xo);
   } else {
     return kBadDType;
   }
@@ -421,10 +431,10 @@ extern "C" int cretif_convert_rows(const float* h, void* out, int out_dt, long l
   cudaStream_t st = (cudaStream_t)stream;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (out_dt == kF32)
-    convert_rows_kernel<float><<<blocks, 256, 0, st>>>(h, (float*)out, (size_t)total);
+    launch_dependent(convert_rows_kernel<float>, blocks, 256, 0, st, h, (float*)out, (size_t)total);
   else if (out_dt == kBF16)
-    convert_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(h, (__nv_bfloat16*)out,
-                                                              (size_t)total);
+    launch_dependent(convert_rows_kernel<__nv_bfloat16>, blocks, 256, 0, st, h, (__nv_bfloat16*)out,
+                     (size_t)total);
   else
     return kBadDType;
   return launch_status();
@@ -440,12 +450,16 @@ extern "C" int cretif_convert_into(const float* h, void* out, int out_dt, int ld
   const bool vec = H % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)h | (uintptr_t)out) & 15) == 0;
   const unsigned blocks = (unsigned)(((vec ? total / 4 : total) + 255) / 256);
   if (out_dt == kF32) {
-    if (vec) convert_into_kernel<float, 4><<<blocks, 256, 0, st>>>(h, (float*)out, ldo, H, total);
-    else convert_into_kernel<float, 1><<<blocks, 256, 0, st>>>(h, (float*)out, ldo, H, total);
+    if (vec) launch_dependent(convert_into_kernel<float, 4>, blocks, 256, 0, st, h, (float*)out,
+                              ldo, H, total);
+    else launch_dependent(convert_into_kernel<float, 1>, blocks, 256, 0, st, h, (float*)out, ldo, H,
+                          total);
   } else {
     typedef __nv_bfloat16 bf16;
-    if (vec) convert_into_kernel<bf16, 4><<<blocks, 256, 0, st>>>(h, (bf16*)out, ldo, H, total);
-    else convert_into_kernel<bf16, 1><<<blocks, 256, 0, st>>>(h, (bf16*)out, ldo, H, total);
+    if (vec) launch_dependent(convert_into_kernel<bf16, 4>, blocks, 256, 0, st, h, (bf16*)out, ldo,
+                              H, total);
+    else launch_dependent(convert_into_kernel<bf16, 1>, blocks, 256, 0, st, h, (bf16*)out, ldo, H,
+                          total);
   }
   return launch_status();
 }
@@ -461,13 +475,13 @@ extern "C" int cretif_proj_norm_kv_append(void* rows, int ld, int dt, int q_dim,
     return kBadArgument;
   cudaStream_t st = (cudaStream_t)stream;
   if (dt == kF32)
-    proj_norm_kv_append_kernel<float><<<T, 256, 0, st>>>(
-        (float*)rows, ld, q_dim, wq, nkv, hd, wk, eps, tok_pos, tok_seq, seq_slot, table,
-        table_stride, (float*)kc, (float*)vc, bt, write_cache, fault);
+    launch_dependent(proj_norm_kv_append_kernel<float>, T, 256, 0, st, (float*)rows, ld, q_dim, wq,
+                     nkv, hd, wk, eps, tok_pos, tok_seq, seq_slot, table, table_stride, (float*)kc,
+                     (float*)vc, bt, write_cache, fault);
   else if (dt == kBF16)
-    proj_norm_kv_append_kernel<__nv_bfloat16><<<T, 256, 0, st>>>(
-        (__nv_bfloat16*)rows, ld, q_dim, wq, nkv, hd, wk, eps, tok_pos, tok_seq, seq_slot, table,
-        table_stride, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, bt, write_cache, fault);
+    launch_dependent(proj_norm_kv_append_kernel<__nv_bfloat16>, T, 256, 0, st, (__nv_bfloat16*)rows,
+                     ld, q_dim, wq, nkv, hd, wk, eps, tok_pos, tok_seq, seq_slot, table,
+                     table_stride, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, bt, write_cache, fault);
   else
     return kBadDType;
   return launch_status();

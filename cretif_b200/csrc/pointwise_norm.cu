@@ -84,6 +84,7 @@ template <typename TD, typename TO, int VEC>
 __global__ void __launch_bounds__(256)
 dyt_rows_kernel(float* __restrict__ h, const TD* __restrict__ delta, DytParams p,
                 TO* __restrict__ out, const int* __restrict__ rows, int R, int H, int write_h) {
+  dependent_begin();
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (idx >= (long long)R * H) return;
   const int r = (int)(idx / H), c = (int)(idx - (long long)r * H);
@@ -102,6 +103,7 @@ template <typename TY, int VEC>
 __global__ void __launch_bounds__(256)
 dyt_add_kernel(float* __restrict__ h, const TY* __restrict__ y, int ldy, DytParams p, int R,
                int H) {
+  dependent_begin();
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (idx >= (long long)R * H) return;
   const int r = (int)(idx / H), c = (int)(idx - (long long)r * H);
@@ -119,6 +121,7 @@ shift_rows_kernel(const float* __restrict__ h, DytParams p, const float* __restr
                   float* __restrict__ state, size_t state_stride,
                   const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
                   const int* __restrict__ cu_seqlens, TO* __restrict__ out, int T, int H) {
+  dependent_begin();
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (idx >= (long long)T * H) return;
   const int t = (int)(idx / H), c = (int)(idx - (long long)t * H);
@@ -170,10 +173,10 @@ extern "C" int cretif_dyt_rows(float* h, const void* delta, int delta_dt, const 
   if (delta && delta_dt != kF32 && delta_dt != kBF16) return kBadDType;
 #define CRETIF_DYT(TD, TO)                                                                      \
   do {                                                                                          \
-    if (vec) dyt_rows_kernel<TD, TO, 4><<<g, 256, 0, st>>>(h, (const TD*)delta, p, (TO*)out,     \
-                                                           rows, R, H, write_h);                 \
-    else dyt_rows_kernel<TD, TO, 1><<<g, 256, 0, st>>>(h, (const TD*)delta, p, (TO*)out, rows,  \
-                                                       R, H, write_h);                           \
+    if (vec) launch_dependent(dyt_rows_kernel<TD, TO, 4>, g, 256, 0, st, h, (const TD*)delta, p,  \
+                              (TO*)out, rows, R, H, write_h);                                     \
+    else launch_dependent(dyt_rows_kernel<TD, TO, 1>, g, 256, 0, st, h, (const TD*)delta, p,      \
+                          (TO*)out, rows, R, H, write_h);                                         \
   } while (0)
   const bool dbf = delta && delta_dt == kBF16;
   if (out_dt == kF32) {
@@ -198,11 +201,14 @@ extern "C" int cretif_dyt_add(float* h, const void* y, int y_dt, int ldy, const 
   const unsigned g = blocks_for(((long long)R * H + (vec ? 3 : 0)) / (vec ? 4 : 1));
   typedef __nv_bfloat16 bf16;
   if (y_dt == kF32) {
-    if (vec) dyt_add_kernel<float, 4><<<g, 256, 0, st>>>(h, (const float*)y, ldy, p, R, H);
-    else dyt_add_kernel<float, 1><<<g, 256, 0, st>>>(h, (const float*)y, ldy, p, R, H);
+    if (vec) launch_dependent(dyt_add_kernel<float, 4>, g, 256, 0, st, h, (const float*)y, ldy, p,
+                              R, H);
+    else launch_dependent(dyt_add_kernel<float, 1>, g, 256, 0, st, h, (const float*)y, ldy, p, R,
+                          H);
   } else if (y_dt == kBF16) {
-    if (vec) dyt_add_kernel<bf16, 4><<<g, 256, 0, st>>>(h, (const bf16*)y, ldy, p, R, H);
-    else dyt_add_kernel<bf16, 1><<<g, 256, 0, st>>>(h, (const bf16*)y, ldy, p, R, H);
+    if (vec) launch_dependent(dyt_add_kernel<bf16, 4>, g, 256, 0, st, h, (const bf16*)y, ldy, p, R,
+                              H);
+    else launch_dependent(dyt_add_kernel<bf16, 1>, g, 256, 0, st, h, (const bf16*)y, ldy, p, R, H);
   } else {
     return kBadDType;
   }
@@ -222,8 +228,8 @@ extern "C" int cretif_shift_rows(const float* h, const float* w, const float* b,
   const unsigned g = blocks_for(((long long)T * H + (vec ? 3 : 0)) / (vec ? 4 : 1));
   typedef __nv_bfloat16 bf16;
 #define CRETIF_SHIFT(TO, V)                                                                     \
-  shift_rows_kernel<TO, V><<<g, 256, 0, st>>>(h, p, shift, state, (size_t)state_stride, tok_seq, \
-                                              seq_slot, cu_seqlens, (TO*)out, T, H)
+  launch_dependent(shift_rows_kernel<TO, V>, g, 256, 0, st, h, p, shift, state,                   \
+                   (size_t)state_stride, tok_seq, seq_slot, cu_seqlens, (TO*)out, T, H)
   if (out_dt == kF32) {
     if (vec) CRETIF_SHIFT(float, 4); else CRETIF_SHIFT(float, 1);
   } else if (out_dt == kBF16) {

@@ -31,6 +31,7 @@ retention_prepare_kernel(const float* __restrict__ proj, int ldp, float* __restr
                          const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                          int pairing, int rot_dim, const int* __restrict__ tok_pos, int H, int d,
                          float k_scale) {
+  dependent_begin();
   const int t = blockIdx.x;
   const int pos = tok_pos[t];
   const int half = rot_dim >> 1;
@@ -66,6 +67,7 @@ retention_recurrence_kernel(const float* __restrict__ prep, int ldp, const float
                             size_t state_stride, const int* __restrict__ cu_seqlens,
                             const int* __restrict__ seq_slot, int H, int d, int e, int P, int ecols,
                             float* __restrict__ o_raw, int write_state) {
+  dependent_begin();
   extern __shared__ __align__(16) float smem[];
   const int b = blockIdx.x, h = blockIdx.y;
   const int col0 = blockIdx.z * ecols;
@@ -560,9 +562,9 @@ extern "C" int cretif_retention_prepare(const float* proj, int ldp, float* prep,
     return kBadArgument;
   if (rot_dim > 0 && (!cos_t || !sin_t)) return kBadArgument;
   const int per_token = T < 64 ? (2 * H * d + 255) / 256 : 1;
-  retention_prepare_kernel<<<dim3(T, per_token > 65535 ? 65535 : per_token), 256, 0,
-                             (cudaStream_t)stream>>>(
-      proj, ldp, prep, ldo, cos_t, sin_t, pairing, rot_dim, tok_pos, H, d, k_scale);
+  launch_dependent(retention_prepare_kernel, dim3(T, per_token > 65535 ? 65535 : per_token), 256, 0,
+                   (cudaStream_t)stream, proj, ldp, prep, ldo, cos_t, sin_t, pairing, rot_dim,
+                   tok_pos, H, d, k_scale);
   return launch_status();
 }
 

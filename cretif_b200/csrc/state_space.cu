@@ -79,6 +79,7 @@ constexpr int kSpTokens = 8;
 template <int TAPS, int NT>
 __global__ void __launch_bounds__(256)
 ssm_prepare_kernel(const SsmArgs a, int save) {
+  dependent_begin();
   const int C = a.channels();
   const int c = blockIdx.y * 256 + threadIdx.x;
   const int first = blockIdx.x * NT, last = min(first + NT, a.T);
@@ -151,8 +152,8 @@ int launch_ssm_prepare(const SsmArgs& a, int save, cudaStream_t st) {
   if (grid.y > 65535) return kBadArgument;
 #define CRETIF_SSM_PREP(TAPS)                                                        \
   do {                                                                               \
-    if (few) ssm_prepare_kernel<TAPS, 1><<<grid, 256, 0, st>>>(a, save);             \
-    else ssm_prepare_kernel<TAPS, kSpTokens><<<grid, 256, 0, st>>>(a, save);         \
+    if (few) launch_dependent(ssm_prepare_kernel<TAPS, 1>, grid, 256, 0, st, a, save);             \
+    else launch_dependent(ssm_prepare_kernel<TAPS, kSpTokens>, grid, 256, 0, st, a, save);         \
   } while (0)
   if (a.taps == 4) CRETIF_SSM_PREP(4);
   else if (a.taps == 3) CRETIF_SSM_PREP(3);
@@ -169,6 +170,7 @@ constexpr int kSsmChunk = 16;
 template <int R>
 __global__ void __launch_bounds__(256)
 ssm_token_kernel(const SsmArgs a, int P, int ecols) {
+  dependent_begin();
   extern __shared__ __align__(16) float smem[];
   const int b = blockIdx.x, h = blockIdx.y, N = a.N, e = a.e;
   const int col0 = blockIdx.z * ecols;
@@ -731,6 +733,7 @@ template <int NT, bool VEC, typename TO>
 __global__ void __launch_bounds__(256)
 ssm_out_kernel(const SsmArgs a, int parts, const float* __restrict__ norm_w, float eps,
                TO* __restrict__ out, int ldo, long long items) {
+  dependent_begin();
   __shared__ float scratch[33];
   const long long item = (long long)blockIdx.x * (256 / NT) + threadIdx.x / NT;
   const int tid = threadIdx.x % NT;
@@ -807,11 +810,15 @@ int launch_ssm_out(const SsmArgs& a, int parts, const float* norm_w, float eps, 
   if (blocks > 0x7fffffffLL) return kBadArgument;
   const unsigned grid = (unsigned)blocks;
   if (warps) {
-    if (vec) ssm_out_kernel<32, true, TO><<<grid, 256, 0, st>>>(a, parts, norm_w, eps, out, ldo, items);
-    else ssm_out_kernel<32, false, TO><<<grid, 256, 0, st>>>(a, parts, norm_w, eps, out, ldo, items);
+    if (vec) launch_dependent(ssm_out_kernel<32, true, TO>, grid, 256, 0, st, a, parts, norm_w, eps,
+                              out, ldo, items);
+    else launch_dependent(ssm_out_kernel<32, false, TO>, grid, 256, 0, st, a, parts, norm_w, eps,
+                          out, ldo, items);
   } else {
-    if (vec) ssm_out_kernel<256, true, TO><<<grid, 256, 0, st>>>(a, parts, norm_w, eps, out, ldo, items);
-    else ssm_out_kernel<256, false, TO><<<grid, 256, 0, st>>>(a, parts, norm_w, eps, out, ldo, items);
+    if (vec) launch_dependent(ssm_out_kernel<256, true, TO>, grid, 256, 0, st, a, parts, norm_w,
+                              eps, out, ldo, items);
+    else launch_dependent(ssm_out_kernel<256, false, TO>, grid, 256, 0, st, a, parts, norm_w, eps,
+                          out, ldo, items);
   }
   return launch_status();
 }
