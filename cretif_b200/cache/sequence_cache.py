@@ -194,6 +194,7 @@ class SequenceCache:
         self._kv_of: Dict[int, Tuple[_KVGroup, int]] = {}
         self._pool_of: Dict[int, Tuple[_KVGroup, int]] = {}
         self._state: Dict[int, torch.Tensor] = {}
+        self._slot_states: Dict[int, List[torch.Tensor]] = {}       # a slot's views of them
         by_request: Dict[KVRequest, List[int]] = {}
         for cid in sorted(requests, key=_id_order):
             # a part may ask for both kinds at once (keys and values, and a state beside them)
@@ -236,8 +237,12 @@ class SequenceCache:
     def alloc_slot(self) -> int:
         slot = self.slots.take()
         self.lengths[slot] = 0
-        for t in self._state.values():
-            t[slot].zero_()
+        if self._state:
+            # all of the slot's states in one launch (a zero_() each was twelve launches of 11 us on
+            # the host a sequence in a model of twelve recurrent layers)
+            if slot not in self._slot_states:
+                self._slot_states[slot] = [t[slot] for t in self._state.values()]
+            torch._foreach_zero_(self._slot_states[slot])
         return slot
 
     def free_slot(self, slot: int) -> None:
