@@ -189,6 +189,26 @@ enum Variant : int {
 };
 void count_variant(int v);
 
+// Block-wide: the sequence of a step that has `rank` longer ones (of equals the earlier counts as
+// longer).  CTAs that walk a whole sequence and do not all run at once are launched with the
+// sequence as the slowest grid index in this order: what starts last is then short, and the chip
+// does not wait for a long one.  With more than 64 sequences they keep their own order.
+__device__ __forceinline__ int sequence_by_length(const int* cu, int B, int rank) {
+  __shared__ int found;
+  if (B > 64) return rank;
+  for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    const int n = cu[b + 1] - cu[b];
+    int longer = 0;
+    for (int i = 0; i < B; ++i) {
+      const int m = cu[i + 1] - cu[i];
+      longer += m > n || (m == n && i < b);
+    }
+    if (longer == rank) found = b;
+  }
+  __syncthreads();
+  return found;
+}
+
 // A kernel of a step's chain of small launches begins with dependent_begin(): the kernel behind it
 // may be launched (its own beginning, and the weights that it asks for ahead, then run under this
 // one), and nothing of the kernels before it is read before they are done.  Every thread goes

@@ -402,7 +402,7 @@ template <int D, int EC, bool GENERAL>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__ v, int ldv,
                          float* __restrict__ state, size_t state_stride,
-                         const int* __restrict__ cu, const int* __restrict__ seq_slot, int H,
+                         const int* __restrict__ cu, const int* __restrict__ seq_slot, int B, int H,
                          int e, float* __restrict__ o_raw, int write_state) {
   using P = StatePlan<D, EC, GENERAL>;
   constexpr int LD = P::LD, KS = P::KS, J = EC / 4, I = D / 64;
@@ -415,7 +415,7 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   float* ST = XO + 2 * P::kXO;               // the state's slice, a row per column: [EC][LD]
   float* red = ST + EC * LD;                 // [KS][2 kC][EC + 4]
   float* X = red + P::kRed;                  // [kC][EC]
-  const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * EC;
+  const int b = sequence_by_length(cu, B, blockIdx.z), h = blockIdx.x, col0 = blockIdx.y * EC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t0 = cu[b], t1 = cu[b + 1];
   const Rows at = rows_of(H, D, e, GENERAL);
@@ -601,8 +601,9 @@ int launch_state_t(const float* ws, const float* v, int ldv, float* state, size_
   auto kern = delta_chunk_state_kernel<D, EC, GENERAL>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return (int)err;
-  kern<<<dim3(B, H, e / EC), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, H, e, o_raw,
-                                               write_state);
+  if (B > 65535) return kBadArgument;
+  kern<<<dim3(H, e / EC, B), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
+                                               o_raw, write_state);
   return launch_status();
 }
 

@@ -531,7 +531,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
   constexpr int NR = kScThreads / CG;      // threads along the rows
   constexpr int RT = C / NR;               // read-out rows a thread
   const int tid = threadIdx.x, H = a.H, N = a.N, e = a.e;
-  const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * EC;
+  const int b = sequence_by_length(a.cu, a.B, blockIdx.z), h = blockIdx.x, col0 = blockIdx.y * EC;
   const int t0 = a.cu[b], t1 = a.cu[b + 1];
   if (t1 <= t0) return;
   const int ldq = ssm_chunk_ld(N);
@@ -703,7 +703,8 @@ int launch_ssm_carry(const SsmArgs& a, cudaStream_t st) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
-  kern<<<dim3(a.B, a.H, a.e / EC), kScThreads, smem, st>>>(a, nbuf);
+  if (a.B > 65535) return kBadArgument;
+  kern<<<dim3(a.H, a.e / EC, a.B), kScThreads, smem, st>>>(a, nbuf);
   return launch_status();
 }
 
