@@ -484,13 +484,14 @@ int cretif_projnorm_rope_kv_append(
 // Matrix memory with exponential gates (matrix_memory.cu): proj rows (float32) [q (H d) | k (H d) |
 // v (H e) | gate (H e) | z_i (H) | z_f (H) | ...] -> out [T, H e], the normed and gated read-outs; a
 // slot's state is [S (H d e) | n (H d) | m (H)].  Scratch: o_raw [T, H e], den and ref [T, H] float32,
-// gates [3, H, T] float64.  form: 0 chooses, 1 token by token, 2 chunks of 64 tokens.
+// gates [3, H, T] float64.  form: 0 chooses, 1 token by token, 2 chunks of 64 tokens, 3 chunks that
+// are walked.  ws (may be null): float32 [(T / 64 + B) H (d e + d + 2)] for chunks that are scanned.
 int cretif_matrix_memory(const float* proj, int ldp, const float* bias_i, const float* bias_f,
                          float cap, float q_scale, float* state, long long state_stride,
                          const int* cu_seqlens, const int* seq_slot, const int* tok_seq, int B, int H,
                          int d, int e, const float* norm_w, float eps, float* o_raw, float* den,
                          float* ref, double* gates, void* out, int out_dt, int ldo, int write_state,
-                         int T, int form, void* stream);
+                         int T, int form, float* ws, void* stream);
 
 // The Mamba-2 recurrence (state_space.cu): proj rows (float32) [z (H e) | x (H e) | B (G N) | C (G N) |
 // dt (H) | ...] -> out [T, H e], the gated and normed read-outs.  conv_w [taps, C'], conv_b [C'],

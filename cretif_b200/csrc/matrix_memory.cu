@@ -222,6 +222,11 @@ int launch_memory_token(const MemArgs& a, int P, int ecols, cudaStream_t st) {
 //   Nothing here depends on the state, so a long prompt fills the chip.
 // * memory_carry_kernel (a CTA per (sequence, head, EC columns of S), and one more per (sequence,
 //   head) that carries n) walks the sequence's chunks with its part of the state in shared memory.
+// * or, where those CTAs would leave the chip idle: memory_intra_kernel also leaves every chunk's own
+//   sum, sum_s exp(u_s - U_n) k_s v_s^T, memory_scan_kernel turns these into the state before every
+//   chunk (a thread per four elements, the chunks' sums asked for ahead), and memory_read_kernel (a
+//   CTA per (chunk, head)) adds what that state gives the read-outs.  What remains of the walk is a
+//   multiply-add per element and chunk instead of two products with three barriers.
 // The matrix products are the retention's (32-bit FMA, 16-byte shared-memory loads, rows padded to
 // 4 mod 8 floats).
 constexpr int kMcTokens = 64;
@@ -268,7 +273,7 @@ __host__ __device__ inline int memory_chunk_ld(int d) {
 inline size_t memory_intra_smem(int d) {
   return sizeof(double) * 2 * kMcTokens +
          sizeof(float) * (2 * (size_t)kMcTokens * memory_chunk_ld(d) + (size_t)kMcTokens * kMcSlab +
-                          (size_t)kMcTokens * kMcScoreLd);
+                          (size_t)kMcTokens * kMcScoreLd + kMcTokens);
 }
 inline size_t memory_carry_smem(int d, int ec, int nbuf) {
   return sizeof(double) * 3 * kMcTokens * nbuf +
@@ -276,25 +281,39 @@ inline size_t memory_carry_smem(int d, int ec, int nbuf) {
                           (size_t)d * ec + kMcTokens);
 }
 
+// The chunks' own sums, then the states before them, where the chunks are scanned: S [chunk][H][d e],
+// n [chunk][H][d] and m [chunk][H]; chunks in the order of the sequences.  S null: they are walked.
+struct ChunkSums {
+  float* S;
+  float* n;
+  double* m;
+};
+
+// Which sequence's which chunk: chunk x of all of them.  c0 < 0: there are fewer.
+__device__ __forceinline__ void memory_chunk(const int* cu, int B, int x, int& b, int& c0, int& t1) {
+  int left = x;
+  c0 = -1;
+  for (b = 0; b < B; ++b) {
+    const int s0 = cu[b], s1 = cu[b + 1];
+    const int chunks = (s1 - s0 + kMcTokens - 1) / kMcTokens;
+    if (left < chunks) {
+      c0 = s0 + left * kMcTokens;
+      t1 = s1;
+      return;
+    }
+    left -= chunks;
+  }
+}
+
 __global__ void __launch_bounds__(kMcThreads)
-memory_intra_kernel(const MemArgs a, double* __restrict__ gates) {
+memory_intra_kernel(const MemArgs a, double* __restrict__ gates, const ChunkSums cs) {
   extern __shared__ __align__(16) float smem[];
   constexpr int C = kMcTokens;
   constexpr int LP = kMcScoreLd;
   const int tid = threadIdx.x, H = a.H, d = a.d, e = a.e;
   const int h = blockIdx.y;
-  // which sequence's which chunk: the grid has a CTA for every chunk there can be
-  int left = blockIdx.x, c0 = -1, t1 = 0;
-  for (int b = 0; b < a.B; ++b) {
-    const int s0 = a.cu[b], s1 = a.cu[b + 1];
-    const int chunks = (s1 - s0 + C - 1) / C;
-    if (left < chunks) {
-      c0 = s0 + left * C;
-      t1 = s1;
-      break;
-    }
-    left -= chunks;
-  }
+  int b, c0, t1 = 0;                       // (the grid has a CTA for every chunk there can be)
+  memory_chunk(a.cu, a.B, blockIdx.x, b, c0, t1);
   if (c0 < 0) return;
   const int nt = min(C, t1 - c0);
   const int ldq = memory_chunk_ld(d);
@@ -305,6 +324,7 @@ memory_intra_kernel(const MemArgs a, double* __restrict__ gates) {
   float* sK = sQ + C * ldq;                          // [C][ldq]
   float* sV = sK + C * ldq;                          // [C][kMcSlab]
   float* sP = sV + C * kMcSlab;                      // [C][LP]
+  float* sW = sP + C * LP;                           // [C] a token's weight in the chunk's own sum
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // q and k of the chunk's tokens, copied asynchronously.  Rows beyond the chunk's last token stay as
   // they are: they reach only scores of rows that are not stored, or of keys after the row, which
@@ -424,7 +444,35 @@ memory_intra_kernel(const MemArgs a, double* __restrict__ gates) {
       stage_v(j0, width);
     }
     mem_cp_wait<0>();
+    if (j0 == 0 && tid < nt) sW[tid] = expf((float)(su[tid] - sU[nt - 1]));
     __syncthreads();                                   // the slab and the scores are in place
+    if (cs.S) {
+      const size_t at = (size_t)blockIdx.x * H + h;
+      if (j0 == 0)
+        for (int i = tid; i < d; i += kMcThreads) {
+          float sum = 0.f;
+#pragma unroll 8
+          for (int s = 0; s < nt; ++s) sum = fmaf(sW[s], sK[s * ldq + i], sum);
+          cs.n[at * d + i] = sum;
+        }
+      // rows 4 ig .. + 3, columns 4 si .. + 3 of the slab
+      for (int ig = ti; ig < d4 && 4 * si < width; ig += 16) {
+        float4 sum[4] = {zero4, zero4, zero4, zero4};
+#pragma unroll 4
+        for (int s = 0; s < nt; ++s) {
+          float4 k4 = *reinterpret_cast<const float4*>(sK + s * ldq + 4 * ig);
+          const float4 v4 = *reinterpret_cast<const float4*>(sV + s * kMcSlab + 4 * si);
+          scale4(k4, sW[s]);
+          fma4(sum[0], k4.x, v4);
+          fma4(sum[1], k4.y, v4);
+          fma4(sum[2], k4.z, v4);
+          fma4(sum[3], k4.w, v4);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          *reinterpret_cast<float4*>(cs.S + (at * d + 4 * ig + r) * e + j0 + 4 * si) = sum[r];
+      }
+    }
     if (4 * si >= width) continue;
     float4 acc[4];
 #pragma unroll
@@ -649,6 +697,184 @@ memory_carry_kernel(const MemArgs a, const double* __restrict__ gates, int nbuf)
   }
 }
 
+// The states before every chunk of a sequence, in place of the chunks' own sums; CTA x of a (sequence,
+// head) has 256 groups of four elements of S, the last one n.  The factors of 64 chunks at a time are
+// worked out together, the sums of eight are asked for at once.
+constexpr int kMsChunks = 64;
+
+__global__ void __launch_bounds__(kMcThreads)
+memory_scan_kernel(const MemArgs a, const double* __restrict__ gates, const ChunkSums cs) {
+  __shared__ double sM[kMsChunks], sX[kMsChunks], sU[kMsChunks], sF[kMsChunks];
+  __shared__ float keep[kMsChunks], add[kMsChunks];
+  const int tid = threadIdx.x, h = blockIdx.y, b = blockIdx.z, H = a.H, d = a.d, e = a.e;
+  const int t0 = a.cu[b], t1 = a.cu[b + 1];
+  if (t1 <= t0) return;
+  int base = 0;                            // the sequence's first chunk
+  for (int i = 0; i < b; ++i) base += (a.cu[i + 1] - a.cu[i] + kMcTokens - 1) / kMcTokens;
+  const int chunks = (t1 - t0 + kMcTokens - 1) / kMcTokens;
+  const bool of_n = blockIdx.x + 1 == gridDim.x;
+  const int groups = (of_n ? d : d * e) / 4, g = of_n ? tid : blockIdx.x * kMcThreads + tid;
+  const size_t step = (size_t)H * groups;
+  float4* sums = reinterpret_cast<float4*>(of_n ? cs.n : cs.S) + ((size_t)base * H + h) * groups + g;
+  float4* state = reinterpret_cast<float4*>(of_n ? a.n(b, h) : a.S(b, h)) + g;
+  const bool mine = g < groups;
+  float4 v = mine ? *state : make_float4(0.f, 0.f, 0.f, 0.f);
+  double m0 = (double)*a.m(b, h);
+  for (int first = 0; first < chunks; first += kMsChunks) {
+    const int n = min(kMsChunks, chunks - first);
+    if (tid < n) {
+      const int last = min(t0 + (first + tid + 1) * kMcTokens, t1) - 1;
+      sU[tid] = gates[((size_t)H + h) * a.T + last];
+      sF[tid] = gates[((size_t)2 * H + h) * a.T + last];
+    }
+    __syncthreads();
+    if (tid == 0) {
+      for (int c = 0; c < n; ++c) {
+        sM[c] = m0;
+        sX[c] = fmax(m0, sU[c]);
+        m0 = sF[c] + sX[c];
+      }
+    }
+    __syncthreads();
+    if (tid < n) {
+      keep[tid] = expf((float)(sM[tid] - sX[tid]));
+      add[tid] = expf((float)(sU[tid] - sX[tid]));
+      if (of_n) cs.m[(size_t)(base + first + tid) * H + h] = sM[tid];
+    }
+    __syncthreads();
+    for (int c = 0; c < n && mine; c += 8) {
+      float4 own[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c + i < n) own[i] = sums[(size_t)(first + c + i) * step];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (c + i >= n) break;
+        sums[(size_t)(first + c + i) * step] = v;
+        scale4(v, keep[c + i]);
+        fma4(v, add[c + i], own[i]);
+      }
+    }
+    __syncthreads();                       // the factors have been read
+  }
+  if (a.write_state && mine) *state = v;
+}
+
+inline size_t memory_read_smem(int d) {
+  return sizeof(float) * ((size_t)kMcTokens * memory_chunk_ld(d) + (size_t)d * kMcSlab + d);
+}
+
+// What the state before a chunk gives its read-outs, 64 columns at a time: rows ti + 16 r, columns
+// 4 si .. + 3 of the slab; n . q as well.
+__global__ void __launch_bounds__(kMcThreads)
+memory_read_kernel(const MemArgs a, const double* __restrict__ gates, const ChunkSums cs) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ float w0[kMcTokens], w1[kMcTokens];
+  constexpr int C = kMcTokens;
+  const int tid = threadIdx.x, h = blockIdx.y, H = a.H, d = a.d, e = a.e, d4 = d >> 2;
+  int b, c0, t1 = 0;
+  memory_chunk(a.cu, a.B, blockIdx.x, b, c0, t1);
+  if (c0 < 0) return;
+  const int nt = min(C, t1 - c0), ldq = memory_chunk_ld(d);
+  const size_t at = (size_t)blockIdx.x * H + h;
+  float* sQ = smem;                        // [C][ldq]
+  float* sS = sQ + C * ldq;                // [d][kMcSlab]
+  float* sN = sS + d * kMcSlab;            // [d]
+  for (int idx = tid; idx < nt * d4; idx += kMcThreads) {
+    const int tt = idx / d4, i4 = idx - tt * d4;
+    mem_cp16(sQ + tt * ldq + 4 * i4, a.q(c0 + tt, h) + 4 * i4);
+  }
+  for (int i = tid; i < d4; i += kMcThreads) mem_cp16(sN + 4 * i, cs.n + at * d + 4 * i);
+  auto stage = [&](int j0) {
+    for (int idx = tid; idx < d * (kMcSlab / 4); idx += kMcThreads) {
+      const int i = idx >> 4, jg = idx & 15;
+      if (j0 + 4 * jg < e)
+        mem_cp16(sS + i * kMcSlab + 4 * jg, cs.S + (at * d + i) * e + j0 + 4 * jg);
+    }
+    mem_cp_commit();
+  };
+  stage(0);
+  if (tid < nt) {
+    const double m0 = cs.m[at], U = gates[((size_t)H + h) * a.T + c0 + tid];
+    const double X = fmax(m0, U);
+    w0[tid] = expf((float)(m0 - X)) * a.q_scale;
+    w1[tid] = expf((float)(U - X));
+    a.ref[(size_t)(c0 + tid) * H + h] =
+        (float)(gates[((size_t)2 * H + h) * a.T + c0 + tid] + X);
+  }
+  const int ti = tid >> 4, si = tid & 15;
+  for (int j0 = 0; j0 < e; j0 += kMcSlab) {
+    const bool in = j0 + 4 * si < e;
+    float4 acc[4], old[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int t = ti + 16 * r;
+      acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      old[r] = acc[r];
+      if (in && t < nt)
+        old[r] = __ldcg(reinterpret_cast<const float4*>(
+            a.o_raw + (size_t)(c0 + t) * H * e + (size_t)h * e + j0 + 4 * si));
+    }
+    if (j0 > 0) {
+      __syncthreads();                     // the slab before has been read
+      stage(j0);
+    }
+    mem_cp_wait<0>();
+    __syncthreads();
+    if (j0 == 0) {                         // n . q of every row: four lanes a row
+      const int t = tid >> 2, part = tid & 3;
+      float sum = 0.f;
+      for (int i4 = part; i4 < d4; i4 += 4)
+        sum = dot4(*reinterpret_cast<const float4*>(sQ + t * ldq + 4 * i4),
+                   *reinterpret_cast<const float4*>(sN + 4 * i4), sum);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (part == 0 && t < nt) {
+        float* den = a.den + (size_t)(c0 + t) * H + h;
+        *den = w0[t] * sum + w1[t] * *den;
+      }
+    }
+    if (!in) continue;
+#pragma unroll 2
+    for (int i = 0; i < d; i += 4) {
+      float4 s4[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        s4[x] = *reinterpret_cast<const float4*>(sS + (i + x) * kMcSlab + 4 * si);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float4 q = *reinterpret_cast<const float4*>(sQ + (ti + 16 * r) * ldq + i);
+        fma4(acc[r], q.x, s4[0]);
+        fma4(acc[r], q.y, s4[1]);
+        fma4(acc[r], q.z, s4[2]);
+        fma4(acc[r], q.w, s4[3]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int t = ti + 16 * r;
+      if (t >= nt) continue;
+      scale4(old[r], w1[t]);
+      fma4(old[r], w0[t], acc[r]);
+      *reinterpret_cast<float4*>(a.o_raw + (size_t)(c0 + t) * H * e + (size_t)h * e + j0 + 4 * si) =
+          old[r];
+    }
+  }
+}
+
+int launch_memory_scan(const MemArgs& a, const double* gates, const ChunkSums& cs, cudaStream_t st) {
+  const size_t smem = memory_read_smem(a.d);
+  const long long parts = ((long long)a.d * a.e / 4 + kMcThreads - 1) / kMcThreads + 1;
+  if (parts > 0x7fffffffLL || a.B > 65535 || a.d > 4 * kMcThreads) return kBadArgument;
+  cudaError_t err = cudaFuncSetAttribute(memory_read_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return (int)err;
+  memory_scan_kernel<<<dim3((unsigned)parts, a.H, a.B), kMcThreads, 0, st>>>(a, gates, cs);
+  memory_read_kernel<<<dim3((unsigned)(a.T / kMcTokens + a.B), a.H), kMcThreads, smem, st>>>(a, gates,
+                                                                                             cs);
+  return launch_status();
+}
+
 template <int EC>
 int launch_memory_carry(const MemArgs& a, const double* gates, cudaStream_t st) {
   const int nbuf = memory_carry_smem(a.d, EC, 2) <= 220 * 1024 ? 2 : 1;
@@ -663,7 +889,7 @@ int launch_memory_carry(const MemArgs& a, const double* gates, cudaStream_t st) 
   return launch_status();
 }
 
-int launch_memory_intra(const MemArgs& a, double* gates, cudaStream_t st) {
+int launch_memory_intra(const MemArgs& a, double* gates, const ChunkSums& cs, cudaStream_t st) {
   const size_t smem = memory_intra_smem(a.d);
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(
@@ -673,7 +899,7 @@ int launch_memory_intra(const MemArgs& a, double* gates, cudaStream_t st) {
   // every sequence has at most one chunk that is not full
   const long long chunks = (long long)a.T / kMcTokens + a.B;
   if (chunks > 0x7fffffffLL) return kBadArgument;
-  memory_intra_kernel<<<dim3((unsigned)chunks, a.H), kMcThreads, smem, st>>>(a, gates);
+  memory_intra_kernel<<<dim3((unsigned)chunks, a.H), kMcThreads, smem, st>>>(a, gates, cs);
   return launch_status();
 }
 
@@ -730,18 +956,19 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 using namespace cretif;
 
 // gates: float64 [3, H, T] scratch; form 0 chooses, 1 token by token, 2 chunks (refused where the
-// sizes or addresses rule out 16-byte accesses).
+// sizes or addresses rule out 16-byte accesses), 3 chunks that are walked.  ws (may be null: chunks
+// are walked): float32 scratch, 16-byte aligned, of (T / 64 + B) H (d e + d + 2) numbers.
 extern "C" int cretif_matrix_memory(const float* proj, int ldp, const float* bias_i,
                                     const float* bias_f, float cap, float q_scale, float* state,
                                     long long state_stride, const int* cu_seqlens,
                                     const int* seq_slot, const int* tok_seq, int B, int H, int d,
                                     int e, const float* norm_w, float eps, float* o_raw, float* den,
                                     float* ref, double* gates, void* out, int out_dt, int ldo,
-                                    int write_state, int T, int form, void* stream) {
+                                    int write_state, int T, int form, float* ws, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (H <= 0 || d <= 0 || e <= 0 || !proj || !bias_i || !bias_f || !state || !norm_w || !o_raw ||
       !den || !ref || !(cap > 0.f) || ldp < 2 * H * (d + e) + 2 * H || ldo < H * e ||
-      state_stride < (long long)H * d * (e + 1) + H || form < 0 || form > 2)
+      state_stride < (long long)H * d * (e + 1) + H || form < 0 || form > 3)
     return kBadArgument;
   static int sm_count = 0;
   if (!sm_count) {
@@ -757,25 +984,40 @@ extern "C" int cretif_matrix_memory(const float* proj, int ldp, const float* bia
   bool done = false;
   // 64 tokens at a time where the step brings a sequence 16 tokens or more on average and the
   // sizes allow 16-byte accesses throughout; token by token otherwise.
-  if (form == 2 || (form == 0 && (long long)T >= 16LL * B)) {
+  if (form >= 2 || (form == 0 && (long long)T >= 16LL * B)) {
     const bool fits = d % 4 == 0 && e % 16 == 0 && ldp % 4 == 0 && state_stride % 4 == 0 && gates &&
                       aligned16(proj) && aligned16(state) && aligned16(o_raw) && H <= 65535 &&
                       memory_carry_smem(d, 16, 1) <= 220 * 1024 &&
                       memory_intra_smem(d) <= 220 * 1024;
     if (fits) {
-      rc = launch_memory_intra(a, gates, st);
+      // (the caller decides by giving the scratch: csrc/ops.py, memory_scans)
+      ChunkSums cs{nullptr, nullptr, nullptr};
+      if (ws && aligned16(ws) && form != 3 && d <= 4 * kMcThreads &&
+          memory_read_smem(d) <= 220 * 1024) {
+        const size_t slots = (size_t)(T / kMcTokens + B) * H;
+        cs.S = ws;
+        cs.n = cs.S + slots * d * e;
+        cs.m = reinterpret_cast<double*>(cs.n + slots * d);
+      }
+      rc = launch_memory_intra(a, gates, cs, st);
       if (rc != kOk) return rc;
+      if (cs.S) {
+        rc = launch_memory_scan(a, gates, cs, st);
+        if (rc != kOk) return rc;
+        done = true;
+      }
       // columns a CTA: as many as divide e and fit, fewer while the chip is not filled
       int ec = e % 64 == 0 ? 64 : e % 32 == 0 ? 32 : 16;
-      while (ec > 16 && (memory_carry_smem(d, ec, 1) > 220 * 1024 ||
+      while (!done && ec > 16 && (memory_carry_smem(d, ec, 1) > 220 * 1024 ||
                          (long long)B * H * (e / ec) < (long long)sm_count))
         ec /= 2;
-      rc = ec == 64   ? launch_memory_carry<64>(a, gates, st)
+      rc = done       ? rc
+           : ec == 64 ? launch_memory_carry<64>(a, gates, st)
            : ec == 32 ? launch_memory_carry<32>(a, gates, st)
                       : launch_memory_carry<16>(a, gates, st);
       if (rc != kOk) return rc;
       done = true;
-    } else if (form == 2) {
+    } else if (form >= 2) {
       return kBadArgument;
     }
   }

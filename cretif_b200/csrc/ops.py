@@ -784,6 +784,16 @@ def retention_recurrence(prep, v, decay, state, cu_seqlens, seq_slot, B: int, H:
         "retention_recurrence")
 
 
+def memory_scans(T: int, B: int, H: int) -> bool:
+    """Whether a step's chunks of the matrix memory are scanned (matrix_memory.cu) instead of walked:
+    sequences of 256 tokens or more on average, while the walk's CTAs (a few a sequence and head)
+    leave the chip idle.  Microseconds, walked and scanned, 9 heads of 64 x 64: one sequence of 1,601
+    tokens 129 and 42, of 256 33 and 26, of 64 20 and 24, sixteen of 512 162 and 151; 16 heads of
+    128 x 128: one of 1,601 210 and 152, four of 1,024 360 and 329, eight 600 and 606, 32 of 256 627
+    and 668."""
+    return T >= 256 * B and B * H < 128
+
+
 def matrix_memory(proj, bias_i, bias_f, cap: float, q_scale: float, state, cu_seqlens, seq_slot,
                   tok_seq, B: int, H: int, d: int, e: int, norm_w, eps: float, out,
                   write_state: bool = True, form: str = "auto") -> None:
@@ -792,8 +802,9 @@ def matrix_memory(proj, bias_i, bias_f, cap: float, q_scale: float, state, cu_se
     per-head RMS norm times ``norm_w`` [H·e] times sigmoid of the gate columns -> ``out`` [T, H·e].
     ``proj`` rows (float32): [q | k | v | gate | input gate (H) | forget gate (H)].  ``form``:
     ``"token"`` walks the tokens one by one, ``"chunk"`` takes 64 at a time as matrix products
-    (refused where sizes or addresses rule out 16-byte accesses), ``"auto"`` takes chunks where the
-    step brings 16 tokens a sequence or more and they are allowed."""
+    (refused where sizes or addresses rule out 16-byte accesses), ``"walk"`` takes chunks one after
+    the other, ``"auto"`` takes chunks where the step brings 16 tokens a sequence or more and they
+    are allowed."""
     _need(proj, "proj", torch.float32, 2); _need(state, "state", torch.float32, 2)
     _need(out, "out", dim=2)
     for name, t, n in (("bias_i", bias_i, H), ("bias_f", bias_f, H), ("norm_w", norm_w, H * e)):
@@ -809,15 +820,19 @@ def matrix_memory(proj, bias_i, bias_f, cap: float, q_scale: float, state, cu_se
         raise KernelError("matrix_memory: the sizes do not fit")
     n_o = T * H * e
     scratch = torch.empty(n_o + 2 * T * H, dtype=torch.float32, device=proj.device)
-    chunks = form == "chunk" or (form == "auto" and T >= 16 * B)
+    chunks = form in ("chunk", "walk") or (form == "auto" and T >= 16 * B)
     gates = torch.empty(3 * H * T, dtype=torch.float64, device=proj.device) if chunks else None
+    scan = chunks and form != "walk" and memory_scans(T, B, H)
+    ws = (torch.empty((T // 64 + B) * H * (d * e + d + 2), dtype=torch.float32, device=proj.device)
+          if scan else None)
     _check(lib().cretif_matrix_memory(
         _p(proj), _rows(proj, "proj"), _p(bias_i), _p(bias_f), ctypes.c_float(cap),
         ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(cu_seqlens),
         _p(seq_slot), _p(tok_seq), B, H, d, e, _p(norm_w), ctypes.c_float(eps), _p(scratch),
         _p(scratch[n_o:]), _p(scratch[n_o + T * H:]), _p(gates), _p(out), _dt(out),
-        _rows(out, "out"), int(write_state), T, {"auto": 0, "token": 1, "chunk": 2}[form],
-        _stream()), "matrix_memory", kernels=3 if chunks else 2)
+        _rows(out, "out"), int(write_state), T,
+        {"auto": 0, "token": 1, "chunk": 2, "walk": 3}[form], _p(ws), _stream()),
+        "matrix_memory", kernels=(4 if scan else 3) if chunks else 2)
 
 
 def state_space(proj, conv_w, conv_b, a_log, dt_bias, d_skip, state, inputs_at: int, cu_seqlens,

@@ -1,0 +1,41 @@
+"""The matrix memory's chunks scanned against chunks walked: the same sums of the same terms in
+another order, over lengths at the edges of a chunk and beyond the scan's 64 chunks at a time."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,d,e,lens", [(2, 64, 64, (64 * 66 + 5, 1, 64, 63)), (3, 20, 48, (65, 700)),
+                                        (1, 256, 80, (129, 128)), (9, 128, 128, (40, 24, 200))])
+@pytest.mark.parametrize("write_state", [True, False])
+def test_scan_and_walk(H, d, e, lens, write_state):
+    """Read-outs are normed, so they are compared by their 2-norm (both forms sum in 32 bits:
+    2^-24 times the square root of the terms, a thousand at most, and the norm's gain); states by
+    theirs."""
+    from cretif_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    T, B, width = sum(lens), len(lens), -(-(2 * H * (d + e) + 2 * H) // 4) * 4
+    proj = torch.randn(T, width, generator=gen, device="cuda")
+    proj[:, -2 * H:] *= 3.0
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    seq = torch.repeat_interleave(torch.arange(B, **i32), torch.tensor(lens, device="cuda")).int()
+    slots = torch.arange(B, 0, -1, **i32)
+    bias, norm_w = torch.zeros(H, device="cuda"), torch.ones(H * e, device="cuda")
+    start = torch.randn(B + 2, -(-(H * (d * (e + 1) + 1)) // 4) * 4, generator=gen, device="cuda")
+    outs, states = [], []
+    for form in ("walk", "chunk"):
+        state, out = start.clone(), torch.empty(T, H * e, device="cuda")
+        kept, ops.memory_scans = ops.memory_scans, lambda *_: True
+        try:
+            ops.matrix_memory(proj, bias, bias, 12.0, d ** -0.5, state, cu, slots, seq, B, H, d, e,
+                              norm_w, 1e-6, out, write_state=write_state, form=form)
+        finally:
+            ops.memory_scans = kept
+        outs.append(out.double())
+        states.append(state.double())
+        assert torch.equal(state[0], start[0]) and torch.equal(state[B + 1], start[B + 1])
+    assert bool(torch.isfinite(outs[0]).all())
+    assert (outs[0] - outs[1]).norm() <= 1e-4 * outs[0].norm()
+    assert (states[0] - states[1]).norm() <= 2e-6 * states[0].norm()
