@@ -25,6 +25,7 @@ import array
 import collections
 import contextlib
 import gc
+import threading
 from typing import Dict, Optional, Sequence, Tuple, Union
 
 import numpy as np
@@ -97,20 +98,30 @@ class _PinnedRing:
         self.events[i].record()
 
 
+_captures = threading.Lock()
+_captures_open = [0, False]          # captures that run in any thread; whether the collector was on
+
+
 @contextlib.contextmanager
 def capturing(graph, pool, stream):
     """Capture into ``graph`` on ``stream``, which is current, with the garbage collector held
     off: an engine that is in a reference cycle holds graphs, and destroying one of them while a
     capture runs is an unsafe call that ends the capture (``cudaErrorStreamCaptureInvalidated``).
+    The collector is the whole process's, so it goes on again with the last capture of all threads.
     """
-    collects = gc.isenabled()
-    gc.disable()
+    with _captures:
+        if not _captures_open[0]:
+            _captures_open[1] = gc.isenabled()
+            gc.disable()
+        _captures_open[0] += 1
     try:
         with torch.cuda.graph(graph, pool=pool, stream=stream):
             yield
     finally:
-        if collects:
-            gc.enable()
+        with _captures:
+            _captures_open[0] -= 1
+            if not _captures_open[0] and _captures_open[1]:
+                gc.enable()
 
 
 def parse_dtype(dtype) -> torch.dtype:
