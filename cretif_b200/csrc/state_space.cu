@@ -531,7 +531,10 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
   constexpr int NR = kScThreads / CG;      // threads along the rows
   constexpr int RT = C / NR;               // read-out rows a thread
   const int tid = threadIdx.x, H = a.H, N = a.N, e = a.e;
-  const int b = sequence_by_length(a.cu, a.B, blockIdx.z), h = blockIdx.x, col0 = blockIdx.y * EC;
+  // the grid: heads, slices of columns, sequences (the slowest)
+  const unsigned part = blockIdx.x / (unsigned)H, slices = (unsigned)(e / EC);
+  const int h = (int)(blockIdx.x - part * H), col0 = (int)(part % slices) * EC;
+  const int b = sequence_by_length(a.cu, a.B, (int)(part / slices));
   const int t0 = a.cu[b], t1 = a.cu[b + 1];
   if (t1 <= t0) return;
   const int ldq = ssm_chunk_ld(N);
@@ -703,8 +706,9 @@ int launch_ssm_carry(const SsmArgs& a, cudaStream_t st) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
-  if (a.B > 65535) return kBadArgument;
-  kern<<<dim3(a.H, a.e / EC, a.B), kScThreads, smem, st>>>(a, nbuf);
+  const long long ctas = (long long)a.B * a.H * (a.e / EC);
+  if (ctas > 0x7fffffffLL) return kBadArgument;
+  kern<<<(unsigned)ctas, kScThreads, smem, st>>>(a, nbuf);
   return launch_status();
 }
 

@@ -1,0 +1,36 @@
+"""Steps of more sequences than a grid's second and third dimension take (65,535)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+B = 65537
+I32 = dict(dtype=torch.int32, device="cuda")
+
+
+def _rand(*shape, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*shape, generator=gen, device="cuda")
+
+
+def test_mamba_chunks():
+    """A token a sequence, by chunks and token by token: the same 32-bit terms, sums of at most
+    four of them, then a norm."""
+    from cretif_b200.csrc import ops
+    H, G, N, e, taps = 1, 1, 4, 16, 2
+    C = H * e + 2 * G * N
+    proj = _rand(B, -(-(H * e + C + H) // 4) * 4)
+    conv_w, conv_b = _rand(taps, C, seed=1), _rand(C, seed=2)
+    start = _rand(B, H * N * e + C * (taps - 1), seed=3)
+    every = torch.arange(B, **I32)
+    cu = torch.arange(B + 1, **I32)
+    got = []
+    for form in ("chunk", "token"):
+        state, out = start.clone(), torch.empty(B, H * e, device="cuda")
+        ops.state_space(proj, conv_w, conv_b, torch.zeros(H, device="cuda"),
+                        torch.zeros(H, device="cuda"), torch.ones(H, device="cuda"), state, H * N * e,
+                        cu, every, every, B, H, G, N, e, 1, torch.ones(H * e, device="cuda"), 1e-5,
+                        out, save_inputs=True, form=form)
+        got.append((out, state))
+    for a, b in zip(*got):
+        assert (a - b).norm() <= 1e-6 * b.norm()
