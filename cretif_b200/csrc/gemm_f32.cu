@@ -5,26 +5,31 @@
 // operand pairs as it lies, and a sum is kept as two chains (even and odd k) that meet at the
 // end, so no operand is ever duplicated or moved.
 //
-// * gemm_f32_few (M <= kFewRows): a step of few tokens is bound by reading W once.  A warp owns
-//   kR = 4 rows of W and 1, 2, 4 or 8 rows of A; its lanes stride k by 16-byte loads (512 bytes of
-//   a W row an instruction); WK warps of a CTA share a row group's k range when N alone gives
-//   too few warps to keep loads in flight.  WK depends on N and K only, so a row's result does
-//   not depend on how many rows are in the call.  More than 8 rows: the row tiles of one group
-//   of W rows are neighbours in the grid and read it from L2.
+// Both sum an output in one order, whatever M and N are, so that a row's result does not depend on how
+// many rows the call has: a slab of 32 k in two chains of its own, the slabs with the same number
+// mod 4 in ascending order, then the four totals in theirs.
+//
+// * gemm_f32_few: a step of few tokens is bound by reading W once, and small matrices by the latency of
+//   that.  A CTA has NT columns and MT rows, a warp the slabs with one number mod 4, U = 32 / NT at a
+//   time: a lane sums one slab of one column for all MT rows.  W and A come through a cp.async ring of
+//   the warp's own (no barrier before the totals meet), slabs 36 floats a row so that neighbouring
+//   columns read different banks.  Fewer columns a CTA put more CTAs and shorter chains on a small
+//   matrix; they read A more often.  More than 8 rows: the row tiles of one group of columns are
+//   neighbours in the grid and read W from L2.
 // * gemm_f32_tile: WM x WN warps, 32 x 32 outputs a warp (8 x 4 a thread: 12 shared 16-byte
-//   loads feed 64 two-wide FMAs), slabs of 32 k through a three-stage cp.async ring with rows of
-//   36 floats (eight consecutive rows lie in different banks).  KS > 1: the warps of a CTA take
-//   the slabs of one 32 x 32 tile in turn and their sums meet in shared memory; that is for
-//   grids of so few tiles that 64 x 64 ones would leave SMs idle.
-//   A slab's 32 products are summed in two chains of their own before they join the running sum.
+//   loads feed 64 two-wide FMAs), slabs through a cp.async ring with rows of 36 floats (eight
+//   consecutive rows lie in different banks).  KS = 4: the warps of a CTA take the slabs of one
+//   32 x 32 tile in turn and the totals meet in shared memory; that is for grids of so few tiles that
+//   64 x 64 ones would leave SMs idle.  KS = 1 visits the slabs 0, 4, 8, .., 1, 5, .. for the same order.
 //
 // Measured beside the 64 x 64 kernel of gemm_simt.cu (one B200, weights not in L2, us before ->
-// now; M x N x K).  Few rows: 1 x 49152 x 576 154 -> 22 (5.2 TB/s), 8 x 49152 x 576 157 -> 37,
-// 3 x 576 x 1536 111 -> 3.8, 3 x 3072 x 576 43 -> 7.1, 8 x 2048 x 8192 589 -> 21.  Tiles:
-// 578 x 3072 x 576 112 -> 72, 2048 x 3072 x 576 302 -> 189, 2048 x 16384 x 2048 5406 -> 3271
-// (42 TFLOP/s of the 74 that 128 FMA lanes an SM give); 8 x 8 outputs a thread need 255 registers
-// and are no faster.  The error against 64 bits is 0.6 to 0.8 of the old kernel's (8.6e-8 and
-// 1.0e-7 against 1.3e-7 at K = 576).
+// now; M x N x K).  Few rows: 1 x 49152 x 576 154 -> 21 (5.3 TB/s), 8 x 49152 x 576 157 -> 31,
+// 3 x 576 x 1536 111 -> 4.0, 3 x 3072 x 576 43 -> 4.5, 8 x 2048 x 8192 589 -> 31, 8 x 16384 x 2048 34.  Tiles:
+// 578 x 3072 x 576 112 -> 67, 2048 x 3072 x 576 302 -> 196, 2048 x 16384 x 2048 5406 -> 3361
+// (41 TFLOP/s of the 74 that 128 FMA lanes an SM give); 8 x 8 outputs a thread need 255 registers
+// and are no faster.  Lanes that take pieces of 8 k of a row as 16-byte loads lie (no shared memory, and
+// sums the tiles can follow piece by piece) cost the tiles a third; a block barrier a chunk of slabs
+// cost the few rows a third.
 #include "api.h"
 #include "common.cuh"
 #include "gemm_f32.h"
@@ -32,94 +37,8 @@
 namespace cretif {
 
 constexpr int kFewRows = 64;
-constexpr int kR = 4;                 // rows of W a warp
-constexpr int kFewWarps = 8;
-
-// The sums of NV values over a warp's lanes; the lane whose number's top bits are i gets value i
-// (NV = 32: lane i).  NV - 1 + log2(32 / NV) shuffles.
-template <int NV>
-__device__ __forceinline__ float warp_sums(float (&v)[NV], int lane) {
-  int off = 16;
-#pragma unroll
-  for (int n = NV / 2; n > 0; n >>= 1, off >>= 1) {
-    const bool up = lane & off;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float send = up ? v[i] : v[i + n];
-      const float keep = up ? v[i + n] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  float r = v[0];
-  for (; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-  return r;
-}
-
-template <int MT>
-__global__ void __launch_bounds__(kFewWarps * 32)
-gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                    int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int WK) {
-  dependent_begin();
-  constexpr int NV = kR * MT;
-  __shared__ float part[kFewWarps][NV];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int group = warp / WK, wk = warp - group * WK;
-  const int n0 = ((int)blockIdx.y * (kFewWarps / WK) + group) * kR;
-  const int m0 = (int)blockIdx.x * MT;
-  const float* wp[kR];
-  const float* ap[MT];
-#pragma unroll
-  for (int r = 0; r < kR; ++r) wp[r] = W + (size_t)min(n0 + r, N - 1) * ldw;
-#pragma unroll
-  for (int m = 0; m < MT; ++m) ap[m] = A + (size_t)min(m0 + m, M - 1) * lda;
-  float2 acc[kR][MT];
-#pragma unroll
-  for (int r = 0; r < kR; ++r)
-#pragma unroll
-    for (int m = 0; m < MT; ++m) acc[r][m] = make_float2(0.f, 0.f);
-  // rows beyond N or M read the last row's numbers; their sums are not stored
-#pragma unroll 2
-  for (int k = wk * 128 + lane * 4; k < K; k += WK * 128) {
-    float4 w[kR];
-#pragma unroll
-    for (int r = 0; r < kR; ++r) w[r] = __ldg(reinterpret_cast<const float4*>(wp[r] + k));
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const float4 a = *reinterpret_cast<const float4*>(ap[m] + k);
-#pragma unroll
-      for (int r = 0; r < kR; ++r) {
-        acc[r][m] = __ffma2_rn(make_float2(a.x, a.y), make_float2(w[r].x, w[r].y), acc[r][m]);
-        acc[r][m] = __ffma2_rn(make_float2(a.z, a.w), make_float2(w[r].z, w[r].w), acc[r][m]);
-      }
-    }
-  }
-  float v[NV];
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int r = 0; r < kR; ++r) v[m * kR + r] = acc[r][m].x + acc[r][m].y;
-  float s = warp_sums(v, lane);
-  constexpr int kPer = 32 / NV;               // lanes that hold the same sum
-  const int at = lane / kPer;
-  if (WK > 1) {
-    if (lane % kPer == 0) part[warp][at] = s;
-    __syncthreads();
-    if (wk != 0) return;
-    s = 0.f;
-    for (int i = 0; i < WK; ++i) s += part[warp + i][at];
-  }
-  const int m = m0 + at / kR, n = n0 + at % kR;
-  if (lane % kPer == 0 && m < M && n < N) {
-    float* c = C + (size_t)m * ldc + n;
-    *c = accumulate ? *c + s : s;
-  }
-}
-
 constexpr int kSlab = 32;             // k's a slab
-constexpr int kRow = kSlab + 4;       // floats a row of it takes in shared memory
-// stages of the ring: a CTA that shares a slab range among its warps takes two (74 KB, so that
-// three of them share an SM and hide each other's loads), the other three
-constexpr int ring_of(int KS) { return KS > 1 ? 2 : 3; }
+constexpr int kRow = kSlab + 4;       // floats it takes in shared memory
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool real) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -127,26 +46,146 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool real) 
                "r"(real ? 16 : 0) : "memory");
 }
 
+// Steps a warp's ring holds (a step: 32 / NT slabs).
+constexpr int few_depth(int NT) { return NT <= 16 ? 3 : 4; }
+// Floats of a slab in it: MT rows of A, NT of W; where two slabs meet in one shared-memory phase (four
+// columns) they lie 16 banks apart.
+constexpr int few_slab(int MT, int NT) {
+  return (MT + NT) * kRow + (NT == 4 ? (48 - 4 * (MT + NT) % 32) % 32 : 0);
+}
+constexpr int few_smem(int MT, int NT) {
+  return 4 * (4 * few_depth(NT) * (32 / NT) * few_slab(MT, NT) + 4 * MT * NT);
+}
+
+template <int MT, int NT>
+__global__ void __launch_bounds__(128)
+gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+                    int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int m_tiles) {
+  dependent_begin();
+  constexpr int D = few_depth(NT), U = 32 / NT, kOne = few_slab(MT, NT), kRows = (MT + NT + 3) / 4;
+  static_assert(U * NT == 32, "a lane has a column of one of U slabs");
+  extern __shared__ __align__(16) float sm[];
+  const int ks = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned bn = blockIdx.x / (unsigned)m_tiles;
+  const int n0 = (int)bn * NT, m0 = (int)(blockIdx.x - bn * m_tiles) * MT;
+  const int slabs = (K + kSlab - 1) / kSlab, mine = (slabs - ks + 3) / 4, steps = (mine + U - 1) / U;
+  float* ring = sm + ks * D * U * kOne;
+  float* totals = sm + 4 * D * U * kOne;           // [4][MT][NT]
+  // a lane copies piece lane & 7 of every fourth row: NT of W, then MT of A (rows beyond N or M are
+  // the last row again; their sums are not stored)
+  const int piece = (lane & 7) * 4, row0 = lane >> 3;
+  const float* src[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int row = row0 + 4 * i;
+    src[i] = row < NT ? W + (size_t)min(n0 + row, N - 1) * ldw
+                      : A + (size_t)min(m0 + row - NT, M - 1) * lda;
+  }
+  auto fetch = [&](int step) {
+    if (step < steps) {
+      float* st = ring + step % D * U * kOne;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = (ks + 4 * (step * U + u)) * kSlab + piece;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+          if ((MT + NT) % 4 == 0 || row0 + 4 * i < MT + NT)
+            copy16(st + u * kOne + (row0 + 4 * i) * kRow + piece, src[i] + (k < K ? k : 0), k < K);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int j = 0; j < D - 1; ++j) fetch(j);
+  const int tx = lane % NT, u = lane / NT;
+  float acc[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
+    __syncwarp();               // this step's slabs are there, the last one's are read no more
+    fetch(step + D - 1);
+    const float* one = ring + (step % D * U + u) * kOne;
+    float2 part[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) part[m] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < kSlab; k += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(one + tx * kRow + k);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float4 a = *reinterpret_cast<const float4*>(one + (NT + m) * kRow + k);
+        part[m] = __ffma2_rn(make_float2(a.x, a.y), make_float2(w.x, w.y), part[m]);
+        part[m] = __ffma2_rn(make_float2(a.z, a.w), make_float2(w.z, w.w), part[m]);
+      }
+    }
+    // (slabs beyond K are zero)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const float sum = part[m].x + part[m].y;
+      if (U == 1) {
+        acc[m] += sum;
+      } else {
+#pragma unroll
+        for (int v = 0; v < U; ++v) acc[m] += __shfl_sync(0xffffffffu, sum, v * NT + tx);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (u == 0) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) totals[(ks * MT + m) * NT + tx] = acc[m];
+  }
+  __syncthreads();
+  for (int o = threadIdx.x; o < MT * NT; o += 128) {
+    const int m = m0 + o / NT, n = n0 + o % NT;
+    float sum = totals[o];
+#pragma unroll
+    for (int g = 1; g < 4; ++g) sum += totals[g * MT * NT + o];
+    if (m < M && n < N) {
+      float* c = C + (size_t)m * ldc + n;
+      *c = accumulate ? *c + sum : sum;
+    }
+  }
+}
+
+// stages of the ring: a CTA that shares a slab range among its warps takes two (74 KB, so that
+// three of them share an SM and hide each other's loads), the other three
+constexpr int ring_of(int KS) { return KS > 1 ? 2 : 3; }
+
 template <int WM, int WN, int KS>
 __global__ void __launch_bounds__(32 * WM * WN * KS)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                     int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
+                     int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int n_tiles) {
   constexpr int BM = 32 * WM, BN = 32 * WN, kThreads = 32 * WM * WN * KS;
   constexpr int kStage = KS * (BM + BN) * kRow, kRing = ring_of(KS);       // (floats)
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ks = warp / (WM * WN), wm = (warp % (WM * WN)) / WN, wn = warp % WN;
   const int ty = lane >> 3, tx = lane & 7;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int rounds = (K + KS * kSlab - 1) / (KS * kSlab);
+  const unsigned bm = blockIdx.x / (unsigned)n_tiles;
+  const int m0 = (int)bm * BM, n0 = (int)(blockIdx.x - bm * n_tiles) * BN;
+  const int slabs = (K + kSlab - 1) / kSlab, quarter = (slabs + 3) / 4;
+  const int rounds = KS == 1 ? slabs : quarter;
+  // KS == 1: the slab of a round; slabs with 0 mod 4 first (`longer`: how many mod 4 have `quarter` slabs)
+  const int longer = slabs - 4 * (quarter - 1);
+  auto slab_of = [&](int round, bool* last = nullptr) {
+    const int of_longer = longer * quarter;
+    const bool in_longer = round < of_longer;
+    const int n = in_longer ? quarter : quarter - 1, at = in_longer ? round : round - of_longer;
+    const int g = at / n, i = at - g * n;
+    if (last) *last = i == n - 1;
+    return 4 * i + g + (in_longer ? 0 : longer);
+  };
 
   auto fetch = [&](int round) {
     float* st = sm + (round % kRing) * kStage;
+    const int slab0 = KS == 1 ? slab_of(round) : round * KS;
     // KS slabs of BM rows of A and BN rows of W, eight 16-byte pieces a row
 #pragma unroll
     for (int i = tid; i < KS * (BM + BN) * 8; i += kThreads) {
       const int piece = i & 7, row = (i >> 3) % (BM + BN), s = (i >> 3) / (BM + BN);
-      const int k = (round * KS + s) * kSlab + piece * 4;
+      const int k = (slab0 + s) * kSlab + piece * 4;
       const bool is_a = row < BM;
       const int at = is_a ? m0 + row : n0 + row - BM;
       const bool real = k < K && at < (is_a ? M : N);
@@ -155,11 +194,15 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     }
   };
 
-  float acc[8][4];
+  // KS == 1: the four totals are added one after the other into `whole`
+  float acc[8][4], whole[KS == 1 ? 8 : 1][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) {
+      acc[i][j] = 0.f;
+      if (KS == 1) whole[i][j] = 0.f;
+    }
 #pragma unroll
   for (int r = 0; r < kRing - 1; ++r) {
     if (r < rounds) fetch(r);
@@ -196,6 +239,19 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j].x + part[i][j].y;
+    if (KS == 1) {
+      bool last;
+      slab_of(round, &last);
+      if (last) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            whole[i][j] += acc[i][j];
+            acc[i][j] = 0.f;
+          }
+      }
+    }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (KS > 1) {
@@ -226,18 +282,25 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
       const int n = n0 + wn * 32 + tx + 8 * j;
       if (n >= N) continue;
       float* c = C + (size_t)m * ldc + n;
-      *c = accumulate ? *c + acc[i][j] : acc[i][j];
+      const float v = KS == 1 ? whole[KS == 1 ? i : 0][j] : acc[i][j];
+      *c = accumulate ? *c + v : v;
     }
   }
 }
 
-template <int MT>
+
+template <int MT, int NT>
 static int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                      int ldc, int accumulate, int WK, cudaStream_t st) {
-  const int rows = kR * (kFewWarps / WK);               // of W, a CTA
-  const dim3 grid((M + MT - 1) / MT, (N + rows - 1) / rows);
-  launch_dependent(gemm_f32_few_kernel<MT>, grid, kFewWarps * 32, 0, st, A, W, C, M, N, K, lda, ldw,
-                   ldc, accumulate, WK);
+                      int ldc, int accumulate, cudaStream_t st) {
+  constexpr int smem = few_smem(MT, NT);
+  auto kern = gemm_f32_few_kernel<MT, NT>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  const int m_tiles = (M + MT - 1) / MT;
+  launch_dependent(kern, (unsigned)((N + NT - 1) / NT) * m_tiles, 128, smem, st, A, W, C, M, N, K, lda,
+                   ldw, ldc, accumulate, m_tiles);
   return launch_status();
 }
 
@@ -249,37 +312,48 @@ static int launch_tile(const float* A, const float* W, float* C, int M, int N, i
   auto kern = gemm_f32_tile_kernel<WM, WN, KS>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  kern<<<grid, 32 * WM * WN * KS, smem, st>>>(A, W, C, M, N, K, lda, ldw, ldc, accumulate);
+  const int n_tiles = (N + BN - 1) / BN;
+  kern<<<(unsigned)n_tiles * ((M + BM - 1) / BM), 32 * WM * WN * KS, smem, st>>>(
+      A, W, C, M, N, K, lda, ldw, ldc, accumulate, n_tiles);
   return launch_status();
 }
 
 bool gemm_f32_takes(const void* A, const void* W, int M, int N, int K, int lda, int ldw) {
-  // 16-byte loads of whole rows; the grid's second dimension
+  // 16-byte loads of whole rows
   return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 &&
          ((uintptr_t)W & 15) == 0 && N <= 4 * 65535 && M <= 32 * 65535;
 }
 
 int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
              int accumulate, cudaStream_t st) {
-  // 17 to 64 rows: the few-row body reads W once per eight rows, the tiles once; the tiles need
-  // enough columns to fill the chip (24 x 49152 x 576: 80 against 64 us, 64 x 49152 x 576: 199 against
-  // 110, 64 x 576 x 576: 8.4 against 8.7).
-  if (M <= 16 || (M <= kFewRows && M * N <= 64 * 576)) {
-    // Enough warps for W's loads to be in flight everywhere (16 an SM); a warp of a shared k
-    // range keeps at least one piece of 128.
-    int WK = 1;
-    while (WK < kFewWarps && (long long)((N + kR - 1) / kR) * WK < 148 * 16 && WK * 128 < K) WK *= 2;
-    if (M == 1) return launch_few<1>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, WK, st);
-    if (M == 2) return launch_few<2>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, WK, st);
-    if (M <= 4) return launch_few<4>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, WK, st);
-    return launch_few<8>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, WK, st);
+  auto tiles = [&](int m, int n) { return ((long long)(M + m - 1) / m) * ((N + n - 1) / n); };
+  // The few-row body reads W once per eight rows, the tiles once; the tiles need enough columns to fill
+  // the chip (us, few rows and tiles: 24 x 49152 x 576 85 and 57, 64 x 3072 x 576 17 and 14,
+  // 24 x 3072 x 576 6.7 and 8.8, 64 x 576 x 576 5.0 and 8.8).
+  if (M <= 8 || (M <= kFewRows && tiles(8, 32) <= 512)) {
+    // 32 columns a CTA while that leaves enough CTAs, more of them for a long K, whose chains are the
+    // time then (3 x 3072 x 576: 4.5 us, 6.3 with 8 columns; 3 x 576 x 1536: 7.1 and 4.0; 8 x 2048 x 8192:
+    // 43 and 31); 8 rows only where half as many CTAs still fill the chip (8 x 576 x 1536: 6.8 us, 4.3
+    // as two times four).
+    const int wide = K > 4096 ? 512 : 96;
+    if (M == 1) {
+      if (tiles(1, 32) >= wide) return launch_few<1, 32>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+      if (tiles(1, 8) >= 96) return launch_few<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+      return launch_few<1, 4>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+    }
+    if (M == 2) {
+      if (tiles(2, 32) >= wide) return launch_few<2, 32>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+      if (tiles(2, 8) >= 96) return launch_few<2, 8>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+      return launch_few<2, 4>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+    }
+    if (M > 4 && tiles(8, 32) >= (wide > kSmCount ? wide : kSmCount))
+      return launch_few<8, 32>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+    if (tiles(4, 32) >= wide) return launch_few<4, 32>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
+    return launch_few<4, 8>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
   }
-  // The tile whose waves of 148 SMs cost less: a 64 x 64 tile is four 32 x 32 ones, and about a
+  // The tile whose waves of SMs cost less: a 64 x 64 tile is four 32 x 32 ones, and about a
   // seventh cheaper than those (fewer shared-memory fills a product).
-  auto waves = [&](int b) {
-    return ((long long)((M + b - 1) / b) * ((N + b - 1) / b) + 147) / 148;
-  };
+  auto waves = [&](int b) { return (tiles(b, b) + kSmCount - 1) / kSmCount; };
   if (waves(32) * 8 < waves(64) * 4 * 7)
     return launch_tile<1, 1, 4>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
   return launch_tile<2, 2, 1>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);

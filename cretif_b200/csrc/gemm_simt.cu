@@ -8,7 +8,8 @@
 // cretif_gemm_simt_batched runs `batch` such products in one launch, product z on operands
 // offset by z times an element stride each (per-head matrices on slices of the rows).
 // Any M, N, K; each output sums its products in ascending k, slab of 16 by slab of 16, whatever
-// M is, so a row's result does not depend on how many other rows are in the call.
+// M is, so a row's result does not depend on how many other rows are in the call.  (gemm_f32.cu, which
+// takes 32-bit rows that are 16-byte aligned, has another order, also the same for every M.)
 #include "api.h"
 #include "common.cuh"
 #include "gemm_f32.h"
