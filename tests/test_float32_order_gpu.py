@@ -1,9 +1,11 @@
-"""The 32-bit product: a row's bits do not depend on what else is in the call, whichever of the fast
-bodies takes it, and the result is the 64-bit one within 32 bits."""
+"""The 32-bit product and the attention of heads of 64: a row's bits do not depend on what else is in
+the call, whichever of the fast bodies takes it, and the result is the 64-bit one within 32 bits."""
+import math
+
 import pytest
 import torch
 
-from test_kernels_gpu import DEV, close, ops, rnd  # noqa: F401
+from test_kernels_gpu import DEV, ToyCache, close, ops, rnd  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -25,3 +27,117 @@ def test_a_row_of_the_product_does_not_depend_on_the_others(ops, N, K):  # noqa:
         assert torch.equal(c, whole[:m]), m
         ops.gemm_simt(a[700 - m:], w, c)
         assert torch.equal(c, whole[700 - m:]), m
+
+
+def _attend(ops, cache, new, cached, qs, nh, nkv, window, kw, use=None):  # noqa: F811
+    """Rows of the sequences ``use`` (all by default) in one step; a sequence's queries are
+    qs[b][cached .. cached + new - 1]."""
+    use = list(range(len(new))) if use is None else use
+    as_ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos = [cached[b] + i for b in use for i in range(new[b])]
+    seq = [i for i, b in enumerate(use) for _ in range(new[b])]
+    q = torch.cat([qs[b][cached[b]:cached[b] + new[b]] for b in use])
+    out = torch.empty_like(q)
+    ops.attn_simt(q, out, cache.k, cache.v, cache.table, as_ints(pos), as_ints(seq),
+                  cache.seq_slot[use].contiguous(), nh, nkv, 64, 0.17, window, 64,
+                  news=[new[b] for b in use], **kw)
+    return list(out.split([new[b] for b in use]))
+
+
+@pytest.mark.parametrize("nh,nkv", [(3, 1), (2, 2)])
+@pytest.mark.parametrize("window,extras", [(0, ""), (40, "sink"), (-48, "slope"), (0, "sink,slope")])
+def test_a_token_of_the_attention_does_not_depend_on_the_step(ops, nh, nkv, window, extras):  # noqa: F811
+    """Prompts in one step, each alone, in cuts, token by token, and single tokens beside a prompt."""
+    lens = [200, 37, 5, 130]
+    cache = ToyCache(lens, nkv, 64, torch.float32)
+    qs = [rnd(n, nh * 64, seed=20 + b, scale=3.0) for b, n in enumerate(lens)]
+    kw = {}
+    if "sink" in extras:
+        kw["sink"] = rnd(nh, seed=9)
+    if "slope" in extras:
+        kw["slope"] = torch.tensor([2.0 ** -(h + 1) for h in range(nh)], device=DEV)
+    none = [0] * len(lens)
+    whole = _attend(ops, cache, lens, none, qs, nh, nkv, window, kw)
+    for b, n in enumerate(lens):
+        alone = _attend(ops, cache, lens, none, qs, nh, nkv, window, kw, use=[b])[0]
+        assert torch.equal(alone, whole[b])
+    for cut in (1, 8, 33, 64):
+        first = [min(n, cut) for n in lens]
+        rest = [n - f for n, f in zip(lens, first)]
+        left = [b for b, r in enumerate(rest) if r]
+        for part, at, use in ((first, none, None), (rest, first, left)):
+            got = _attend(ops, cache, part, at, qs, nh, nkv, window, kw, use=use)
+            for g, b in zip(got, use or range(len(lens))):
+                assert torch.equal(g, whole[b][at[b]:at[b] + part[b]]), (cut, b)
+    for i in range(0, lens[1], 3):                # one token each, and single ones beside a prompt
+        at = [min(i * 5, n - 1) for n in lens]
+        ones = _attend(ops, cache, [1] * 4, at, qs, nh, nkv, window, kw)
+        for b in range(4):
+            assert torch.equal(ones[b][0], whole[b][at[b]])
+        mixed = _attend(ops, cache, [lens[0], 1, 1, 1], [0] + at[1:], qs, nh, nkv, window, kw)
+        assert torch.equal(mixed[0], whole[0])
+        for b in (1, 2, 3):
+            assert torch.equal(mixed[b][0], whole[b][at[b]])
+
+
+@pytest.mark.parametrize("new,cached", [([1, 1], [2047, 2100]), ([1], [9000]), ([300], [0]),
+                                        ([40, 1], [5000, 63]), ([2500], [0])])
+@pytest.mark.parametrize("sharp", [1.0, 8.0, 1e4])
+def test_attention_against_64_bits(ops, new, cached, sharp):  # noqa: F811
+    """Contexts past the tiles whose sums the decode body keeps (2,048 keys).  A score is a sum of 64
+    products: 2^-24 sqrt(64) of its terms, at most 6e-7 of the largest score, and so much may every
+    probability be off; the sums add a few units of the last place."""
+    nh, nkv = 3, 1
+    lens = [c + n for c, n in zip(cached, new)]
+    cache = ToyCache(lens, nkv, 64, torch.float32)
+    qs = [rnd(n, nh * 64, seed=30 + b, scale=sharp) for b, n in enumerate(lens)]
+    got = torch.cat(_attend(ops, cache, new, cached, qs, nh, nkv, 0, {}))
+    want, most = [], 0.0
+    for b, n in enumerate(lens):
+        blocks = cache.table_host[cache.slots[b], :-(-n // 64)]
+        k, v = (x[torch.as_tensor(blocks).long()].permute(1, 0, 2, 3).reshape(64 * len(blocks), 64)[:n]
+                .double() for x in (cache.k, cache.v))
+        q = qs[b][cached[b]:].double().view(new[b], nh, 64)
+        s = torch.einsum("thd,kd->thk", q, k) * 0.17
+        ahead = torch.arange(n, device=DEV)[None] > torch.arange(cached[b], n, device=DEV)[:, None]
+        s = s.masked_fill(ahead[:, None], -math.inf)
+        most = max(most, float((torch.einsum("thd,kd->thk", q.abs(), k.abs()) * 0.17).max()))
+        want.append(torch.einsum("thk,kd->thd", torch.softmax(s, -1), v).reshape(new[b], -1))
+    want = torch.cat(want)
+    off = float((got.double() - want).norm() / want.norm())
+    assert off <= 1e-6 + 8 * 2.0 ** -24 * most, off
+
+
+def test_scores_without_bounds(ops):  # noqa: F811
+    """Scores of 1e30 and minus infinity: the largest key's value, and no number where one is none."""
+    cache = ToyCache([100, 100, 100], 1, 64, torch.float32)
+    as_ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    row = lambda b, i: (int(cache.table_host[cache.slots[b], i // 64]), 0, i % 64)  # noqa: E731
+    q = torch.zeros(3, 64, device=DEV)
+    q[:, 0] = 1e15
+    for b in range(3):
+        for i in range(100):
+            cache.k[row(b, i)][0] = -1e15
+    cache.k[row(0, 70)][0] = 1e15                  # one key far above the others
+    cache.k[row(1, 3)][0] = -math.inf              # ... one that is seen and weighs nothing
+    cache.k[row(2, 5)][0] = math.nan
+    outs = []
+    for new in ([1, 1, 1], None):
+        out = torch.empty(3, 64, device=DEV)
+        if new:
+            ops.attn_simt(q, out, cache.k, cache.v, cache.table, as_ints([99] * 3), as_ints([0, 1, 2]),
+                          cache.seq_slot, 1, 1, 64, 1.0, 0, 64, news=new)
+        else:                                      # the prompt body: eight rows of each
+            wide = q.repeat_interleave(8, 0)
+            pos = [92 + i for _ in range(3) for i in range(8)]
+            full = torch.empty(24, 64, device=DEV)
+            ops.attn_simt(wide, full, cache.k, cache.v, cache.table, as_ints(pos),
+                          as_ints([i // 8 for i in range(24)]), cache.seq_slot, 1, 1, 64, 1.0, 0, 64,
+                          news=[8, 8, 8])
+            out = full[7::8]
+        outs.append(out)
+        close(out[0], cache.v[row(0, 70)], 1e-6)
+        others = torch.stack([cache.v[row(1, i)] for i in range(100) if i != 3]).double().mean(0)
+        close(out[1], others, 2e-6)
+        assert bool(torch.isnan(out[2]).all())
+    assert torch.equal(outs[0][:2], outs[1][:2])
