@@ -198,6 +198,9 @@ int cretif_advance_decode(int* tok_ids, int* tok_pos, int* seq_start, const int*
 // C[M,N] (= or +=) A[M,K] · W[N,K]^T, 32-bit FMA on the CUDA cores.
 int cretif_gemm_simt(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, int M,
                      int N, int K, int lda, int ldw, int ldc, int accumulate, void* stream);
+// The same by the kernel that takes every shape, whatever the operands are (the yardstick of the others).
+int cretif_gemm_plain(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, int M,
+                      int N, int K, int lda, int ldw, int ldc, int accumulate, void* stream);
 
 // `batch` products in one launch: product z reads A + z*sa, W + z*sw and writes C + z*sc
 // (strides in elements), e.g. a matrix per head applied to that head's columns of the rows.

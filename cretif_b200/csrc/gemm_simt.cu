@@ -117,9 +117,9 @@ static int launch(const void* A, const void* W, void* C, int M, int N, int K, in
 
 using namespace cretif;
 
-extern "C" int cretif_gemm_simt(const void* A, int a_dt, const void* W, int w_dt, void* C,
-                                int c_dt, int M, int N, int K, int lda, int ldw, int ldc,
-                                int accumulate, void* stream) {
+// fast 0: this file's kernel whatever the operands are.
+static int gemm_any(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt, int M, int N,
+                    int K, int lda, int ldw, int ldc, int accumulate, bool fast, void* stream) {
   if (M <= 0 || N <= 0) return kOk;
   if (K <= 0 || lda < K || ldw < K || ldc < N) return kBadArgument;
   if ((M + BM - 1) / BM > 65535) return kBadArgument;
@@ -127,7 +127,7 @@ extern "C" int cretif_gemm_simt(const void* A, int a_dt, const void* W, int w_dt
   typedef __nv_bfloat16 bf16;
   if (a_dt == kF32 && w_dt == kF32 && c_dt == kF32) {
     // rows that 16-byte loads reach: the fast bodies of the same 32-bit product
-    if (gemm_f32_takes(A, W, M, N, K, lda, ldw))
+    if (fast && gemm_f32_takes(A, W, M, N, K, lda, ldw))
       return gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc,
                       accumulate, st);
     return launch<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
@@ -139,6 +139,18 @@ extern "C" int cretif_gemm_simt(const void* A, int a_dt, const void* W, int w_dt
   if (a_dt == kF32 && w_dt == kBF16 && c_dt == kF32)
     return launch<float, bf16, float>(A, W, C, M, N, K, lda, ldw, ldc, accumulate, st);
   return kBadDType;
+}
+
+extern "C" int cretif_gemm_simt(const void* A, int a_dt, const void* W, int w_dt, void* C,
+                                int c_dt, int M, int N, int K, int lda, int ldw, int ldc,
+                                int accumulate, void* stream) {
+  return gemm_any(A, a_dt, W, w_dt, C, c_dt, M, N, K, lda, ldw, ldc, accumulate, true, stream);
+}
+
+extern "C" int cretif_gemm_plain(const void* A, int a_dt, const void* W, int w_dt, void* C, int c_dt,
+                                 int M, int N, int K, int lda, int ldw, int ldc, int accumulate,
+                                 void* stream) {
+  return gemm_any(A, a_dt, W, w_dt, C, c_dt, M, N, K, lda, ldw, ldc, accumulate, false, stream);
 }
 
 extern "C" int cretif_gemm_simt_batched(const void* A, int a_dt, const void* W, int w_dt, void* C,

@@ -259,16 +259,17 @@ def advance_decode(tok_ids, tok_pos, seq_start, sampled, B: int) -> None:
 
 
 # ------------------------------------------------------------------ matrix products
-def gemm_simt(a, w, c, accumulate: bool = False) -> None:
-    """c[M,N] (+)= a[M,K] · w[N,K]ᵀ in 32-bit FMA arithmetic."""
+def gemm_simt(a, w, c, accumulate: bool = False, plain: bool = False) -> None:
+    """c[M,N] (+)= a[M,K] · w[N,K]ᵀ in 32-bit FMA arithmetic.  ``plain``: by the kernel that takes
+    every shape, also where a faster one would (float32 rows that are 16-byte aligned)."""
     _need(a, "a", dim=2); _need(w, "w", dim=2); _need(c, "c", dim=2)
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or tuple(c.shape) != (M, N):
         raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(c.shape)}")
-    _check(lib().cretif_gemm_simt(_p(a), _dt(a), _p(w), _dt(w), _p(c), _dt(c), M, N, K,
-                                  _rows(a, "a"), _rows(w, "w"), _rows(c, "c"), int(accumulate),
-                                  _stream()), "gemm_simt")
+    product = lib().cretif_gemm_plain if plain else lib().cretif_gemm_simt
+    _check(product(_p(a), _dt(a), _p(w), _dt(w), _p(c), _dt(c), M, N, K, _rows(a, "a"),
+                   _rows(w, "w"), _rows(c, "c"), int(accumulate), _stream()), "gemm_simt")
 
 
 _batched_simt_only = False

@@ -5,7 +5,7 @@ kernel here wants), ``x`` is ``[tokens, in]``.  The reference dispatches on the
 weight format (``matmul_dispatch``, src/model.cu:797-825); here the choice is by
 compute dtype and by the number of rows:
 
-* float32: the CUDA-core FMA kernel, always (true 32-bit arithmetic);
+* float32: the CUDA-core FMA kernels, always (true 32-bit arithmetic);
 * bfloat16, few rows (decode): the weight-streaming kernel;
 * bfloat16, many rows (prefill): the tcgen05 tensor-core kernel;
 * any shape a fast kernel refuses (alignment, size) goes to the CUDA-core kernel,
@@ -26,7 +26,8 @@ _force_plain = False
 
 
 def force_plain_kernels(on: bool) -> None:
-    """Route every product to the CUDA-core kernel (used by tests as the yardstick)."""
+    """Route every product to the CUDA-core kernel that takes every shape (used by tests as the
+    yardstick)."""
     global _force_plain
     _force_plain = bool(on)
 
@@ -54,7 +55,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         if ops.gemm_tc_supported(x, w, out):
             ops.gemm_tc(x, w, out, accumulate)
             return out
-    ops.gemm_simt(x, w, out, accumulate)
+    ops.gemm_simt(x, w, out, accumulate, plain=_force_plain)
     return out
 
 

@@ -29,6 +29,25 @@ def test_a_row_of_the_product_does_not_depend_on_the_others(ops, N, K):  # noqa:
         assert torch.equal(c, whole[700 - m:]), m
 
 
+@pytest.mark.parametrize("M", [3, 70])
+def test_the_plain_product_can_be_chosen(ops, M):  # noqa: F811
+    """With the plain kernels forced, float32 rows that a fast body would take go to the kernel that
+    takes every shape as well: the bits of the same numbers in rows that no fast body takes."""
+    from cretif_b200.parts.linear import force_plain_kernels, linear
+    a, w = rnd(M, 576), rnd(200, 576, seed=1)
+    odd = torch.empty(200, 577, device=DEV)[:, :576]
+    odd.copy_(w)
+    want = linear(a, odd)
+    fast = linear(a, w)
+    force_plain_kernels(True)
+    try:
+        plain = linear(a, w)
+    finally:
+        force_plain_kernels(False)
+    assert torch.equal(plain, want) and not torch.equal(fast, want)
+    close(fast, want, 2e-6)
+
+
 def _attend(ops, cache, new, cached, qs, nh, nkv, window, kw, use=None):  # noqa: F811
     """Rows of the sequences ``use`` (all by default) in one step; a sequence's queries are
     qs[b][cached .. cached + new - 1]."""
