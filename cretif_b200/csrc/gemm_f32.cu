@@ -319,9 +319,11 @@ static int launch_tile(const float* A, const float* W, float* C, int M, int N, i
 }
 
 bool gemm_f32_takes(const void* A, const void* W, int M, int N, int K, int lda, int ldw) {
-  // 16-byte loads of whole rows
+  // 16-byte loads of whole rows; the grids have one dimension (few rows: at most 64 of them, four
+  // columns a CTA and more)
   return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 &&
-         ((uintptr_t)W & 15) == 0 && N <= 4 * 65535 && M <= 32 * 65535;
+         ((uintptr_t)W & 15) == 0 && N <= 1 << 26 &&
+         (M + 31LL) / 32 * ((N + 31) / 32) <= 0x7fffffffLL;
 }
 
 int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,

@@ -29,6 +29,20 @@ def test_a_row_of_the_product_does_not_depend_on_the_others(ops, N, K):  # noqa:
         assert torch.equal(c, whole[700 - m:]), m
 
 
+@pytest.mark.parametrize("M", [1, 8, 33])
+def test_a_vocabulary_of_262144(ops, M):  # noqa: F811
+    """More columns than four times a grid's second dimension still take the fast bodies: their bits, by
+    a smaller matrix of some of the rows, which are not those of the kernel that takes every shape."""
+    N, K = 262144, 96
+    a, w = rnd(M, K), rnd(N, K, seed=1)
+    c, part, plain = (torch.empty(M, n, device=DEV) for n in (N, 1000, 1000))
+    ops.gemm_simt(a, w, c)
+    ops.gemm_simt(a, w[-1000:], part)
+    ops.gemm_simt(a, w[-1000:], plain, plain=True)
+    assert torch.equal(c[:, -1000:], part) and not torch.equal(part, plain)
+    close(c[:, :1000], a.double() @ w[:1000].double().T, 2e-6)
+
+
 @pytest.mark.parametrize("M", [3, 70])
 def test_the_plain_product_can_be_chosen(ops, M):  # noqa: F811
     """With the plain kernels forced, float32 rows that a fast body would take go to the kernel that
