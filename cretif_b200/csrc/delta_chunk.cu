@@ -415,7 +415,10 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   float* ST = XO + 2 * P::kXO;               // the state's slice, a row per column: [EC][LD]
   float* red = ST + EC * LD;                 // [KS][2 kC][EC + 4]
   float* X = red + P::kRed;                  // [kC][EC]
-  const int b = sequence_by_length(cu, B, blockIdx.z), h = blockIdx.x, col0 = blockIdx.y * EC;
+  // the grid: heads, slices of columns, sequences (the slowest)
+  const unsigned part = blockIdx.x / (unsigned)H, slices = (unsigned)(e / EC);
+  const int h = (int)(blockIdx.x - part * H), col0 = (int)(part % slices) * EC;
+  const int b = sequence_by_length(cu, B, (int)(part / slices));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t0 = cu[b], t1 = cu[b + 1];
   const Rows at = rows_of(H, D, e, GENERAL);
@@ -601,9 +604,8 @@ int launch_state_t(const float* ws, const float* v, int ldv, float* state, size_
   auto kern = delta_chunk_state_kernel<D, EC, GENERAL>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return (int)err;
-  if (B > 65535) return kBadArgument;
-  kern<<<dim3(H, e / EC, B), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
-                                               o_raw, write_state);
+  kern<<<(unsigned)B * H * (e / EC), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
+                                                       o_raw, write_state);
   return launch_status();
 }
 
@@ -632,8 +634,8 @@ int allow_smem(K kern, int bytes) {
   return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-bool takes(int H, int d, int e, const float* state, long long stride) {
-  return (d == 64 || d == 128) && e > 0 && e <= 256 && e % 16 == 0 && H > 0 && H <= 65535 &&
+bool takes(int B, int H, int d, int e, const float* state, long long stride) {
+  return (long long)B * H * (e / 16) <= 0x7fffffffLL && (d == 64 || d == 128) && e > 0 && e <= 256 && e % 16 == 0 && H > 0 && H <= 65535 &&
          stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
 }
 
@@ -653,7 +655,7 @@ extern "C" int cretif_delta_chunks(const float* prep, int ldp, float* state, lon
                                    int e, float* ws, float* o_raw, int write_state, int T,
                                    void* stream) {
   if (B <= 0 || T <= 0) return kOk;
-  if (!takes(H, d, e, state, stride) || G <= 0 || H % G || ldp < 2 * G * d + H * e + 2 * H)
+  if (!takes(B, H, d, e, state, stride) || G <= 0 || H % G || ldp < 2 * G * d + H * e + 2 * H)
     return kBadArgument;
   if (ldp % 4 || (((uintptr_t)prep | (uintptr_t)ws | (uintptr_t)o_raw) & 15)) return kMisaligned;
   cudaStream_t st = (cudaStream_t)stream;
@@ -679,7 +681,7 @@ extern "C" int cretif_general_delta_chunks(const float* proj, int ldp, const flo
                                            float* ws, float* o_raw, int write_state, int T,
                                            void* stream) {
   if (B <= 0 || T <= 0) return kOk;
-  if (!takes(H, d, e, state, stride) || ldp < 2 * H * d + H * e || ldq < 3 * H * d)
+  if (!takes(B, H, d, e, state, stride) || ldp < 2 * H * d + H * e || ldq < 3 * H * d)
     return kBadArgument;
   if (ldp % 4 || ldq % 4 ||
       (((uintptr_t)proj | (uintptr_t)prep | (uintptr_t)ws | (uintptr_t)o_raw) & 15))

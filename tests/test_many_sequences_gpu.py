@@ -34,3 +34,22 @@ def test_mamba_chunks():
         got.append((out, state))
     for a, b in zip(*got):
         assert (a - b).norm() <= 1e-6 * b.norm()
+
+
+def test_delta_chunks():
+    """A token a sequence, through the chunk kernels and token by token, the gated rule."""
+    from cretif_b200.csrc import ops
+    H, d, e = 1, 64, 16
+    prep = _rand(B, 148)[:, :2 * d + e + 2]
+    prep[:, -2:] = torch.sigmoid(prep[:, -2:])
+    start, gate = _rand(B, d * e, seed=3), _rand(B, e, seed=4)
+    every = torch.arange(B, **I32)
+    cu = torch.arange(B + 1, **I32)
+    got = []
+    for longest in (1 << 20, 1):
+        state, out = start.clone(), torch.empty(B, e, device="cuda")
+        ops.delta_recurrence(prep, gate, state, cu, every, B, H, 1, d, e, torch.ones(e, device="cuda"),
+                             1e-5, out, longest=longest)
+        got.append((out, state))
+    for a, b in zip(*got):
+        assert (a - b).norm() <= 1e-6 * b.norm()
