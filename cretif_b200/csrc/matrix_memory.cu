@@ -991,9 +991,10 @@ extern "C" int cretif_matrix_memory(const float* proj, int ldp, const float* bia
                       memory_carry_smem(d, 16, 1) <= 220 * 1024 &&
                       memory_intra_smem(d) <= 220 * 1024;
     if (fits) {
-      // (the caller decides by giving the scratch: csrc/ops.py, memory_scans)
+      // (the caller decides by giving the scratch: csrc/ops.py, memory_scans; the scan's grid has the
+      // sequences in its third dimension)
       ChunkSums cs{nullptr, nullptr, nullptr};
-      if (ws && aligned16(ws) && form != 3 && d <= 4 * kMcThreads &&
+      if (ws && aligned16(ws) && form != 3 && d <= 4 * kMcThreads && B <= 65535 &&
           memory_read_smem(d) <= 220 * 1024) {
         const size_t slots = (size_t)(T / kMcTokens + B) * H;
         cs.S = ws;

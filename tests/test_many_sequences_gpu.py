@@ -53,3 +53,24 @@ def test_delta_chunks():
         got.append((out, state))
     for a, b in zip(*got):
         assert (a - b).norm() <= 1e-6 * b.norm()
+
+
+def test_matrix_memory_chunks(monkeypatch):
+    """A token a sequence, in chunks although a scan is asked for, and token by token.  A read-out is normed
+    and a small one is normed up with its rounding: 1e-4 of the 2-norm."""
+    from cretif_b200.csrc import ops
+    monkeypatch.setattr(ops, "memory_scans", lambda *_: True)
+    H, d, e = 1, 4, 16
+    proj = _rand(B, 2 * H * (d + e) + 4)
+    start = _rand(B, H * d * (e + 1) + 4, seed=3).abs()
+    every = torch.arange(B, **I32)
+    cu = torch.arange(B + 1, **I32)
+    zero = torch.zeros(H, device="cuda")
+    got = []
+    for form in ("chunk", "token"):
+        state, out = start.clone(), torch.empty(B, H * e, device="cuda")
+        ops.matrix_memory(proj, zero, zero, 10.0, 0.5, state, cu, every, every, B, H, d, e,
+                          torch.ones(H * e, device="cuda"), 1e-5, out, form=form)
+        got.append((out, state))
+    for (a, b), bound in zip(zip(*got), (1e-4, 1e-6)):
+        assert (a - b).norm() <= bound * b.norm()
