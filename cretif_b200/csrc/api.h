@@ -75,26 +75,29 @@ int cretif_delta_prepare(const float* proj, int ldp, float* prep, int ldo, const
 int cretif_delta_conv_state(const float* proj, int ldp, float* conv_state, long long state_stride,
                             int taps, int C, const int* cu_seqlens, const int* seq_slot, int B,
                             void* stream);
-// o_raw: float32 scratch [T, H e] for the read-outs before their norm.
+// o_raw: float32 scratch [T, H e] for the read-outs before their norm.  below > 0: only sequences of
+// fewer than `below` tokens, whose read-outs stay in o_raw without the norm.
 int cretif_delta_recurrence(const float* prep, int ldp, const float* gate, int ldg, float* state,
                             long long state_stride, const int* cu_seqlens, const int* seq_slot,
                             int B, int H, int G, int d, int e, const float* norm_w, float eps,
                             float* o_raw, void* out, int out_dt, int ldo, int write_state, int T,
-                            void* stream);
+                            int below, void* stream);
 
 // Dynamic Tanh, dyt(x) = (tanh(alpha x) w + b) gain, a norm without statistics (pointwise_norm.cu);
 // alpha points at one float on the device, gain may be null.
 // The same recurrences over prompts in chunks of 32 tokens (delta_chunk.cu), read-outs before
 // their norm into o_raw [T, H e].  ws: float32 workspace of T x cretif_delta_chunk_row(...)
-// floats (0: sizes not taken; d is 64 or 128, e a multiple of 16).  16-byte aligned rows.
+// floats (0: sizes not taken; d is 64 or 128, e a multiple of 16).  16-byte aligned rows.  Sequences of
+// fewer than `from` tokens are left out.
 long long cretif_delta_chunk_row(int H, int d, int e, int general);
 int cretif_delta_chunks(const float* prep, int ldp, float* state, long long state_stride,
                         const int* cu_seqlens, const int* seq_slot, int B, int H, int G, int d,
-                        int e, float* ws, float* o_raw, int write_state, int T, void* stream);
+                        int e, float* ws, float* o_raw, int write_state, int T, int from,
+                        void* stream);
 int cretif_general_delta_chunks(const float* proj, int ldp, const float* prep, int ldq,
                                 float* state, long long state_stride, const int* cu_seqlens,
                                 const int* seq_slot, int B, int H, int d, int e, float* ws,
-                                float* o_raw, int write_state, int T, void* stream);
+                                float* o_raw, int write_state, int T, int from, void* stream);
 
 // dyt_rows: v = h[src] (+ delta[src]); if write_h, h[src] = v; out[r] = dyt(v); src = rows ? rows[r] : r.
 int cretif_dyt_rows(float* h, const void* delta, int delta_dt, const float* w, const float* b,
@@ -138,7 +141,7 @@ int cretif_general_delta_recurrence(const float* proj, int ldp, const float* pre
                                     const int* seq_slot, int B, int H, int d, int e,
                                     const float* norm_w, int per_head_weight, int gate_sigmoid,
                                     float eps, float* o_raw, void* out, int out_dt, int ldo,
-                                    int write_state, int T, void* stream);
+                                    int write_state, int T, int below, void* stream);
 
 // Attention over a cached latent (latent_ops.cu).  A projection row holds
 // [cq (q_rank) | c (rank) | kr (rot) | ...]: cq and c are brought to unit RMS and multiplied by wq

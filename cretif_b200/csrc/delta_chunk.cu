@@ -58,18 +58,19 @@ __host__ __device__ __forceinline__ Rows rows_of(int H, int d, int e, bool gener
   return r;
 }
 
-// Which tokens chunk `x` of the grid holds.  Sequence b's chunks are numbered from
+// Which tokens chunk `x` of the grid holds (none of sequences of fewer than `from` tokens: those are
+// walked by delta_rule.cu).  Sequence b's chunks are numbered from
 // cu[b] / kC + b: the ranges of two sequences do not meet, and the last number is below
 // T / kC + B.
 struct Span {
   int t0, n;
 };
-__device__ __forceinline__ Span find_span(const int* cu, int B, int x, Span* shared) {
+__device__ __forceinline__ Span find_span(const int* cu, int B, int x, int from, Span* shared) {
   if (threadIdx.x == 0) shared->n = 0;
   __syncthreads();
   for (int b = threadIdx.x; b < B; b += blockDim.x) {
     const int lo = cu[b], hi = cu[b + 1], at = x - (lo / kC + b);
-    if (at >= 0 && at < (hi - lo + kC - 1) / kC) {
+    if (hi - lo >= from && at >= 0 && at < (hi - lo + kC - 1) / kC) {
       shared->t0 = lo + at * kC;
       shared->n = min(kC, hi - shared->t0);
     }
@@ -140,7 +141,7 @@ __device__ __forceinline__ void put2(float* p, float2 v) { *reinterpret_cast<flo
 template <int D>
 __global__ void __launch_bounds__(128, 4)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __restrict__ ws,
-                           const int* __restrict__ cu, int B, int H, int G, int e) {
+                           const int* __restrict__ cu, int B, int H, int G, int e, int from) {
   constexpr int LD = D + 4;
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;                            // [kC][LD], then W
@@ -153,7 +154,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __res
   float* Vs = g + kC;                        // [kC][e], then X
   __shared__ Span span;
   const int tid = threadIdx.x, h = blockIdx.y, grp = h / (H / G);
-  const Span sp = find_span(cu, B, blockIdx.x, &span);
+  const Span sp = find_span(cu, B, blockIdx.x, from, &span);
   const int n = sp.n;
   if (n == 0) return;
   const int C0 = 2 * G * D + H * e;
@@ -254,7 +255,7 @@ template <int D>
 __global__ void __launch_bounds__(128, 2)
 general_chunk_prepare_kernel(const float* __restrict__ proj, int ldp,
                              const float* __restrict__ prep, int ldq, float* __restrict__ ws,
-                             const int* __restrict__ cu, int B, int H, int e) {
+                             const int* __restrict__ cu, int B, int H, int e, int from) {
   constexpr int LD = D + 4, V = D / 16;      // V: 16-byte pieces a lane holds
   extern __shared__ __align__(16) float sm[];
   float* Us = sm;                            // [kC][LD], then W
@@ -265,7 +266,7 @@ general_chunk_prepare_kernel(const float* __restrict__ proj, int ldp,
   float* Xs = Vs + kC * e;                   // [kC][e]
   __shared__ Span span;
   const int tid = threadIdx.x, h = blockIdx.y;
-  const Span sp = find_span(cu, B, blockIdx.x, &span);
+  const Span sp = find_span(cu, B, blockIdx.x, from, &span);
   const int n = sp.n;
   if (n == 0) return;
   const size_t Hd = (size_t)H * D;
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(256, 2)
 delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__ v, int ldv,
                          float* __restrict__ state, size_t state_stride,
                          const int* __restrict__ cu, const int* __restrict__ seq_slot, int B, int H,
-                         int e, float* __restrict__ o_raw, int write_state) {
+                         int e, float* __restrict__ o_raw, int write_state, int from) {
   using P = StatePlan<D, EC, GENERAL>;
   constexpr int LD = P::LD, KS = P::KS, J = EC / 4, I = D / 64;
   extern __shared__ __align__(16) float sm[];
@@ -421,6 +422,7 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   const int b = sequence_by_length(cu, B, (int)(part / slices));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t0 = cu[b], t1 = cu[b + 1];
+  if (t1 - t0 < from) return;
   const Rows at = rows_of(H, D, e, GENERAL);
 
   // A thread copies the same 16 bytes of every kStep-th row, and the same of every cStep-th row
@@ -598,21 +600,21 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
 template <int D, int EC, bool GENERAL>
 int launch_state_t(const float* ws, const float* v, int ldv, float* state, size_t stride,
                    const int* cu, const int* slot, int B, int H, int e, float* o_raw,
-                   int write_state, cudaStream_t st) {
+                   int write_state, int from, cudaStream_t st) {
   constexpr int bytes = StatePlan<D, EC, GENERAL>::kFloats * 4;
   static_assert(bytes <= 227 * 1024, "a chunk's stages do not fit");
   auto kern = delta_chunk_state_kernel<D, EC, GENERAL>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return (int)err;
   kern<<<(unsigned)B * H * (e / EC), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
-                                                       o_raw, write_state);
+                                                       o_raw, write_state, from);
   return launch_status();
 }
 
 template <int D, bool GENERAL>
 int launch_state(const float* ws, const float* v, int ldv, float* state, size_t stride,
                  const int* cu, const int* slot, int B, int H, int e, float* o_raw,
-                 int write_state, cudaStream_t st) {
+                 int write_state, int from, cudaStream_t st) {
   // Slices of 32 columns halve the reads of a chunk's rows; slices of 16 while 32 would not give
   // every SM its two CTAs (four sequences of 300 to 1,500 tokens, 16 heads of 128: 408 us in
   // slices of 16, 439 in slices of 32).
@@ -624,9 +626,9 @@ int launch_state(const float* ws, const float* v, int ldv, float* state, size_t 
   }();
   if (e % 32 == 0 && (long long)B * H * (e / 32) >= 2LL * sms)
     return launch_state_t<D, 32, GENERAL>(ws, v, ldv, state, stride, cu, slot, B, H, e, o_raw,
-                                          write_state, st);
+                                          write_state, from, st);
   return launch_state_t<D, 16, GENERAL>(ws, v, ldv, state, stride, cu, slot, B, H, e, o_raw,
-                                        write_state, st);
+                                        write_state, from, st);
 }
 
 template <typename K>
@@ -653,7 +655,7 @@ extern "C" long long cretif_delta_chunk_row(int H, int d, int e, int general) {
 extern "C" int cretif_delta_chunks(const float* prep, int ldp, float* state, long long stride,
                                    const int* cu, const int* seq_slot, int B, int H, int G, int d,
                                    int e, float* ws, float* o_raw, int write_state, int T,
-                                   void* stream) {
+                                   int from, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (!takes(B, H, d, e, state, stride) || G <= 0 || H % G || ldp < 2 * G * d + H * e + 2 * H)
     return kBadArgument;
@@ -665,21 +667,21 @@ extern "C" int cretif_delta_chunks(const float* prep, int ldp, float* state, lon
                    : allow_smem(delta_chunk_prepare_kernel<128>, bytes);
   if (rc) return rc;
   if (d == 64)
-    delta_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e);
+    delta_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from);
   else
-    delta_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e);
+    delta_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from);
   if ((rc = launch_status())) return rc;
   return d == 64 ? launch_state<64, false>(ws, nullptr, 0, state, (size_t)stride, cu, seq_slot, B,
-                                           H, e, o_raw, write_state, st)
+                                           H, e, o_raw, write_state, from, st)
                  : launch_state<128, false>(ws, nullptr, 0, state, (size_t)stride, cu, seq_slot, B,
-                                            H, e, o_raw, write_state, st);
+                                            H, e, o_raw, write_state, from, st);
 }
 
 extern "C" int cretif_general_delta_chunks(const float* proj, int ldp, const float* prep, int ldq,
                                            float* state, long long stride, const int* cu,
                                            const int* seq_slot, int B, int H, int d, int e,
                                            float* ws, float* o_raw, int write_state, int T,
-                                           void* stream) {
+                                           int from, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (!takes(B, H, d, e, state, stride) || ldp < 2 * H * d + H * e || ldq < 3 * H * d)
     return kBadArgument;
@@ -694,14 +696,14 @@ extern "C" int cretif_general_delta_chunks(const float* proj, int ldp, const flo
   if (rc) return rc;
   if (d == 64)
     general_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
-                                                               e);
+                                                               e, from);
   else
     general_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
-                                                                e);
+                                                                e, from);
   if ((rc = launch_status())) return rc;
   const float* v = proj + 2 * (size_t)H * d;
   return d == 64 ? launch_state<64, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H, e,
-                                          o_raw, write_state, st)
+                                          o_raw, write_state, from, st)
                  : launch_state<128, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H,
-                                           e, o_raw, write_state, st);
+                                           e, o_raw, write_state, from, st);
 }

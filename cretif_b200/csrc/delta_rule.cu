@@ -234,9 +234,10 @@ delta_recurrence_kernel(const float* __restrict__ prep, int ldp, float* __restri
                         size_t state_stride,
                         const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
                         int H, int G, int d, int e, int P, int ecols, float* __restrict__ o_raw,
-                        int write_state, int vec) {
+                        int write_state, int vec, int below) {
   dependent_begin();
   extern __shared__ __align__(16) float sm[];
+  if (below && cu_seqlens[blockIdx.x + 1] - cu_seqlens[blockIdx.x] >= below) return;
   // with at most 512 threads a lane also keeps the token's key slice in registers between
   // the two passes over its rows
   constexpr bool kKeepK = MAXT <= 512 && DREG <= 32;
@@ -417,8 +418,8 @@ delta_out_norm_kernel(const float* __restrict__ o_raw, const float* __restrict__
 template <int DREG, int MAXT>
 static int launch_recurrence_t(const float* prep, int ldp, float* state, size_t state_stride,
                                const int* cu, const int* seq_slot, int B, int H, int G, int d,
-                               int e, int P, int ecols, float* o_raw, int write_state, int threads,
-                               cudaStream_t st) {
+                               int e, int P, int ecols, float* o_raw, int write_state, int below,
+                               int threads, cudaStream_t st) {
   const size_t stage = (size_t)kChunk * (2 * P * (DREG + 4) + ecols + 2);
   const size_t smem = sizeof(float) * 2 * stage;
   auto kern = delta_recurrence_kernel<DREG, MAXT>;
@@ -432,20 +433,20 @@ static int launch_recurrence_t(const float* prep, int ldp, float* state, size_t 
   const int vec = ldp % 4 == 0 && d % 4 == 0 && e % 4 == 0 && ecols % 4 == 0 &&
                   ((uintptr_t)prep & 15) == 0;
   kern<<<dim3(B, H, e / ecols), threads, smem, st>>>(prep, ldp, state, state_stride, cu, seq_slot,
-                                                     H, G, d, e, P, ecols, o_raw, write_state, vec);
+                                                     H, G, d, e, P, ecols, o_raw, write_state, vec, below);
   return launch_status();
 }
 
 template <int DREG>
 static int launch_recurrence(const float* prep, int ldp, float* state, size_t state_stride,
                              const int* cu, const int* seq_slot, int B, int H, int G, int d, int e,
-                             int P, int ecols, float* o_raw, int write_state, cudaStream_t st) {
+                             int P, int ecols, float* o_raw, int write_state, int below, cudaStream_t st) {
   const int threads = ((ecols * P + 31) / 32) * 32;
   if (threads <= 512)
     return launch_recurrence_t<DREG, 512>(prep, ldp, state, state_stride, cu, seq_slot, B, H, G, d,
-                                          e, P, ecols, o_raw, write_state, threads, st);
+                                          e, P, ecols, o_raw, write_state, below, threads, st);
   return launch_recurrence_t<DREG, 1024>(prep, ldp, state, state_stride, cu, seq_slot, B, H, G, d,
-                                         e, P, ecols, o_raw, write_state, threads, st);
+                                         e, P, ecols, o_raw, write_state, below, threads, st);
 }
 
 }  // namespace cretif
@@ -493,12 +494,14 @@ extern "C" int cretif_delta_conv_state(const float* proj, int ldp, float* conv_s
   return launch_status();
 }
 
+// below > 0: only the sequences of fewer than `below` tokens (delta_chunk.cu takes the others), and
+// the read-outs stay as they are in o_raw.
 extern "C" int cretif_delta_recurrence(const float* prep, int ldp, const float* gate, int ldg,
                                        float* state, long long state_stride,
                                        const int* cu_seqlens, const int* seq_slot, int B, int H,
                                        int G, int d, int e, const float* norm_w, float eps,
                                        float* o_raw, void* out, int out_dt, int ldo,
-                                       int write_state, int T, void* stream) {
+                                       int write_state, int T, int below, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (H <= 0 || G <= 0 || H % G || d <= 0 || e <= 0 || !o_raw) return kBadArgument;
   if (out_dt != kF32 && out_dt != kBF16) return kBadDType;
@@ -534,14 +537,14 @@ extern "C" int cretif_delta_recurrence(const float* prep, int ldp, const float* 
   int rc;
 #define CRETIF_DELTA(DREG)                                                                      \
   launch_recurrence<DREG>(prep, ldp, state, (size_t)state_stride, cu_seqlens, seq_slot, B, H, G, \
-                          d, e, P, ecols, o_raw, write_state, st)
+                          d, e, P, ecols, o_raw, write_state, below, st)
   if (rows <= 8) rc = CRETIF_DELTA(8);
   else if (rows <= 16) rc = CRETIF_DELTA(16);
   else if (rows <= 32) rc = CRETIF_DELTA(32);
   else if (rows <= 64) rc = CRETIF_DELTA(64);
   else rc = CRETIF_DELTA(128);
 #undef CRETIF_DELTA
-  if (rc) return rc;
+  if (rc || below) return rc;
   const long long items = (long long)T * H;
   const unsigned blocks = (unsigned)((items + 7) / 8);
   if (out_dt == kF32)
@@ -663,9 +666,11 @@ general_delta_recurrence_kernel(const float* __restrict__ proj, int ldp,
                                 float* __restrict__ state, size_t state_stride,
                                 const int* __restrict__ cu_seqlens,
                                 const int* __restrict__ seq_slot, int H, int d, int e, int P,
-                                int ecols, float* __restrict__ o_raw, int write_state, int vec) {
+                                int ecols, float* __restrict__ o_raw, int write_state, int vec,
+                                int below) {
   dependent_begin();
   extern __shared__ __align__(16) float sm[];
+  if (below && cu_seqlens[blockIdx.x + 1] - cu_seqlens[blockIdx.x] >= below) return;
   const int b = blockIdx.x, h = blockIdx.y;
   constexpr int kSlice = DREG + 4;               // see delta_recurrence_kernel
   const int dpad = P * kSlice;
@@ -789,7 +794,7 @@ general_delta_recurrence_kernel(const float* __restrict__ proj, int ldp,
 template <int DREG, int MAXT>
 static int launch_general_t(const float* proj, int ldp, const float* prep, int ldq, float* state,
                             size_t state_stride, const int* cu, const int* seq_slot, int B, int H,
-                            int d, int e, int P, int ecols, float* o_raw, int write_state,
+                            int d, int e, int P, int ecols, float* o_raw, int write_state, int below,
                             int threads, cudaStream_t st) {
   const size_t stage = (size_t)kGenChunk * (5 * P * (DREG + 4) + ecols);
   const size_t smem = sizeof(float) * 2 * stage;
@@ -804,21 +809,21 @@ static int launch_general_t(const float* proj, int ldp, const float* prep, int l
                   (((uintptr_t)proj | (uintptr_t)prep) & 15) == 0;
   kern<<<dim3(B, H, e / ecols), threads, smem, st>>>(proj, ldp, prep, ldq, state, state_stride, cu,
                                                      seq_slot, H, d, e, P, ecols, o_raw,
-                                                     write_state, vec);
+                                                     write_state, vec, below);
   return launch_status();
 }
 
 template <int DREG>
 static int launch_general(const float* proj, int ldp, const float* prep, int ldq, float* state,
                           size_t state_stride, const int* cu, const int* seq_slot, int B, int H,
-                          int d, int e, int P, int ecols, float* o_raw, int write_state,
+                          int d, int e, int P, int ecols, float* o_raw, int write_state, int below,
                           cudaStream_t st) {
   const int threads = ((ecols * P + 31) / 32) * 32;
   if (threads <= 512)
     return launch_general_t<DREG, 512>(proj, ldp, prep, ldq, state, state_stride, cu, seq_slot, B,
-                                       H, d, e, P, ecols, o_raw, write_state, threads, st);
+                                       H, d, e, P, ecols, o_raw, write_state, below, threads, st);
   return launch_general_t<DREG, 1024>(proj, ldp, prep, ldq, state, state_stride, cu, seq_slot, B,
-                                      H, d, e, P, ecols, o_raw, write_state, threads, st);
+                                      H, d, e, P, ecols, o_raw, write_state, below, threads, st);
 }
 
 }  // namespace cretif
@@ -878,7 +883,7 @@ extern "C" int cretif_general_delta_recurrence(
     const float* proj, int ldp, const float* prep, int ldq, const float* gate, int ldg,
     float* state, long long state_stride, const int* cu_seqlens, const int* seq_slot, int B, int H,
     int d, int e, const float* norm_w, int per_head_weight, int gate_sigmoid, float eps,
-    float* o_raw, void* out, int out_dt, int ldo, int write_state, int T, void* stream) {
+    float* o_raw, void* out, int out_dt, int ldo, int write_state, int T, int below, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (H <= 0 || d <= 0 || e <= 0 || !o_raw) return kBadArgument;
   if (out_dt != kF32 && out_dt != kBF16) return kBadDType;
@@ -915,12 +920,12 @@ extern "C" int cretif_general_delta_recurrence(
   int rc;
 #define CRETIF_GDELTA(DREG)                                                                     \
   launch_general<DREG>(proj, ldp, prep, ldq, state, (size_t)state_stride, cu_seqlens, seq_slot, \
-                       B, H, d, e, P, ecols, o_raw, write_state, st)
+                       B, H, d, e, P, ecols, o_raw, write_state, below, st)
   if (rows <= 8) rc = CRETIF_GDELTA(8);
   else if (rows <= 16) rc = CRETIF_GDELTA(16);
   else rc = CRETIF_GDELTA(32);
 #undef CRETIF_GDELTA
-  if (rc) return rc;
+  if (rc || below) return rc;
   const long long items = (long long)T * H;
   const unsigned blocks = (unsigned)((items + 7) / 8);
   const int w_stride = per_head_weight ? e : 0;

@@ -403,12 +403,30 @@ DELTA_CHUNKS_FROM = 64
 # (9 heads of 64 by 256 tokens, walk and chunks: 16 sequences 122 and 100 us, 32 161 and 170, 64
 # 261 and 329).
 DELTA_CHUNKS_HEADS64 = 256
+# A sequence of fewer tokens than this is walked all the same, in a launch beside the chunks', where
+# there are that many heads of such sequences or more: a lone token in a chunk costs all of the
+# chunk's work, which a few of them hide under the long sequences'.  Microseconds, everything walked,
+# everything in chunks and as here: a prompt of 64 beside 63 single tokens 108, 185 and 97 (gated,
+# 16 heads of 128), 154, 255 and 130 (general), 34, 44 and 30 (gated, 9 heads of 64); of 512 493, 219 and
+# 153; beside 8 of them 296, 97 and 99.  32 sequences of 8 tokens: 137 in chunks, 150 walked.
+DELTA_WALK_BELOW = 8
+DELTA_WALK_HEADS = 256
 
 
-def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: bool, state, rows):
+def _delta_short(news, H: int) -> int:
+    """The tokens of a step's sequences that are walked beside the chunks of the others (0 where
+    ``news``, how many each brings, is not known)."""
+    short = [n for n in news if n < DELTA_WALK_BELOW]
+    return sum(short) if len(short) * H >= DELTA_WALK_HEADS else 0
+
+
+def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: bool, state, rows,
+                      short: int = 0):
     """The workspace of a step whose delta rule goes in chunks, or None where it walks token by
-    token: few tokens, or sizes and strides that the chunk kernels' 16-byte accesses do not take."""
-    if longest < DELTA_CHUNKS_FROM or (d == 64 and T * H > DELTA_CHUNKS_HEADS64 * longest):
+    token: few tokens, or sizes and strides that the chunk kernels' 16-byte accesses do not take.
+    ``short``: how many of the step's ``T`` tokens are walked all the same."""
+    if longest < DELTA_CHUNKS_FROM or (d == 64
+                                       and (T - short) * H > DELTA_CHUNKS_HEADS64 * longest):
         return None
     if any(r.stride(0) % 4 or r.data_ptr() % 16 for r in rows):
         return None
@@ -420,11 +438,12 @@ def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: boo
 
 def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G: int, d: int,
                      e: int, norm_w, eps: float, out, write_state: bool = True,
-                     longest: int = 0) -> None:
+                     longest: int = 0, news=()) -> None:
     """The recurrence over the step's tokens of every (sequence, head), from and to ``state``
     (view [slots, H·d·e] float32), then the per-head RMS norm times ``norm_w`` times
     SiLU(``gate``) → ``out`` [T, H·e].  ``longest``: the most tokens a sequence brings (0: not
-    known), by which the step goes token by token or in chunks."""
+    known: every sequence is walked token by token), ``news``: how many each brings (empty: not
+    known, all go as the longest does), by which they go token by token or in chunks."""
     _need(prep, "prep", torch.float32, 2); _need(gate, "gate", torch.float32, 2)
     _need(state, "state", torch.float32, 2); _need(out, "out", dim=2)
     _need(norm_w, "norm_w", torch.float32, 1)
@@ -432,18 +451,23 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
         raise KernelError("delta_recurrence: the state's sizes do not fit")
     T = prep.shape[0]
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=prep.device)
-    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,))
+    short = _delta_short(news, H)
+    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), short)
+    below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_delta_chunks(
             _p(prep), _rows(prep, "prep"), _p(state), ctypes.c_longlong(state.stride(0)),
             _p(cu_seqlens), _p(seq_slot), B, H, G, d, e, _p(ws), _p(o_raw), int(write_state), T,
-            _stream()), "delta_chunks", kernels=2)
-        return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
+            below, _stream()), "delta_chunks", kernels=2)
+        if not below:
+            return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
     _check(lib().cretif_delta_recurrence(
         _p(prep), _rows(prep, "prep"), _p(gate), _rows(gate, "gate"), _p(state),
         ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, G, d, e,
         _p(norm_w), ctypes.c_float(eps), _p(o_raw), _p(out), _dt(out), _rows(out, "out"),
-        int(write_state), T, _stream()), "delta_recurrence", kernels=2)
+        int(write_state), T, below, _stream()), "delta_recurrence", kernels=1 if below else 2)
+    if below:
+        heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
 
 
 # ------------------------------------------------------------------ per-head work, retention
@@ -1030,10 +1054,10 @@ def general_delta_prepare(proj, prep, a_bias, z, w0, H: int, d: int, e: int, uni
 def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, d: int,
                              e: int, norm_w, eps: float, out, per_head_weight: bool = True,
                              gate_sigmoid: bool = True, write_state: bool = True,
-                             longest: int = 0) -> None:
+                             longest: int = 0, news=()) -> None:
     """The generalized delta rule over the step's tokens of every (sequence, head), from and to
     ``state`` (view [slots, H·d·e] float32), then the per-head RMS norm times ``norm_w`` times
-    the gate -> ``out`` [T, H·e].  ``longest``: see ``delta_recurrence``."""
+    the gate -> ``out`` [T, H·e].  ``longest`` and ``news``: see ``delta_recurrence``."""
     _need(proj, "proj", torch.float32, 2); _need(prep, "prep", torch.float32, 2)
     _need(gate, "gate", torch.float32, 2); _need(state, "state", torch.float32, 2)
     _need(out, "out", dim=2); _need(norm_w, "norm_w", torch.float32, 1)
@@ -1042,19 +1066,24 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
             or out.shape[1] < H * e or norm_w.numel() != (H * e if per_head_weight else e)):
         raise KernelError("general_delta_recurrence: sizes do not fit")
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=proj.device)
-    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep))
+    short = _delta_short(news, H)
+    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), short)
+    below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_general_delta_chunks(
             _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(state),
             ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, d, e, _p(ws),
-            _p(o_raw), int(write_state), T, _stream()), "general_delta_chunks", kernels=2)
-        return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
+            _p(o_raw), int(write_state), T, below, _stream()), "general_delta_chunks", kernels=2)
+        if not below:
+            return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
     _check(lib().cretif_general_delta_recurrence(
         _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(gate),
         _rows(gate, "gate"), _p(state), ctypes.c_longlong(state.stride(0)), _p(cu_seqlens),
         _p(seq_slot), B, H, d, e, _p(norm_w), int(per_head_weight), int(gate_sigmoid),
         ctypes.c_float(eps), _p(o_raw), _p(out), _dt(out), _rows(out, "out"), int(write_state), T,
-        _stream()), "general_delta_recurrence", kernels=2)
+        below, _stream()), "general_delta_recurrence", kernels=1 if below else 2)
+    if below:
+        heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
 
 
 # ------------------------------------------------------------------ routed experts

@@ -99,7 +99,8 @@ class GatedDeltaRule(Part):
         out = torch.empty((T, H * e), dtype=self.dtype, device=x.device)
         ops.delta_recurrence(prep, proj[:, C:C + H * e], matrices, ctx.cu_seqlens, ctx.seq_slot,
                              ctx.B, H, G, d, e, self.norm_w, self.eps, out,
-                             write_state=cache.writes, longest=ctx.max_new)
+                             write_state=cache.writes, longest=ctx.max_new,
+                             news=ctx.seq_new_host)
         if cache.writes:
             ops.delta_conv_state(proj, inputs, self.taps, C, ctx.cu_seqlens, ctx.seq_slot, ctx.B)
         return linear(out, self.w_o, out_dtype=torch.float32)
@@ -201,7 +202,7 @@ class GeneralDeltaRule(Part):
         ops.general_delta_recurrence(proj, prep, gate, cache.state, ctx.cu_seqlens, ctx.seq_slot,
                                      ctx.B, H, d, e, self.norm_w, self.eps, out,
                                      per_head_weight=True, gate_sigmoid=True, write_state=True,
-                                     longest=ctx.max_new)
+                                     longest=ctx.max_new, news=ctx.seq_new_host)
         return linear(out, self.w_o, out_dtype=torch.float32)
 
     def weight_bytes(self):

@@ -126,3 +126,47 @@ def test_small_or_odd_sizes_walk():
     assert room(70, 70, 2, 64, 16, False, state, (prep[:, 1:],)) is None
     assert room(70, 70, 2, 64, 16, False, state, (torch.zeros(70, 257, device="cuda"),)) is None
     assert room(70, 70, 2, 64, 16, False, state[:, 2:], (prep,)) is None
+
+
+@pytest.mark.parametrize("general,H,G,d,e", [(False, 16, 8, 128, 32), (True, 9, 9, 64, 64)])
+@pytest.mark.parametrize("lens", [(70,) + (1,) * 40, (1,) * 20 + (100, 0, 7, 33) + (3,) * 30])
+def test_mixed_steps(general, H, G, d, e, lens):
+    """Single tokens beside a prompt are walked, the others go in chunks: the read-outs and states of
+    either are, to the bit, those of the whole step walked and of the whole step in chunks."""
+    from cretif_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    T, B = sum(lens), len(lens)
+    short = [n < ops.DELTA_WALK_BELOW for n in lens]
+    assert ops._delta_short(lens, H) == sum(n for n, s in zip(lens, short) if s)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    decays = torch.rand(T, H * d if general else H, generator=gen, device="cuda")
+    start, gate, norm_w = rand(B, H * d * e), rand(T, H * e), torch.ones(e, device="cuda")
+    key = rand(T, G * d)
+    key = (key.view(T, G, d) / key.view(T, G, d).norm(dim=2, keepdim=True)).reshape(T, G * d)
+    if general:
+        proj = torch.cat([rand(T, H * d), key, rand(T, H * e)], 1)
+        prep = torch.cat([key, -torch.rand(T, H * d, generator=gen, device="cuda") * key, decays], 1)
+    else:
+        prep = torch.cat([rand(T, G * d), key, rand(T, H * e), decays, decays], 1)
+    at = torch.tensor([0] + list(lens)).cumsum(0).tolist()
+
+    cu = torch.tensor(at, dtype=torch.int32, device="cuda")
+    slots = torch.arange(B, dtype=torch.int32, device="cuda")
+
+    def step(**kw):
+        state, out = start.clone(), torch.empty(T, H * e, device="cuda")
+        if general:
+            ops.general_delta_recurrence(proj, prep, gate, state, cu, slots, B, H, d, e, norm_w, 1e-5,
+                                         out, per_head_weight=False, **kw)
+        else:
+            ops.delta_recurrence(prep, gate, state, cu, slots, B, H, G, d, e, norm_w, 1e-5, out, **kw)
+        return out, state
+    walked, chunked = step(longest=1), step(longest=max(lens))
+    out, state = step(longest=max(lens), news=lens)
+    for b in range(B):
+        want = walked if short[b] else chunked
+        assert torch.equal(out[at[b]:at[b + 1]], want[0][at[b]:at[b + 1]]), b
+        assert torch.equal(state[b], want[1][b]), b
+    assert not torch.equal(out, walked[0]) and not torch.equal(out, chunked[0])
