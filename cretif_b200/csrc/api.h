@@ -86,18 +86,20 @@ int cretif_delta_recurrence(const float* prep, int ldp, const float* gate, int l
 // Dynamic Tanh, dyt(x) = (tanh(alpha x) w + b) gain, a norm without statistics (pointwise_norm.cu);
 // alpha points at one float on the device, gain may be null.
 // The same recurrences over prompts in chunks of 32 tokens (delta_chunk.cu), read-outs before
-// their norm into o_raw [T, H e].  ws: float32 workspace of T x cretif_delta_chunk_row(...)
-// floats (0: sizes not taken; d is 64 or 128, e a multiple of 16).  16-byte aligned rows.  Sequences of
+// their norm into o_raw [T, H e].  ws: float32 workspace of ws_floats, cretif_delta_chunk_row(...) a
+// token (0: sizes not taken; d is 64 or 128, e a multiple of 16); one that does not hold all tokens (32
+// at least) takes the step span by span, with write_state only.  16-byte aligned rows.  Sequences of
 // fewer than `from` tokens are left out.
 long long cretif_delta_chunk_row(int H, int d, int e, int general);
 int cretif_delta_chunks(const float* prep, int ldp, float* state, long long state_stride,
                         const int* cu_seqlens, const int* seq_slot, int B, int H, int G, int d,
-                        int e, float* ws, float* o_raw, int write_state, int T, int from,
-                        void* stream);
+                        int e, float* ws, long long ws_floats, float* o_raw, int write_state, int T,
+                        int from, void* stream);
 int cretif_general_delta_chunks(const float* proj, int ldp, const float* prep, int ldq,
                                 float* state, long long state_stride, const int* cu_seqlens,
                                 const int* seq_slot, int B, int H, int d, int e, float* ws,
-                                float* o_raw, int write_state, int T, int from, void* stream);
+                                long long ws_floats, float* o_raw, int write_state, int T,
+                                int from, void* stream);
 
 // dyt_rows: v = h[src] (+ delta[src]); if write_h, h[src] = v; out[r] = dyt(v); src = rows ? rows[r] : r.
 int cretif_dyt_rows(float* h, const void* delta, int delta_dt, const float* w, const float* b,

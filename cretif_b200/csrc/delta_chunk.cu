@@ -17,6 +17,9 @@
 //   two-wide FMAs), then the rank-32 update of the state the threads hold in registers.  A
 //   chunk's operands arrive by cp.async a chunk ahead; three barriers a chunk.
 //
+// The prepared vectors lie in a workspace; a step that it does not hold goes span by span of
+// its tokens, the state passing from one to the next through memory.
+//
 // All arithmetic is 32-bit FMA.  A token-by-token walk is a chain of two dependent reductions and
 // an update, 0.47 us a token (0.54 to 1.1 for the general rule, whose five vectors a token load
 // the shared memory) whatever the chip has idle.  Microseconds a layer with the norm of the
@@ -59,18 +62,19 @@ __host__ __device__ __forceinline__ Rows rows_of(int H, int d, int e, bool gener
 }
 
 // Which tokens chunk `x` of the grid holds (none of sequences of fewer than `from` tokens: those are
-// walked by delta_rule.cu).  Sequence b's chunks are numbered from
-// cu[b] / kC + b: the ranges of two sequences do not meet, and the last number is below
-// T / kC + B.
+// walked by delta_rule.cu).  The launch takes the tokens s0 .. s1 - 1, of sequence b those from lo to
+// hi - 1; its chunks are numbered from (lo - s0) / kC + b: the ranges of two sequences do not meet,
+// and the last number is below (s1 - s0) / kC + B.
 struct Span {
   int t0, n;
 };
-__device__ __forceinline__ Span find_span(const int* cu, int B, int x, int from, Span* shared) {
+__device__ __forceinline__ Span find_span(const int* cu, int B, int x, int from, int s0, int s1,
+                                          Span* shared) {
   if (threadIdx.x == 0) shared->n = 0;
   __syncthreads();
   for (int b = threadIdx.x; b < B; b += blockDim.x) {
-    const int lo = cu[b], hi = cu[b + 1], at = x - (lo / kC + b);
-    if (hi - lo >= from && at >= 0 && at < (hi - lo + kC - 1) / kC) {
+    const int lo = max(cu[b], s0), hi = min(cu[b + 1], s1), at = x - ((lo - s0) / kC + b);
+    if (cu[b + 1] - cu[b] >= from && lo < hi && at >= 0 && at < (hi - lo + kC - 1) / kC) {
       shared->t0 = lo + at * kC;
       shared->n = min(kC, hi - shared->t0);
     }
@@ -141,7 +145,8 @@ __device__ __forceinline__ void put2(float* p, float2 v) { *reinterpret_cast<flo
 template <int D>
 __global__ void __launch_bounds__(128, 4)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __restrict__ ws,
-                           const int* __restrict__ cu, int B, int H, int G, int e, int from) {
+                           const int* __restrict__ cu, int B, int H, int G, int e, int from,
+                           int s0, int s1) {
   constexpr int LD = D + 4;
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;                            // [kC][LD], then W
@@ -154,7 +159,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __res
   float* Vs = g + kC;                        // [kC][e], then X
   __shared__ Span span;
   const int tid = threadIdx.x, h = blockIdx.y, grp = h / (H / G);
-  const Span sp = find_span(cu, B, blockIdx.x, from, &span);
+  const Span sp = find_span(cu, B, blockIdx.x, from, s0, s1, &span);
   const int n = sp.n;
   if (n == 0) return;
   const int C0 = 2 * G * D + H * e;
@@ -216,7 +221,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __res
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   const Rows at = rows_of(H, D, e, false);
-  float* out = ws + (size_t)sp.t0 * at.ld;
+  float* out = ws + (size_t)(sp.t0 - s0) * at.ld;
   const float g0 = g[0];
   if (tid == 0) out[at.gamma + h] = g0 * R[n - 1];
   for (int c = 2 * tid; c < D + e; c += 256) {
@@ -255,7 +260,8 @@ template <int D>
 __global__ void __launch_bounds__(128, 2)
 general_chunk_prepare_kernel(const float* __restrict__ proj, int ldp,
                              const float* __restrict__ prep, int ldq, float* __restrict__ ws,
-                             const int* __restrict__ cu, int B, int H, int e, int from) {
+                             const int* __restrict__ cu, int B, int H, int e, int from, int s0,
+                             int s1) {
   constexpr int LD = D + 4, V = D / 16;      // V: 16-byte pieces a lane holds
   extern __shared__ __align__(16) float sm[];
   float* Us = sm;                            // [kC][LD], then W
@@ -266,7 +272,7 @@ general_chunk_prepare_kernel(const float* __restrict__ proj, int ldp,
   float* Xs = Vs + kC * e;                   // [kC][e]
   __shared__ Span span;
   const int tid = threadIdx.x, h = blockIdx.y;
-  const Span sp = find_span(cu, B, blockIdx.x, from, &span);
+  const Span sp = find_span(cu, B, blockIdx.x, from, s0, s1, &span);
   const int n = sp.n;
   if (n == 0) return;
   const size_t Hd = (size_t)H * D;
@@ -340,7 +346,7 @@ general_chunk_prepare_kernel(const float* __restrict__ proj, int ldp,
   __syncthreads();
   const float *A = M, *Bv = M + kC * kA, *E = Bv + kC * kA, *F = E + kC * kA;
   const Rows at = rows_of(H, D, e, true);
-  float* out = ws + (size_t)sp.t0 * at.ld;
+  float* out = ws + (size_t)(sp.t0 - s0) * at.ld;
   for (int c = 2 * tid; c < D + e; c += 256) {
     if (c < D) {
       float* col = out + (size_t)h * D + c;
@@ -404,7 +410,8 @@ __global__ void __launch_bounds__(256, 2)
 delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__ v, int ldv,
                          float* __restrict__ state, size_t state_stride,
                          const int* __restrict__ cu, const int* __restrict__ seq_slot, int B, int H,
-                         int e, float* __restrict__ o_raw, int write_state, int from) {
+                         int e, float* __restrict__ o_raw, int write_state, int from, int s0,
+                         int s1) {
   using P = StatePlan<D, EC, GENERAL>;
   constexpr int LD = P::LD, KS = P::KS, J = EC / 4, I = D / 64;
   extern __shared__ __align__(16) float sm[];
@@ -421,8 +428,8 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   const int h = (int)(blockIdx.x - part * H), col0 = (int)(part % slices) * EC;
   const int b = sequence_by_length(cu, B, (int)(part / slices));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int t0 = cu[b], t1 = cu[b + 1];
-  if (t1 - t0 < from) return;
+  const int t0 = max(cu[b], s0), t1 = min(cu[b + 1], s1);
+  if (cu[b + 1] - cu[b] < from || t0 >= t1) return;
   const Rows at = rows_of(H, D, e, GENERAL);
 
   // A thread copies the same 16 bytes of every kStep-th row, and the same of every cStep-th row
@@ -443,7 +450,7 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   };
   auto issue_wq = [&](int c0, int half) {
     const int n = min(kC, t1 - c0);
-    const float* base = ws + (size_t)c0 * at.ld;
+    const float* base = ws + (size_t)(c0 - s0) * at.ld;
     copy_rows(WQ, base, 0, n);
     float* dst = XO + half * P::kXO;
 #pragma unroll
@@ -456,7 +463,7 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
   };
   auto issue_k = [&](int c0) {
     const int n = min(kC, t1 - c0);
-    const float* base = ws + (size_t)c0 * at.ld;
+    const float* base = ws + (size_t)(c0 - s0) * at.ld;
     copy_rows(Kh, base, 2, n);
     if constexpr (GENERAL) {
       for (int t = ct; t < kC; t += cStep)
@@ -469,7 +476,7 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
                    : "memory");
     }
   };
-  if (t0 < t1) issue_wq(t0, 0);
+  issue_wq(t0, 0);
   asm volatile("cp.async.commit_group;" ::: "memory");
 
   // the thread's part of the state: columns jb .. jb+J-1 (in pairs), rows ib .. ib+I-1
@@ -600,21 +607,21 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
 template <int D, int EC, bool GENERAL>
 int launch_state_t(const float* ws, const float* v, int ldv, float* state, size_t stride,
                    const int* cu, const int* slot, int B, int H, int e, float* o_raw,
-                   int write_state, int from, cudaStream_t st) {
+                   int write_state, int from, int s0, int s1, cudaStream_t st) {
   constexpr int bytes = StatePlan<D, EC, GENERAL>::kFloats * 4;
   static_assert(bytes <= 227 * 1024, "a chunk's stages do not fit");
   auto kern = delta_chunk_state_kernel<D, EC, GENERAL>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return (int)err;
   kern<<<(unsigned)B * H * (e / EC), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
-                                                       o_raw, write_state, from);
+                                                       o_raw, write_state, from, s0, s1);
   return launch_status();
 }
 
 template <int D, bool GENERAL>
 int launch_state(const float* ws, const float* v, int ldv, float* state, size_t stride,
                  const int* cu, const int* slot, int B, int H, int e, float* o_raw,
-                 int write_state, int from, cudaStream_t st) {
+                 int write_state, int from, int s0, int s1, cudaStream_t st) {
   // Slices of 32 columns halve the reads of a chunk's rows; slices of 16 while 32 would not give
   // every SM its two CTAs (four sequences of 300 to 1,500 tokens, 16 heads of 128: 408 us in
   // slices of 16, 439 in slices of 32).
@@ -626,9 +633,9 @@ int launch_state(const float* ws, const float* v, int ldv, float* state, size_t 
   }();
   if (e % 32 == 0 && (long long)B * H * (e / 32) >= 2LL * sms)
     return launch_state_t<D, 32, GENERAL>(ws, v, ldv, state, stride, cu, slot, B, H, e, o_raw,
-                                          write_state, from, st);
+                                          write_state, from, s0, s1, st);
   return launch_state_t<D, 16, GENERAL>(ws, v, ldv, state, stride, cu, slot, B, H, e, o_raw,
-                                        write_state, from, st);
+                                        write_state, from, s0, s1, st);
 }
 
 template <typename K>
@@ -646,64 +653,88 @@ bool takes(int B, int H, int d, int e, const float* state, long long stride) {
 
 using namespace cretif;
 
-// Floats of workspace a token needs (times T), or 0 where the sizes are not taken.
+// Floats of workspace a token needs, or 0 where the sizes are not taken.
 extern "C" long long cretif_delta_chunk_row(int H, int d, int e, int general) {
   if (H <= 0 || (d != 64 && d != 128) || e <= 0 || e > 256 || e % 16) return 0;
   return rows_of(H, d, e, general != 0).ld;
 }
 
+namespace cretif {
+namespace {
+// Tokens of a span, whole chunks of them, for a workspace of that many floats; 0: it is too small, or
+// the step needs several spans and may not write the state that passes between them.
+int span_tokens(long long ws_floats, const Rows& at, int T, int write_state) {
+  const long long rows = ws_floats / at.ld;
+  if (rows >= T) return T;
+  return write_state ? (int)(rows / kC * kC) : 0;
+}
+}  // namespace
+}  // namespace cretif
+
 extern "C" int cretif_delta_chunks(const float* prep, int ldp, float* state, long long stride,
                                    const int* cu, const int* seq_slot, int B, int H, int G, int d,
-                                   int e, float* ws, float* o_raw, int write_state, int T,
-                                   int from, void* stream) {
+                                   int e, float* ws, long long ws_floats, float* o_raw,
+                                   int write_state, int T, int from, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (!takes(B, H, d, e, state, stride) || G <= 0 || H % G || ldp < 2 * G * d + H * e + 2 * H)
     return kBadArgument;
   if (ldp % 4 || (((uintptr_t)prep | (uintptr_t)ws | (uintptr_t)o_raw) & 15)) return kMisaligned;
+  const int step = span_tokens(ws_floats, rows_of(H, d, e, false), T, write_state);
+  if (step <= 0) return kBadArgument;
   cudaStream_t st = (cudaStream_t)stream;
-  const dim3 grid(T / kC + B, H);
   const int bytes = 4 * (2 * kC * (d + 4) + 3 * kC * kA + 2 * kC + kC * e);
   int rc = d == 64 ? allow_smem(delta_chunk_prepare_kernel<64>, bytes)
                    : allow_smem(delta_chunk_prepare_kernel<128>, bytes);
-  if (rc) return rc;
-  if (d == 64)
-    delta_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from);
-  else
-    delta_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from);
-  if ((rc = launch_status())) return rc;
-  return d == 64 ? launch_state<64, false>(ws, nullptr, 0, state, (size_t)stride, cu, seq_slot, B,
-                                           H, e, o_raw, write_state, from, st)
+  for (int s0 = 0; s0 < T && !rc; s0 += step) {
+    const int s1 = T - s0 < step ? T : s0 + step;
+    const dim3 grid((s1 - s0) / kC + B, H);
+    if (d == 64)
+      delta_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from,
+                                                               s0, s1);
+    else
+      delta_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(prep, ldp, ws, cu, B, H, G, e, from,
+                                                                s0, s1);
+    if ((rc = launch_status())) return rc;
+    rc = d == 64 ? launch_state<64, false>(ws, nullptr, 0, state, (size_t)stride, cu, seq_slot, B, H,
+                                           e, o_raw, write_state, from, s0, s1, st)
                  : launch_state<128, false>(ws, nullptr, 0, state, (size_t)stride, cu, seq_slot, B,
-                                            H, e, o_raw, write_state, from, st);
+                                            H, e, o_raw, write_state, from, s0, s1, st);
+  }
+  return rc;
 }
 
 extern "C" int cretif_general_delta_chunks(const float* proj, int ldp, const float* prep, int ldq,
                                            float* state, long long stride, const int* cu,
                                            const int* seq_slot, int B, int H, int d, int e,
-                                           float* ws, float* o_raw, int write_state, int T,
-                                           int from, void* stream) {
+                                           float* ws, long long ws_floats, float* o_raw,
+                                           int write_state, int T, int from, void* stream) {
   if (B <= 0 || T <= 0) return kOk;
   if (!takes(B, H, d, e, state, stride) || ldp < 2 * H * d + H * e || ldq < 3 * H * d)
     return kBadArgument;
   if (ldp % 4 || ldq % 4 ||
       (((uintptr_t)proj | (uintptr_t)prep | (uintptr_t)ws | (uintptr_t)o_raw) & 15))
     return kMisaligned;
+  const int step = span_tokens(ws_floats, rows_of(H, d, e, true), T, write_state);
+  if (step <= 0) return kBadArgument;
   cudaStream_t st = (cudaStream_t)stream;
-  const dim3 grid(T / kC + B, H);
   const int bytes = 4 * (3 * kC * (d + 4) + 4 * kC * kA + 2 * kC * e);
   int rc = d == 64 ? allow_smem(general_chunk_prepare_kernel<64>, bytes)
                    : allow_smem(general_chunk_prepare_kernel<128>, bytes);
-  if (rc) return rc;
-  if (d == 64)
-    general_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
-                                                               e, from);
-  else
-    general_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
-                                                                e, from);
-  if ((rc = launch_status())) return rc;
   const float* v = proj + 2 * (size_t)H * d;
-  return d == 64 ? launch_state<64, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H, e,
-                                          o_raw, write_state, from, st)
-                 : launch_state<128, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H,
-                                           e, o_raw, write_state, from, st);
+  for (int s0 = 0; s0 < T && !rc; s0 += step) {
+    const int s1 = T - s0 < step ? T : s0 + step;
+    const dim3 grid((s1 - s0) / kC + B, H);
+    if (d == 64)
+      general_chunk_prepare_kernel<64><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
+                                                                 e, from, s0, s1);
+    else
+      general_chunk_prepare_kernel<128><<<grid, 128, bytes, st>>>(proj, ldp, prep, ldq, ws, cu, B, H,
+                                                                  e, from, s0, s1);
+    if ((rc = launch_status())) return rc;
+    rc = d == 64 ? launch_state<64, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H, e,
+                                          o_raw, write_state, from, s0, s1, st)
+                 : launch_state<128, true>(ws, v, ldp, state, (size_t)stride, cu, seq_slot, B, H, e,
+                                           o_raw, write_state, from, s0, s1, st);
+  }
+  return rc;
 }

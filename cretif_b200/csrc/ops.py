@@ -403,6 +403,10 @@ DELTA_CHUNKS_FROM = 64
 # (9 heads of 64 by 256 tokens, walk and chunks: 16 sequences 122 and 100 us, 32 161 and 170, 64
 # 261 and 329).
 DELTA_CHUNKS_HEADS64 = 256
+# The chunks' workspace at most (16 heads of 128 x 128 take 41 KB a token, of the general rule 57 KB);
+# a longer step goes through it span by span (9,000 tokens and more: a launch of both kernels each,
+# whose sequences still fill the chip).
+DELTA_CHUNKS_BYTES = 512 << 20
 # A sequence of fewer tokens than this is walked all the same, in a launch beside the chunks', where
 # there are that many heads of such sequences or more: a lone token in a chunk costs all of the
 # chunk's work, which a few of them hide under the long sequences'.  Microseconds, everything walked,
@@ -421,10 +425,12 @@ def _delta_short(news, H: int) -> int:
 
 
 def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: bool, state, rows,
-                      short: int = 0):
+                      short: int = 0, write_state: bool = True):
     """The workspace of a step whose delta rule goes in chunks, or None where it walks token by
     token: few tokens, or sizes and strides that the chunk kernels' 16-byte accesses do not take.
-    ``short``: how many of the step's ``T`` tokens are walked all the same."""
+    ``short``: how many of the step's ``T`` tokens are walked all the same.  A step beyond
+    DELTA_CHUNKS_BYTES gets a workspace for a part of its tokens, and none where it may not
+    write the state between the parts; so does a step for which there is no memory left."""
     if longest < DELTA_CHUNKS_FROM or (d == 64
                                        and (T - short) * H > DELTA_CHUNKS_HEADS64 * longest):
         return None
@@ -433,7 +439,19 @@ def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: boo
     row = int(lib().cretif_delta_chunk_row(H, d, e, int(general)))
     if not row or state.stride(0) % 4 or state.data_ptr() % 16 or H > 65535:
         return None
-    return torch.empty(T * row, dtype=torch.float32, device=state.device)
+    most = DELTA_CHUNKS_BYTES // (4 * row)
+    if T > most and (not write_state or most < 32):
+        return None
+    try:
+        return torch.empty(min(T, most) * row, dtype=torch.float32, device=state.device)
+    except torch.OutOfMemoryError:
+        return None
+
+
+def _delta_chunk_launches(ws, T: int, H: int, d: int, e: int, general: bool) -> int:
+    """Kernels that a step launches with that workspace: two a span of whole chunks."""
+    rows = ws.numel() // int(lib().cretif_delta_chunk_row(H, d, e, int(general)))
+    return 2 * (1 if rows >= T else -(-T // (rows // 32 * 32)))
 
 
 def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G: int, d: int,
@@ -452,13 +470,14 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
     T = prep.shape[0]
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=prep.device)
     short = _delta_short(news, H)
-    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), short)
+    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), short, write_state)
     below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_delta_chunks(
             _p(prep), _rows(prep, "prep"), _p(state), ctypes.c_longlong(state.stride(0)),
-            _p(cu_seqlens), _p(seq_slot), B, H, G, d, e, _p(ws), _p(o_raw), int(write_state), T,
-            below, _stream()), "delta_chunks", kernels=2)
+            _p(cu_seqlens), _p(seq_slot), B, H, G, d, e, _p(ws),
+            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()), "delta_chunks",
+            kernels=_delta_chunk_launches(ws, T, H, d, e, False))
         if not below:
             return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
     _check(lib().cretif_delta_recurrence(
@@ -1067,13 +1086,14 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
         raise KernelError("general_delta_recurrence: sizes do not fit")
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=proj.device)
     short = _delta_short(news, H)
-    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), short)
+    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), short, write_state)
     below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_general_delta_chunks(
             _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(state),
             ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, d, e, _p(ws),
-            _p(o_raw), int(write_state), T, below, _stream()), "general_delta_chunks", kernels=2)
+            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()), "general_delta_chunks",
+            kernels=_delta_chunk_launches(ws, T, H, d, e, True))
         if not below:
             return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
     _check(lib().cretif_general_delta_recurrence(

@@ -170,3 +170,76 @@ def test_mixed_steps(general, H, G, d, e, lens):
         assert torch.equal(out[at[b]:at[b + 1]], want[0][at[b]:at[b + 1]]), b
         assert torch.equal(state[b], want[1][b]), b
     assert not torch.equal(out, walked[0]) and not torch.equal(out, chunked[0])
+
+
+@pytest.mark.parametrize("general,H,G,d,e", [(False, 4, 2, 64, 48), (True, 3, 3, 128, 32)])
+def test_the_workspace_has_a_bound(monkeypatch, general, H, G, d, e):
+    """A step beyond it goes span by span (spans that end inside a chunk, inside a sequence and between
+    two), and one that may not write its state between spans, or finds no memory, is walked."""
+    from cretif_b200.csrc import ops
+    row = int(ops.lib().cretif_delta_chunk_row(16, 128, 128, 1))
+    room = ops._delta_chunk_room(2048, 1 << 20, 16, 128, 128, True, torch.empty(1, 4, device="cuda"), ())
+    assert 4 * room.numel() <= ops.DELTA_CHUNKS_BYTES and room.numel() >= 2048 * row
+    del room
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    lens = (200, 0, 65, 2, 130)
+    T, B = sum(lens), len(lens)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+
+    def unit(x, heads):
+        x = x.view(T, heads, d)
+        return (x / x.norm(dim=2, keepdim=True)).reshape(T, heads * d)
+    decays = torch.rand(T, H * d if general else H, generator=gen, device="cuda") * 0.5 + 0.5
+    start, gate, norm_w = rand(B, H * d * e), rand(T, H * e), torch.ones(e, device="cuda")
+    slots = list(range(B))
+    if general:
+        key = unit(rand(T, H * d), H)
+        proj = torch.cat([rand(T, H * d), key, rand(T, H * e)], 1)
+        prep = torch.cat([key, -torch.rand(T, H * d, generator=gen, device="cuda") * key, decays], 1)
+        want, want_state = _general(proj, prep, start, lens, slots, H, d, e)
+    else:
+        prep = torch.cat([unit(rand(T, G * d), G), unit(rand(T, G * d), G), rand(T, H * e),
+                          torch.rand(T, H, generator=gen, device="cuda"), decays], 1)
+        want, want_state = _gated(prep, start, lens, slots, H, G, d, e)
+    w64 = want.view(T, H, e)
+    w64 = (w64 / torch.sqrt((w64 * w64).mean(2, keepdim=True) + 1e-5)).reshape(T, H * e)
+    w64 = w64 * (torch.sigmoid(gate.double()) if general else
+                 gate.double() * torch.sigmoid(gate.double()))
+    cu = torch.tensor([0] + list(lens)).cumsum(0).int().cuda()
+    seq_slot = torch.tensor(slots, dtype=torch.int32, device="cuda")
+
+    def step(longest, write_state=True):
+        state, out = start.clone(), torch.empty(T, H * e, device="cuda")
+        if general:
+            ops.general_delta_recurrence(proj, prep, gate, state, cu, seq_slot, B, H, d, e, norm_w, 1e-5,
+                                         out, per_head_weight=False, longest=longest,
+                                         write_state=write_state)
+        else:
+            ops.delta_recurrence(prep, gate, state, cu, seq_slot, B, H, G, d, e, norm_w, 1e-5, out,
+                                 longest=longest, write_state=write_state)
+        return out, state
+    whole, walked = step(200), step(1)
+    row = int(ops.lib().cretif_delta_chunk_row(H, d, e, int(general)))
+    for tokens in (32, 96, 100, 265, T - 1):
+        monkeypatch.setattr(ops, "DELTA_CHUNKS_BYTES", 4 * row * tokens)
+        before = ops.launch_count()
+        out, state = step(200)
+        assert ops.launch_count() - before == 2 * -(-T // (tokens // 32 * 32)) + 1, tokens
+        # (the bounds of test_chunks_against_the_formula)
+        assert _off(out, w64) <= 1e-6 and _off(state, want_state) <= 1e-6, tokens
+        out, state = step(200, write_state=False)
+        assert torch.equal(out, walked[0]) and torch.equal(state, start)
+    monkeypatch.setattr(ops, "DELTA_CHUNKS_BYTES", 4 * row * 31)
+    assert all(torch.equal(a, b) for a, b in zip(step(200), walked))
+    monkeypatch.setattr(ops, "DELTA_CHUNKS_BYTES", 4 * row * T)
+    assert all(torch.equal(a, b) for a, b in zip(step(200), whole))
+    empty = torch.empty
+
+    def full(*args, **kw):
+        if args and args[0] == T * row:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*args, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    assert all(torch.equal(a, b) for a, b in zip(step(200), walked))
