@@ -828,6 +828,23 @@ def retention_recurrence(prep, v, decay, state, cu_seqlens, seq_slot, B: int, H:
         "retention_recurrence")
 
 
+# The scanned chunks' workspace at most (16 heads of 128 x 128 take 16.5 KB a token); a longer step
+# walks its chunks, which needs none.
+MEMORY_SCAN_BYTES = 512 << 20
+
+
+def _memory_scan_room(T: int, B: int, H: int, d: int, e: int, device):
+    """The workspace of a step whose chunks are scanned, or None where they are walked: as
+    ``memory_scans`` says, where it is too large, or where no memory is left for it."""
+    floats = (T // 64 + B) * H * (d * e + d + 2)
+    if not memory_scans(T, B, H) or 4 * floats > MEMORY_SCAN_BYTES:
+        return None
+    try:
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def memory_scans(T: int, B: int, H: int) -> bool:
     """Whether a step's chunks of the matrix memory are scanned (matrix_memory.cu) instead of walked:
     sequences of 256 tokens or more on average, while the walk's CTAs (a few a sequence and head)
@@ -866,9 +883,7 @@ def matrix_memory(proj, bias_i, bias_f, cap: float, q_scale: float, state, cu_se
     scratch = torch.empty(n_o + 2 * T * H, dtype=torch.float32, device=proj.device)
     chunks = form in ("chunk", "walk") or (form == "auto" and T >= 16 * B)
     gates = torch.empty(3 * H * T, dtype=torch.float64, device=proj.device) if chunks else None
-    scan = chunks and form != "walk" and memory_scans(T, B, H)
-    ws = (torch.empty((T // 64 + B) * H * (d * e + d + 2), dtype=torch.float32, device=proj.device)
-          if scan else None)
+    ws = _memory_scan_room(T, B, H, d, e, proj.device) if chunks and form != "walk" else None
     _check(lib().cretif_matrix_memory(
         _p(proj), _rows(proj, "proj"), _p(bias_i), _p(bias_f), ctypes.c_float(cap),
         ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(cu_seqlens),
@@ -876,7 +891,7 @@ def matrix_memory(proj, bias_i, bias_f, cap: float, q_scale: float, state, cu_se
         _p(scratch[n_o:]), _p(scratch[n_o + T * H:]), _p(gates), _p(out), _dt(out),
         _rows(out, "out"), int(write_state), T,
         {"auto": 0, "token": 1, "chunk": 2, "walk": 3}[form], _p(ws), _stream()),
-        "matrix_memory", kernels=(4 if scan else 3) if chunks else 2)
+        "matrix_memory", kernels=(3 if ws is None else 4) if chunks else 2)
 
 
 def state_space(proj, conv_w, conv_b, a_log, dt_bias, d_skip, state, inputs_at: int, cu_seqlens,

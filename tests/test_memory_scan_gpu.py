@@ -39,3 +39,37 @@ def test_scan_and_walk(H, d, e, lens, write_state):
     assert bool(torch.isfinite(outs[0]).all())
     assert (outs[0] - outs[1]).norm() <= 1e-4 * outs[0].norm()
     assert (states[0] - states[1]).norm() <= 2e-6 * states[0].norm()
+
+
+def test_a_step_beyond_the_workspace_walks(monkeypatch):
+    """The scan's workspace has a bound, and a step that finds no memory for it still runs: by the
+    bits of the walk."""
+    from cretif_b200.csrc import ops
+    H, d, e, T = 2, 64, 64, 700
+    room = ops._memory_scan_room(T, 1, H, d, e, "cuda")
+    assert room is not None and 4 * room.numel() <= ops.MEMORY_SCAN_BYTES
+    assert ops._memory_scan_room(1 << 20, 1, 16, 128, 128, "cuda") is None     # 17 GB
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    proj = torch.randn(T, 2 * H * (d + e) + 2 * H, generator=gen, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    zero = torch.zeros(H, device="cuda")
+
+    def run(form):
+        state, out = torch.zeros(1, H * (d * (e + 1) + 1) + 2, device="cuda"), \
+            torch.empty(T, H * e, device="cuda")
+        ops.matrix_memory(proj, zero, zero, 12.0, 0.1, state, torch.tensor([0, T], **i32),
+                          torch.zeros(1, **i32), torch.zeros(T, **i32), 1, H, d, e,
+                          torch.ones(H * e, device="cuda"), 1e-6, out, form=form)
+        return out, state
+    walked = run("walk")
+    monkeypatch.setattr(ops, "MEMORY_SCAN_BYTES", 4 * room.numel() - 4)
+    assert all(torch.equal(a, b) for a, b in zip(run("auto"), walked))
+    monkeypatch.undo()
+    empty = torch.empty
+
+    def full(*args, **kw):
+        if args and args[0] == room.numel():
+            raise torch.OutOfMemoryError("no room")
+        return empty(*args, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    assert all(torch.equal(a, b) for a, b in zip(run("auto"), walked))
