@@ -185,6 +185,7 @@ enum Variant : int {
   kVarPrefillAttnSplit,     // ... one tile per CTA, its key steps split between two slots
   kVarTcBulkAdd,            // tcgen05 product added into a float32 matrix through TMA
   kVarTcPair,               // tcgen05 product with two CTAs on a tile (cta_group::2)
+  kVarDeltaPrepareRows,     // gated delta rule's preparation, eight tokens a warp
   kVarCount
 };
 void count_variant(int v);

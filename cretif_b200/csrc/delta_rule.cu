@@ -100,10 +100,10 @@ delta_prepare_kernel(const float* __restrict__ proj, int ldp, float* __restrict_
   }
 }
 
-// The same for a prompt's tokens with four taps and heads of up to 128 channels: a warp takes eight
+// The same for a prompt's tokens with four taps and heads of 65 to 128 channels: a warp takes eight
 // tokens of its unit in turn, a lane four neighbouring channels in 16-byte accesses, so a projected row
-// is read once, not once a tap, and the taps' weights stay in registers.  2,048 tokens of 6,144
-// channels: 105.7 -> 43.8 us (100 MB, 0.35 of the copy rate; the exponentials are next).
+// is read once, not once a tap, and the taps' weights stay in registers.  2,048 tokens of 4,096
+// channels: 62 -> 26 us (50 MB, 0.3 of the copy rate; the exponentials are next).
 constexpr int kPrepTokens = 8;
 
 __global__ void __launch_bounds__(kPrepWarps * 32)
@@ -468,9 +468,13 @@ extern "C" int cretif_delta_prepare(const float* proj, int ldp, float* prep, int
   dim3 grid(T, (units + kPrepWarps - 1) / kPrepWarps);
   if (grid.y > 65535) return kBadArgument;
   // Prompts whose rows 16-byte accesses take: eight tokens a warp.  (Below 256 tokens a warp a token
-  // has more loads in flight.)
-  if (T > 256 && taps == 4 && d <= 128 && d % 4 == 0 && e % 4 == 0 && ldp % 4 == 0 && ldo % 4 == 0 &&
+  // has more loads in flight.  Heads of 64 leave half of such a warp's lanes idle and gain nothing: us,
+  // a warp a token and eight tokens a warp, 4 heads 4.2 and 10.3 at 260 tokens, 16.4 and 17.8 at 2,048;
+  // 9 heads 6.3 and 10.4, 32.8 and 34.0; 16 heads of 128 10.3 and 7.8, 62 and 26.)
+  if (T > 256 && taps == 4 && d > 64 && d <= 128 && e > 64 && d % 4 == 0 && e % 4 == 0 &&
+      ldp % 4 == 0 && ldo % 4 == 0 &&
       (((uintptr_t)proj | (uintptr_t)prep | (uintptr_t)conv_w) & 15) == 0) {
+    count_variant(kVarDeltaPrepareRows);
     delta_prepare_rows_kernel<<<dim3((T + kPrepTokens - 1) / kPrepTokens, grid.y), kPrepWarps * 32, 0,
                                 (cudaStream_t)stream>>>(
         proj, ldp, prep, ldo, conv_w, conv_state, (size_t)state_stride, a_log, dt_bias, tok_pos,

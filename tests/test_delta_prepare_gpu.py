@@ -47,3 +47,22 @@ def test_prompt_rows(H, G, d, e, lens):
     for a, b in ((0, 2 * G * d), (2 * G * d, C), (C, C + H), (C + H, C + 2 * H)):
         off = (prep[:, a:b].double() - want[:, a:b]).norm() / want[:, a:b].norm()
         assert off <= 1e-6, (a, float(off))
+
+
+@pytest.mark.parametrize("H,G,d,e", [(2, 1, 96, 72), (1, 1, 68, 260), (5, 5, 128, 128)])
+@pytest.mark.parametrize("lens", [(1, 2, 3, 300, 4, 11), (257,), (248, 9)])
+def test_prompt_rows_of_wide_heads(H, G, d, e, lens):
+    """The sizes that go eight tokens a warp, odd ones among them; see above."""
+    from cretif_b200.csrc import ops
+    before = ops.variant_counts()["delta_prepare_rows"]
+    test_prompt_rows(H, G, d, e, lens)
+    assert ops.variant_counts()["delta_prepare_rows"] == before + 1
+
+
+@pytest.mark.parametrize("H,G,d,e", [(4, 4, 64, 64), (2, 1, 64, 128), (2, 1, 128, 64)])
+def test_narrow_heads_keep_a_warp_a_token(H, G, d, e):
+    """Heads of 64 leave half of the lanes idle that take eight tokens in turn."""
+    from cretif_b200.csrc import ops
+    before = ops.variant_counts()["delta_prepare_rows"]
+    test_prompt_rows(H, G, d, e, (260,))
+    assert ops.variant_counts()["delta_prepare_rows"] == before
