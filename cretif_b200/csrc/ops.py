@@ -403,6 +403,21 @@ DELTA_CHUNKS_FROM = 64
 # (9 heads of 64 by 256 tokens, walk and chunks: 16 sequences 122 and 100 us, 32 161 and 170, 64
 # 261 and 329).
 DELTA_CHUNKS_HEADS64 = 256
+
+
+def _delta_chunk_heads(d: int, e: int, general: bool) -> float:
+    """The same bound where the lengths of a step's sequences are known, counted in whole chunks of
+    them, for every size.  Walk and chunks at it, microseconds: heads of 64, gated 24 x 9 by 96 tokens
+    60 and 61, 28 x 9 61 and 71; general 28 x 9 111 and 108.  Heads of 128 by 32 columns share a
+    chunk's keys among few columns: gated 16 x 16 by 64 tokens 48 and 52, general 82 and 94, 8 x 16 57
+    and 51; by 64 columns, general 64 x 16 420 and 431, 64 x 32 802 and 849."""
+    if e < 64 or (d == 64 and not general):
+        return 200
+    if d == 64:
+        return 256
+    return 1024 if general and e < 128 else float("inf")
+
+
 # The chunks' workspace at most (16 heads of 128 x 128 take 41 KB a token, of the general rule 57 KB);
 # a longer step goes through it span by span (9,000 tokens and more: a launch of both kernels each,
 # whose sequences still fill the chip).
@@ -424,15 +439,25 @@ def _delta_short(news, H: int) -> int:
     return sum(short) if len(short) * H >= DELTA_WALK_HEADS else 0
 
 
+def _delta_in_chunks(news, short: int) -> int:
+    """The tokens of a step's chunks, the last one of every sequence counted as full (0: not known)."""
+    least = DELTA_WALK_BELOW if short else 1
+    return sum(-(-n // 32) * 32 for n in news if n >= least)
+
+
 def _delta_chunk_room(longest: int, T: int, H: int, d: int, e: int, general: bool, state, rows,
-                      short: int = 0, write_state: bool = True):
+                      write_state: bool = True, in_chunks: int = 0):
     """The workspace of a step whose delta rule goes in chunks, or None where it walks token by
     token: few tokens, or sizes and strides that the chunk kernels' 16-byte accesses do not take.
-    ``short``: how many of the step's ``T`` tokens are walked all the same.  A step beyond
+    ``in_chunks``: how many tokens the step's chunks hold (0: not known).  A step beyond
     DELTA_CHUNKS_BYTES gets a workspace for a part of its tokens, and none where it may not
     write the state between the parts; so does a step for which there is no memory left."""
-    if longest < DELTA_CHUNKS_FROM or (d == 64
-                                       and (T - short) * H > DELTA_CHUNKS_HEADS64 * longest):
+    if longest < DELTA_CHUNKS_FROM:
+        return None
+    if in_chunks:
+        if in_chunks * H > _delta_chunk_heads(d, e, general) * longest:
+            return None
+    elif d == 64 and T * H > DELTA_CHUNKS_HEADS64 * longest:
         return None
     if any(r.stride(0) % 4 or r.data_ptr() % 16 for r in rows):
         return None
@@ -470,7 +495,8 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
     T = prep.shape[0]
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=prep.device)
     short = _delta_short(news, H)
-    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), short, write_state)
+    ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), write_state,
+                           _delta_in_chunks(news, short))
     below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_delta_chunks(
@@ -1101,7 +1127,8 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
         raise KernelError("general_delta_recurrence: sizes do not fit")
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=proj.device)
     short = _delta_short(news, H)
-    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), short, write_state)
+    ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), write_state,
+                           _delta_in_chunks(news, short))
     below = DELTA_WALK_BELOW if ws is not None and short else 0
     if ws is not None:
         _check(lib().cretif_general_delta_chunks(

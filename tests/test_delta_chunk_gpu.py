@@ -243,3 +243,19 @@ def test_the_workspace_has_a_bound(monkeypatch, general, H, G, d, e):
         return empty(*args, **kw)
     monkeypatch.setattr(torch, "empty", full)
     assert all(torch.equal(a, b) for a, b in zip(step(200), walked))
+
+
+@pytest.mark.parametrize("general,H,d,e,lens,chunks", [
+    (False, 9, 64, 64, (96,) * 20, True), (False, 9, 64, 64, (96,) * 28, False),
+    (True, 9, 64, 64, (96,) * 28, True), (False, 9, 64, 64, (64,) + (48,) * 32, False),
+    (False, 9, 64, 64, (64,) + (1,) * 63, True), (False, 16, 128, 32, (64,) * 8, True),
+    (False, 16, 128, 32, (64,) * 16, False), (True, 32, 128, 64, (64,) * 64, False),
+    (False, 32, 128, 64, (64,) * 64, True), (True, 32, 128, 128, (64,) * 64, True)])
+def test_which_steps_go_in_chunks(general, H, d, e, lens, chunks):
+    """By the heads that the chunks keep in flight: the walk is as fast or faster beyond."""
+    from cretif_b200.csrc import ops
+    state, row = torch.zeros(1, 4, device="cuda"), torch.zeros(1, 4, device="cuda")
+    short = ops._delta_short(lens, H)
+    room = ops._delta_chunk_room(max(lens), sum(lens), H, d, e, general, state, (row,), True,
+                                 ops._delta_in_chunks(lens, short))
+    assert (room is not None) == chunks

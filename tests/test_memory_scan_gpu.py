@@ -62,6 +62,7 @@ def test_a_step_beyond_the_workspace_walks(monkeypatch):
                           torch.ones(H * e, device="cuda"), 1e-6, out, form=form)
         return out, state
     walked = run("walk")
+    assert not torch.equal(run("auto")[0], walked[0])          # (scanned)
     monkeypatch.setattr(ops, "MEMORY_SCAN_BYTES", 4 * room.numel() - 4)
     assert all(torch.equal(a, b) for a, b in zip(run("auto"), walked))
     monkeypatch.undo()
