@@ -186,6 +186,11 @@ enum Variant : int {
   kVarTcBulkAdd,            // tcgen05 product added into a float32 matrix through TMA
   kVarTcPair,               // tcgen05 product with two CTAs on a tile (cta_group::2)
   kVarDeltaPrepareRows,     // gated delta rule's preparation, eight tokens a warp
+  kVarF32Few,               // 32-bit product, few rows
+  kVarF32Tile64,            // ... 64 x 64 tiles
+  kVarF32Tile32,            // ... 32 x 32 tiles, the slabs dealt to four warps
+  kVarDeltaSlices32,        // chunks of a delta rule, 32 columns a CTA
+  kVarDeltaSlices16,        // ... 16
   kVarCount
 };
 void count_variant(int v);

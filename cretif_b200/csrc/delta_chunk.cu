@@ -613,6 +613,7 @@ int launch_state_t(const float* ws, const float* v, int ldv, float* state, size_
   auto kern = delta_chunk_state_kernel<D, EC, GENERAL>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return (int)err;
+  count_variant(EC == 32 ? kVarDeltaSlices32 : kVarDeltaSlices16);
   kern<<<(unsigned)B * H * (e / EC), 256, bytes, st>>>(ws, v, ldv, state, stride, cu, slot, B, H, e,
                                                        o_raw, write_state, from, s0, s1);
   return launch_status();

@@ -293,6 +293,7 @@ template <int MT, int NT>
 static int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
                       int ldc, int accumulate, cudaStream_t st) {
   constexpr int smem = few_smem(MT, NT);
+  count_variant(kVarF32Few);
   auto kern = gemm_f32_few_kernel<MT, NT>;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -309,6 +310,7 @@ static int launch_tile(const float* A, const float* W, float* C, int M, int N, i
                        int ldw, int ldc, int accumulate, cudaStream_t st) {
   constexpr int BM = 32 * WM, BN = 32 * WN;
   constexpr int smem = ring_of(KS) * KS * (BM + BN) * kRow * (int)sizeof(float);
+  count_variant(KS == 1 ? kVarF32Tile64 : kVarF32Tile32);
   auto kern = gemm_f32_tile_kernel<WM, WN, KS>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;

@@ -259,3 +259,16 @@ def test_which_steps_go_in_chunks(general, H, d, e, lens, chunks):
     room = ops._delta_chunk_room(max(lens), sum(lens), H, d, e, general, state, (row,), True,
                                  ops._delta_in_chunks(lens, short))
     assert (room is not None) == chunks
+
+
+@pytest.mark.parametrize("general,H,G", [(False, 16, 4), (True, 16, 16)])
+@pytest.mark.parametrize("lens,slices", [((70, 0, 33, 96, 1, 40), 32), ((200, 95), 16)])
+def test_slices_of_columns(general, H, G, lens, slices):
+    """Heads of 128 x 128 in both widths of a slice (32 columns from two CTAs an SM on), a short last
+    chunk and an empty sequence among them."""
+    from cretif_b200.csrc import ops
+    before = ops.variant_counts()
+    test_chunks_against_the_formula(general, H, G, 128, 128, lens)
+    after = ops.variant_counts()
+    assert {k for k in after if k.startswith("delta_slices") and after[k] != before[k]} \
+        == {"delta_slices%d" % slices}

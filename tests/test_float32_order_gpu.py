@@ -29,6 +29,35 @@ def test_a_row_of_the_product_does_not_depend_on_the_others(ops, N, K):  # noqa:
         assert torch.equal(c, whole[700 - m:]), m
 
 
+# every body at remainders in rows, columns and k, with strided rows and added onto what is there
+@pytest.mark.parametrize("M,N,K,body", [
+    (1, 577, 260, "few"), (2, 70, 2052, "few"), (3, 3081, 36, "few"), (5, 333, 8196, "few"),
+    (8, 9001, 132, "few"), (33, 577, 1540, "few"), (64, 130, 36, "few"),
+    (65, 577, 576, "tile32"), (24, 20001, 36, "tile32"), (130, 333, 8196, "tile32"), (577, 2305, 260, "tile32"),
+    (580, 2605, 260, "tile64"), (580, 2605, 36, "tile64"), (580, 2605, 4, "tile64"),
+    (1153, 1665, 2052, "tile64")])
+def test_product_bodies(ops, M, N, K, body):  # noqa: F811
+    a = rnd(M, K + 4)[:, :K]
+    w = rnd(N, K, seed=1)
+    c = torch.full((M, N + 3), 7.0, device=DEV)
+    before = ops.variant_counts()
+    ops.gemm_simt(a, w, c[:, :N])
+    after = ops.variant_counts()
+    assert {k for k in after if after[k] != before[k]} == {"f32_" + body}
+    want = a.double() @ w.double().T
+    close(c[:, :N], want, 2e-6)
+    assert bool((c[:, N:] == 7.0).all())
+    ops.gemm_simt(a, w, c[:, :N], accumulate=True)
+    close(c[:, :N], 2 * want, 2e-6)
+    # 2-norm: a slab's two chains of 16, their sum and K / 128 slabs four times over, each rounding to
+    # 2^-24 of a partial sum, random in sign
+    plain = torch.empty(M, N, device=DEV)
+    ops.gemm_simt(a, w, c[:, :N])
+    ops.gemm_simt(a, w, plain, plain=True)
+    off, plain_off = (float((x.double() - want).norm() / want.norm()) for x in (c[:, :N], plain))
+    assert off <= 2.0 ** -24 * (16 + 4 + K / 128) ** 0.5 + 1e-8, (off, plain_off)
+
+
 @pytest.mark.parametrize("M", [1, 8, 33])
 def test_a_vocabulary_of_262144(ops, M):  # noqa: F811
     """More columns than four times a grid's second dimension still take the fast bodies: their bits, by

@@ -74,3 +74,43 @@ def test_a_step_beyond_the_workspace_walks(monkeypatch):
         return empty(*args, **kw)
     monkeypatch.setattr(torch, "empty", full)
     assert all(torch.equal(a, b) for a, b in zip(run("auto"), walked))
+
+
+@pytest.mark.parametrize("H,d,e,lens", [(2, 64, 64, (600,)), (1, 128, 48, (320, 300)), (3, 20, 32, (777,))])
+@pytest.mark.parametrize("strong", [False, True])
+def test_scan_and_walk_against_64_bits(H, d, e, lens, strong):
+    """Both forms beside the recurrence written out in 64 bits: the scan may be no further from it than
+    the walk by more than half (each is one draw of the same rounding), and neither than 1e-5 of the
+    read-outs' 2-norm: 2^-24 times the square root of some hundred terms, normed up where a read-out is a
+    small difference of large ones."""
+    import plain_gibipel as plain
+    from cretif_b200.csrc import ops
+    from test_gibipel_gpu import _gates
+    gen = torch.Generator().manual_seed(12)
+    T, B, cap, qs = sum(lens), len(lens), 10.0, d ** -0.5
+    assert ops.memory_scans(T, B, H)
+    parts, want = [], []
+    for n in lens:
+        q, k, v = (torch.randn(n, H * x, generator=gen) for x in (d, d, e))
+        gate = torch.randn(n, H * e, generator=gen)
+        zi, zf = _gates(gen, n, H, strong)
+        parts.append(torch.cat([q, k, v, gate, zi, zf], 1))
+        li = cap * torch.tanh(zi.double() / cap)
+        lf = plain.log_sigmoid(cap * torch.tanh(zf.double() / cap))
+        o = plain.memory(q.double().reshape(n, H, d) * qs, k.double().reshape(n, H, d),
+                         v.double().reshape(n, H, e), li, lf)
+        want.append(plain.unit(o, 1e-5).reshape(n, H * e) * torch.sigmoid(gate.double()))
+    proj, want = torch.cat(parts), torch.cat(want)
+    proj = torch.nn.functional.pad(proj, (0, -proj.shape[1] % 4)).cuda()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + list(lens)).cumsum(0).int().cuda()
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).int().cuda()
+    zero, off = torch.zeros(H, device="cuda"), {}
+    for form in ("walk", "chunk", "token"):
+        state = torch.zeros(B, -(-(H * (d * (e + 1) + 1)) // 4) * 4, device="cuda")
+        out = torch.empty(T, H * e, device="cuda")
+        ops.matrix_memory(proj, zero, zero, cap, qs, state, cu, torch.arange(B, **i32), seq, B, H, d, e,
+                          torch.ones(H * e, device="cuda"), 1e-5, out, form=form)
+        off[form] = float((out.cpu().double() - want).norm() / want.norm())
+    print(off)
+    assert off["chunk"] <= 1.5 * max(off["walk"], off["token"]) and max(off.values()) <= 1e-5, off
