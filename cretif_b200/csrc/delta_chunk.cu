@@ -88,7 +88,10 @@ __device__ __forceinline__ Span find_span(const int* cu, int B, int x, int from,
 //     y_t = out_t + sum_{s<=t} E[t][s] x_s (+ sum_{s<=t} F[t][s] v_s),
 // eight tokens at a time.  The matrices are stored with s first, so that eight tokens' factors
 // are two 16-byte reads that the whole warp shares, for sixteen two-wide FMAs; a token's sums
-// never touch later tokens' values.  x goes to shared memory (X, row stride ldx) for the rows to
+// never touch later tokens' values.  rhs_t, the larger part of x_t, joins its corrections when they are
+// summed: as the first term of the chain it was rounded with each of them.  (With that, the prepared rows
+// first in the state's products and one chain over a head's channels, state and read-outs of the gated
+// rule were 1.65e-7 and 2.1e-7 from 64 bits, now 0.95e-7 and 1.5e-7, the token walk's figures.)  x goes to shared memory (X, row stride ldx) for the rows to
 // come.  (The whole substitution unrolled with x in registers ran at a third of this: 50 KB of
 // straight-line code, and 160 registers a thread.)
 template <bool TWO, typename Rhs, typename Out, typename Store>
@@ -97,9 +100,10 @@ __device__ __forceinline__ void substitute(float* X, int ldx, const float* V, in
                                            const float* F, int n, Rhs rhs, Out out, Store store) {
 #pragma unroll 1
   for (int t8 = 0; t8 < n; t8 += 8) {
-    float2 x[8], y[8];
+    float2 x[8], y[8], own[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = rhs(t8 + j), y[j] = out(t8 + j);
+    for (int j = 0; j < 8; ++j)
+      own[j] = rhs(t8 + j), x[j] = make_float2(0.f, 0.f), y[j] = out(t8 + j);
     auto add = [&](const float* m, float2* acc, float2 z, int from) {
       const float4 lo = *reinterpret_cast<const float4*>(m);
       const float4 hi = *reinterpret_cast<const float4*>(m + 4);
@@ -122,6 +126,7 @@ __device__ __forceinline__ void substitute(float* X, int ldx, const float* V, in
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int s = t8 + j;
+      x[j] = make_float2(own[j].x + x[j].x, own[j].y + x[j].y);
       if (TWO) {
         const float2 vs = *reinterpret_cast<const float2*>(V + s * ldv);
         add(Bv + s * kA + t8, x, vs, j + 1);
@@ -193,29 +198,37 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, int ldp, float* __res
     // a warp gives eight tokens' products with all earlier ones; the four warps take the
     // chunk's quarters
     const int t = tid >> 2, s0 = tid & 3, last = (tid >> 5) * 2 + 2;
-    float2 kk[8], qk[8];
+    float kk[8], qk[8];
 #pragma unroll
-    for (int y = 0; y < 8; ++y) kk[y] = qk[y] = make_float2(0.f, 0.f);
+    for (int y = 0; y < 8; ++y) kk[y] = qk[y] = 0.f;
+#pragma unroll 1
+    for (int i0 = 0; i0 < D; i0 += 32) {     // (32 channels on their own: eight terms a chain)
+      float2 k2[8], q2[8];
+#pragma unroll
+      for (int y = 0; y < 8; ++y) k2[y] = q2[y] = make_float2(0.f, 0.f);
 #pragma unroll 2
-    for (int i = 0; i < D; i += 4) {
-      const float4 kt = *reinterpret_cast<const float4*>(Ks + t * LD + i);
-      const float4 qt = *reinterpret_cast<const float4*>(Qs + t * LD + i);
+      for (int i = i0; i < i0 + 32; i += 4) {
+        const float4 kt = *reinterpret_cast<const float4*>(Ks + t * LD + i);
+        const float4 qt = *reinterpret_cast<const float4*>(Qs + t * LD + i);
 #pragma unroll
-      for (int y = 0; y < 8; ++y) {
-        if (y >= last) break;
-        const float4 ks = *reinterpret_cast<const float4*>(Ks + (s0 + 4 * y) * LD + i);
-        kk[y] = __ffma2_rn(make_float2(kt.x, kt.y), make_float2(ks.x, ks.y), kk[y]);
-        kk[y] = __ffma2_rn(make_float2(kt.z, kt.w), make_float2(ks.z, ks.w), kk[y]);
-        qk[y] = __ffma2_rn(make_float2(qt.x, qt.y), make_float2(ks.x, ks.y), qk[y]);
-        qk[y] = __ffma2_rn(make_float2(qt.z, qt.w), make_float2(ks.z, ks.w), qk[y]);
+        for (int y = 0; y < 8; ++y) {
+          if (y >= last) break;
+          const float4 ks = *reinterpret_cast<const float4*>(Ks + (s0 + 4 * y) * LD + i);
+          k2[y] = __ffma2_rn(make_float2(kt.x, kt.y), make_float2(ks.x, ks.y), k2[y]);
+          k2[y] = __ffma2_rn(make_float2(kt.z, kt.w), make_float2(ks.z, ks.w), k2[y]);
+          q2[y] = __ffma2_rn(make_float2(qt.x, qt.y), make_float2(ks.x, ks.y), q2[y]);
+          q2[y] = __ffma2_rn(make_float2(qt.z, qt.w), make_float2(ks.z, ks.w), q2[y]);
+        }
       }
+#pragma unroll
+      for (int y = 0; y < 8; ++y) kk[y] += k2[y].x + k2[y].y, qk[y] += q2[y].x + q2[y].y;
     }
 #pragma unroll
     for (int y = 0; y < 8; ++y) {
       const int s = s0 + 4 * y;
       const float r = R[s * kA + t];
-      A[s * kA + t] = s < t ? -beta[t] * (r * (kk[y].x + kk[y].y)) : 0.f;
-      E[s * kA + t] = s <= t ? r * (qk[y].x + qk[y].y) : 0.f;
+      A[s * kA + t] = s < t ? -beta[t] * (r * kk[y]) : 0.f;
+      E[s * kA + t] = s <= t ? r * qk[y] : 0.f;
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -548,11 +561,12 @@ delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__
 #pragma unroll
     for (int i = 0; i < (2 * kC + cStep - 1) / cStep; ++i) {
       const int r = ct + i * cStep;
-      float4 sum = *reinterpret_cast<const float4*>(xo + r * EC + cc);
+      const float* rp = red + r * (EC + 4) + cc;
+      float4 sum = *reinterpret_cast<const float4*>(rp);
 #pragma unroll
-      for (int k = 0; k < KS; ++k) {
-        const float4 p =
-            *reinterpret_cast<const float4*>(red + (k * 2 * kC + r) * (EC + 4) + cc);
+      for (int k = 1; k <= KS; ++k) {
+        const float4 p = *reinterpret_cast<const float4*>(
+            k < KS ? rp + k * 2 * kC * (EC + 4) : xo + r * EC + cc);
         sum.x += p.x, sum.y += p.y, sum.z += p.z, sum.w += p.w;
       }
       if (r < kC)

@@ -272,3 +272,53 @@ def test_slices_of_columns(general, H, G, lens, slices):
     after = ops.variant_counts()
     assert {k for k in after if k.startswith("delta_slices") and after[k] != before[k]} \
         == {"delta_slices%d" % slices}
+
+
+@pytest.mark.parametrize("general,H,G,d,e", [(False, 8, 4, 128, 64), (False, 9, 9, 64, 64),
+                                             (True, 8, 8, 128, 64)])
+@pytest.mark.parametrize("T", [64, 300])
+def test_chunks_are_as_exact_as_the_walk(general, H, G, d, e, T):
+    """Both round the same terms to 32 bits; the 2-norms are over 20,000 numbers and more, so that two
+    orders of like exactness differ by a few parts in a hundred."""
+    from cretif_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(2)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+
+    def uniform(*shape):
+        return torch.rand(*shape, generator=gen, device="cuda")
+
+    def unit(x, heads):
+        x = x.view(T, heads, d)
+        return (x / x.norm(dim=2, keepdim=True)).reshape(T, heads * d)
+    decays = torch.exp(-0.2 * uniform(T, H * d if general else H))
+    start, gate, norm_w = torch.zeros(1, H * d * e, device="cuda"), rand(T, H * e), torch.ones(e, device="cuda")
+    if general:
+        key = unit(rand(T, H * d), H)
+        proj = torch.cat([rand(T, H * d), key, rand(T, H * e)], 1)
+        prep = torch.cat([key, -uniform(T, H * d) * key, decays], 1)
+        want, want_state = _general(proj, prep, start, [T], [0], H, d, e)
+    else:
+        prep = torch.cat([unit(rand(T, G * d), G), unit(rand(T, G * d), G), rand(T, H * e), uniform(T, H),
+                          decays], 1)
+        prep = torch.nn.functional.pad(prep, (0, -prep.shape[1] % 4))[:, :prep.shape[1]]
+        want, want_state = _gated(prep, start, [T], [0], H, G, d, e)
+    w64 = want.view(T, H, e)
+    w64 = (w64 / torch.sqrt((w64 * w64).mean(2, keepdim=True) + 1e-5)).reshape(T, H * e)
+    w64 = w64 * (torch.sigmoid(gate.double()) if general else
+                 gate.double() * torch.sigmoid(gate.double()))
+    cu = torch.tensor([0, T], dtype=torch.int32, device="cuda")
+    slot = torch.zeros(1, dtype=torch.int32, device="cuda")
+    off = {}
+    for longest in (1, T):
+        state, out = start.clone(), torch.empty(T, H * e, device="cuda")
+        if general:
+            ops.general_delta_recurrence(proj, prep, gate, state, cu, slot, 1, H, d, e, norm_w, 1e-5, out,
+                                         per_head_weight=False, longest=longest)
+        else:
+            ops.delta_recurrence(prep, gate, state, cu, slot, 1, H, G, d, e, norm_w, 1e-5, out,
+                                 longest=longest)
+        off[longest] = _off(out, w64), _off(state, want_state)
+    for chunks, walk in zip(off[T], off[1]):
+        assert chunks <= 1.25 * walk, off
