@@ -83,8 +83,6 @@ int cretif_delta_recurrence(const float* prep, int ldp, const float* gate, int l
                             float* o_raw, void* out, int out_dt, int ldo, int write_state, int T,
                             int below, void* stream);
 
-// Dynamic Tanh, dyt(x) = (tanh(alpha x) w + b) gain, a norm without statistics (pointwise_norm.cu);
-// alpha points at one float on the device, gain may be null.
 // The same recurrences over prompts in chunks of 32 tokens (delta_chunk.cu), read-outs before
 // their norm into o_raw [T, H e].  ws: float32 workspace of ws_floats, cretif_delta_chunk_row(...) a
 // token (0: sizes not taken; d is 64 or 128, e a multiple of 16); one that does not hold all tokens (32
@@ -101,6 +99,8 @@ int cretif_general_delta_chunks(const float* proj, int ldp, const float* prep, i
                                 long long ws_floats, float* o_raw, int write_state, int T,
                                 int from, void* stream);
 
+// Dynamic Tanh, dyt(x) = (tanh(alpha x) w + b) gain, a norm without statistics (pointwise_norm.cu);
+// alpha points at one float on the device, gain may be null.
 // dyt_rows: v = h[src] (+ delta[src]); if write_h, h[src] = v; out[r] = dyt(v); src = rows ? rows[r] : r.
 int cretif_dyt_rows(float* h, const void* delta, int delta_dt, const float* w, const float* b,
                     const float* alpha, const float* gain, void* out, int out_dt, const int* rows,

@@ -26,7 +26,8 @@
 // read-outs, walk -> chunks: 16 heads of 128 x 128, one sequence of 2,048 tokens 996 -> 242 (the
 // general rule 1,468 -> 360), four of 300 to 1,500 870 -> 408 (1,668 -> 610), sixteen of 256
 // 468 -> 339 (866 -> 558); 9 heads of 64 x 64, one of 2,048 822 -> 125 (1,091 -> 189).  What
-// bounds the state kernel is issue: two CTAs an SM keep the FMA pipe about half busy.
+// bounds the state kernel is shared memory's pipe (ncu: stalls on it 4.1 an issue, the FMA pipe busy 39 %
+// of the time with two CTAs an SM).
 #include "api.h"
 #include "common.cuh"
 
@@ -91,9 +92,9 @@ __device__ __forceinline__ Span find_span(const int* cu, int B, int x, int from,
 // never touch later tokens' values.  rhs_t, the larger part of x_t, joins its corrections when they are
 // summed: as the first term of the chain it was rounded with each of them.  (With that, the prepared rows
 // first in the state's products and one chain over a head's channels, state and read-outs of the gated
-// rule were 1.65e-7 and 2.1e-7 from 64 bits, now 0.95e-7 and 1.5e-7, the token walk's figures.)  x goes to shared memory (X, row stride ldx) for the rows to
-// come.  (The whole substitution unrolled with x in registers ran at a third of this: 50 KB of
-// straight-line code, and 160 registers a thread.)
+// rule were 1.65e-7 and 2.1e-7 from 64 bits, now 0.95e-7 and 1.5e-7, the token walk's figures.)  x
+// goes to shared memory (X, row stride ldx) for the rows to come.  (The whole substitution unrolled with
+// x in registers ran at a third of this: 50 KB of straight-line code, and 160 registers a thread.)
 template <bool TWO, typename Rhs, typename Out, typename Store>
 __device__ __forceinline__ void substitute(float* X, int ldx, const float* V, int ldv,
                                            const float* A, const float* E, const float* Bv,
@@ -416,8 +417,8 @@ struct StatePlan {
 
 // One buffer for what the products read (W, Q), refilled while the update runs, one for what the
 // update reads (K, K2, V, decays), refilled while the products run: two CTAs share an SM and hide
-// each other's barriers (with two stages of everything one CTA filled it and its FMA pipe was
-// busy 44 % of the time).
+// each other's barriers (with two stages of everything one CTA filled it: 490 us against 456 for eight
+// prompts; of the general rule with heads of 128 one CTA of 32 columns fits all the same).
 template <int D, int EC, bool GENERAL>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_state_kernel(const float* __restrict__ ws, const float* __restrict__ v, int ldv,
@@ -637,9 +638,11 @@ template <int D, bool GENERAL>
 int launch_state(const float* ws, const float* v, int ldv, float* state, size_t stride,
                  const int* cu, const int* slot, int B, int H, int e, float* o_raw,
                  int write_state, int from, int s0, int s1, cudaStream_t st) {
-  // Slices of 32 columns halve the reads of a chunk's rows; slices of 16 while 32 would not give
-  // every SM its two CTAs (four sequences of 300 to 1,500 tokens, 16 heads of 128: 408 us in
-  // slices of 16, 439 in slices of 32).
+  // Slices of 32 columns halve the reads of a chunk's rows; slices of 16 while there are fewer than two
+  // of 32 an SM (four sequences of 300 to 1,500 tokens, 16 heads of 128: 408 us in slices of 16, 439 in
+  // slices of 32).  Of the general rule with heads of 128 one CTA of 32 columns fits an SM (128 KB) and
+  // is still the faster one from there on: 5 x 512 tokens 419 us in slices of 32, 417 of 16, 8 x 512 589
+  // and 599, 32 x 256 1,099 and 1,185.
   static const int sms = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
@@ -659,8 +662,8 @@ int allow_smem(K kern, int bytes) {
 }
 
 bool takes(int B, int H, int d, int e, const float* state, long long stride) {
-  return (long long)B * H * (e / 16) <= 0x7fffffffLL && (d == 64 || d == 128) && e > 0 && e <= 256 && e % 16 == 0 && H > 0 && H <= 65535 &&
-         stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
+  return (d == 64 || d == 128) && e > 0 && e <= 256 && e % 16 == 0 && H > 0 && H <= 65535 &&
+         (long long)B * H * (e / 16) <= 0x7fffffffLL && stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
 }
 
 }  // namespace

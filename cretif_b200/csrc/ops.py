@@ -503,8 +503,8 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
         _check(lib().cretif_delta_chunks(
             _p(prep), _rows(prep, "prep"), _p(state), ctypes.c_longlong(state.stride(0)),
             _p(cu_seqlens), _p(seq_slot), B, H, G, d, e, _p(ws),
-            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()), "delta_chunks",
-            kernels=_delta_chunk_launches(ws, T, H, d, e, False))
+            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()),
+            "delta_chunks", kernels=_delta_chunk_launches(ws, T, H, d, e, False))
         if not below:
             return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e)
     _check(lib().cretif_delta_recurrence(
@@ -1135,8 +1135,8 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
         _check(lib().cretif_general_delta_chunks(
             _p(proj), _rows(proj, "proj"), _p(prep), _rows(prep, "prep"), _p(state),
             ctypes.c_longlong(state.stride(0)), _p(cu_seqlens), _p(seq_slot), B, H, d, e, _p(ws),
-            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()), "general_delta_chunks",
-            kernels=_delta_chunk_launches(ws, T, H, d, e, True))
+            ctypes.c_longlong(ws.numel()), _p(o_raw), int(write_state), T, below, _stream()),
+            "general_delta_chunks", kernels=_delta_chunk_launches(ws, T, H, d, e, True))
         if not below:
             return heads_out_norm(o_raw, gate, norm_w, eps, out, H, e, per_head_weight, gate_sigmoid)
     _check(lib().cretif_general_delta_recurrence(

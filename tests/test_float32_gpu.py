@@ -10,8 +10,9 @@ from test_kernels_gpu import DEV, ToyCache, close, ops, rnd  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
-# rows around the few-row body's tiles (1, 2, 4, 8), its last row count and the tiles' edges; columns
-# around a warp's four and a tile's 32 and 64; k around a lane's four, a slab's 32 and a warp's 128
+# rows around the few-row body's tiles (1, 2, 4, 8) and its last row count; columns around a CTA's 4, 8 and 32;
+# k around a lane's four and a slab's 32.  (All but the last rows go to the few-row body and the 32 x 32
+# tiles; test_float32_order_gpu.py names the body of every shape, the 64 x 64 tiles among them.)
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 64, 65, 130])
 @pytest.mark.parametrize("N,K", [(1, 4), (5, 36), (33, 128), (70, 132), (577, 576), (2305, 260)])
 def test_product(ops, M, N, K):  # noqa: F811
