@@ -274,7 +274,7 @@ __host__ __device__ inline int memory_chunk_ld(int d) {
 inline size_t memory_intra_smem(int d) {
   return sizeof(double) * 2 * kMcTokens +
          sizeof(float) * (2 * (size_t)kMcTokens * memory_chunk_ld(d) + (size_t)kMcTokens * kMcSlab +
-                          (size_t)kMcTokens * kMcScoreLd + kMcTokens);
+                          (size_t)kMcTokens * kMcScoreLd);
 }
 inline size_t memory_carry_smem(int d, int ec, int nbuf) {
   return sizeof(double) * 3 * kMcTokens * nbuf +
@@ -309,6 +309,7 @@ __device__ __forceinline__ void memory_chunk(const int* cu, int B, int x, int& b
 __global__ void __launch_bounds__(kMcThreads)
 memory_intra_kernel(const MemArgs a, double* __restrict__ gates, const ChunkSums cs) {
   extern __shared__ __align__(16) float smem[];
+  __shared__ float sW[kMcTokens];          // a token's weight in the chunk's own sum
   constexpr int C = kMcTokens;
   constexpr int LP = kMcScoreLd;
   const int tid = threadIdx.x, H = a.H, d = a.d, e = a.e;
@@ -325,7 +326,6 @@ memory_intra_kernel(const MemArgs a, double* __restrict__ gates, const ChunkSums
   float* sK = sQ + C * ldq;                          // [C][ldq]
   float* sV = sK + C * ldq;                          // [C][kMcSlab]
   float* sP = sV + C * kMcSlab;                      // [C][LP]
-  float* sW = sP + C * LP;                           // [C] a token's weight in the chunk's own sum
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // q and k of the chunk's tokens, copied asynchronously.  Rows beyond the chunk's last token stay as
   // they are: they reach only scores of rows that are not stored, or of keys after the row, which

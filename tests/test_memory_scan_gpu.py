@@ -114,3 +114,25 @@ def test_scan_and_walk_against_64_bits(H, d, e, lens, strong):
         off[form] = float((out.cpu().double() - want).norm() / want.norm())
     print(off)
     assert off["chunk"] <= 1.5 * max(off["walk"], off["token"]) and max(off.values()) <= 1e-5, off
+
+
+@pytest.mark.parametrize("d", [364, 368, 372])
+def test_the_widest_heads_in_chunks(d):
+    """Heads whose chunk fills the shared memory that the kernels take are not refused: chunks beside token
+    by token (read-outs by their 2-norm, as above)."""
+    from cretif_b200.csrc import ops
+    H, e, T = 1, 16, 300
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    proj = torch.randn(T, -(-(2 * H * (d + e) + 2 * H) // 4) * 4, generator=gen, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    zero, got = torch.zeros(H, device="cuda"), []
+    for form in ("chunk", "walk", "token"):
+        state = torch.zeros(1, -(-(H * (d * (e + 1) + 1)) // 4) * 4, device="cuda")
+        out = torch.empty(T, H * e, device="cuda")
+        ops.matrix_memory(proj, zero, zero, 12.0, d ** -0.5, state, torch.tensor([0, T], **i32),
+                          torch.zeros(1, **i32), torch.zeros(T, **i32), 1, H, d, e,
+                          torch.ones(H * e, device="cuda"), 1e-6, out, form=form)
+        got.append((out, state))
+    for out, state in got[:2]:
+        assert (out - got[2][0]).norm() <= 1e-4 * out.norm()
+        assert (state - got[2][1]).norm() <= 2e-6 * state.norm()
