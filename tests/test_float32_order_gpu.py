@@ -203,3 +203,41 @@ def test_scores_without_bounds(ops):  # noqa: F811
         close(out[1], others, 2e-6)
         assert bool(torch.isnan(out[2]).all())
     assert torch.equal(outs[0][:2], outs[1][:2])
+
+
+def test_logits_of_small_steps_do_not_depend_on_the_cut(tmp_path):
+    """A whole float32 model with heads of 64: a prompt alone, beside others, in two cuts and token by token
+    gives the same bits, as long as its steps bring fewer than 64 tokens (from there on the norms sum a
+    row in another order)."""
+    from cretif_b200.engine import Engine
+    from cretif_b200.weights.random_model import write_random_model
+    config = {"architectures": ["LlamaForCausalLM"], "hidden_size": 192, "num_hidden_layers": 2,
+              "num_attention_heads": 3, "num_key_value_heads": 1, "intermediate_size": 320,
+              "vocab_size": 500, "rope_theta": 10000.0, "rms_norm_eps": 1e-5,
+              "tie_word_embeddings": True, "max_position_embeddings": 256}
+    write_random_model(str(tmp_path), config, seed=4)
+    engine = Engine(str(tmp_path), dtype="float32", max_tokens=1024, step_graphs=False)
+    gen = torch.Generator().manual_seed(3)
+    texts = [torch.randint(500, (n,), generator=gen).tolist() for n in (31, 5, 20)]
+
+    def logits(cuts):
+        """Logits [sum of the first text's tokens] of a list of steps, each {text: tokens it brings}."""
+        slots, at, rows = {}, {}, []
+        for step in cuts:
+            for b in step:
+                if b not in slots:
+                    slots[b], at[b] = engine.alloc_slot(), 0
+            entries = [(slots[b], texts[b][at[b]:at[b] + n]) for b, n in step.items()]
+            out, first = engine.step(entries, "all"), 0
+            for b, n in step.items():
+                if b == 0:
+                    rows.append(out[first:first + n])
+                first += n
+                at[b] += n
+        for s in slots.values():
+            engine.free_slot(s)
+        return torch.cat(rows)
+    alone = logits([{0: 31}])
+    for cuts in ([{1: 5, 0: 31, 2: 20}], [{0: 13, 2: 20}, {0: 18}], [{0: 30, 1: 5}, {2: 20, 0: 1}],
+                 [{2: 20}] + [{0: 1}] * 31, [{1: 1, 0: 1} for _ in range(5)] + [{0: 26}]):
+        assert torch.equal(logits(cuts), alone), cuts
