@@ -433,6 +433,11 @@ DELTA_WALK_BELOW = 8
 DELTA_WALK_HEADS = 256
 
 
+def _delta_lengths(longest: int, news):
+    """``news`` where a step's lengths matter: beside a sequence that is long enough for chunks."""
+    return news if longest >= DELTA_CHUNKS_FROM else ()
+
+
 def _delta_short(news, H: int) -> int:
     """The tokens of a step's sequences that are walked beside the chunks of the others (0 where
     ``news``, how many each brings, is not known)."""
@@ -495,6 +500,7 @@ def delta_recurrence(prep, gate, state, cu_seqlens, seq_slot, B: int, H: int, G:
         raise KernelError("delta_recurrence: the state's sizes do not fit")
     T = prep.shape[0]
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=prep.device)
+    news = _delta_lengths(longest, news)
     short = _delta_short(news, H)
     ws = _delta_chunk_room(longest, T, H, d, e, False, state, (prep,), write_state,
                            _delta_in_chunks(news, short))
@@ -1127,6 +1133,7 @@ def general_delta_recurrence(proj, prep, gate, state, cu_seqlens, seq_slot, B: i
             or out.shape[1] < H * e or norm_w.numel() != (H * e if per_head_weight else e)):
         raise KernelError("general_delta_recurrence: sizes do not fit")
     o_raw = torch.empty((T, H * e), dtype=torch.float32, device=proj.device)
+    news = _delta_lengths(longest, news)
     short = _delta_short(news, H)
     ws = _delta_chunk_room(longest, T, H, d, e, True, state, (proj, prep), write_state,
                            _delta_in_chunks(news, short))
