@@ -107,8 +107,6 @@ static long long g_stream_min_bytes = 16LL << 20;
 static const int g_stream_max_rows = 64;
 // Depth of the streaming ring; 0: chosen per launch.
 static const int g_stream_stages = 0;
-// Stages of weights asked for before the kernel waits for the kernel before it.
-static const int g_stream_early = 1;
 
 template <int NT, int PRO, int EPI>
 static int launch_stream(const FusedParams& whole, int tiles, cudaStream_t st) {
@@ -172,7 +170,7 @@ static int launch_stream(const FusedParams& whole, int tiles, cudaStream_t st) {
   }
   count_variant(groups > 1 ? kVarStreamRowGroups : kVarStream);
   cudaError_t e = cudaLaunchKernelEx(&cfg, skinny_stream_kernel<NT, PRO, EPI>, whole, map_w, map_x,
-                                     tiles, stages, g_stream_early);
+                                     tiles, stages);
   return e == cudaSuccess ? launch_status() : (int)e;
 }
 
