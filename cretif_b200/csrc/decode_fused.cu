@@ -16,7 +16,7 @@ void count_variant(int v) {
 // Largest cluster that shares a norm prologue (1: none; at most kFuClusterMax).
 static int g_fused_cluster = kFuClusterMax;
 
-template <int NT, int PRO, int EPI>
+template <int NT, int PRO, int EPI, int PRE = 3>
 static int launch_fused(const FusedParams& p, int tiles, cudaStream_t st, int groups = 1,
                         int group_rows = 0) {
   if (groups == 1) group_rows = p.M;
@@ -24,7 +24,7 @@ static int launch_fused(const FusedParams& p, int tiles, cudaStream_t st, int gr
   static size_t configured = 48 * 1024;
   if (smem > configured) {
     if (smem > 200 * 1024) return kBadArgument;
-    cudaError_t e = cudaFuncSetAttribute(skinny_fused_kernel<NT, PRO, EPI>,
+    cudaError_t e = cudaFuncSetAttribute(skinny_fused_kernel<NT, PRO, EPI, PRE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     configured = smem;
@@ -75,17 +75,21 @@ static int launch_fused(const FusedParams& p, int tiles, cudaStream_t st, int gr
     }
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, skinny_fused_kernel<NT, PRO, EPI>, p, tiles,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, skinny_fused_kernel<NT, PRO, EPI, PRE>, p, tiles,
                                        group_rows);
     return e == cudaSuccess ? launch_status() : (int)e;
   }
-  skinny_fused_kernel<NT, PRO, EPI><<<grid, kFuWarps * 32, smem, st>>>(p, tiles, group_rows);
+  skinny_fused_kernel<NT, PRO, EPI, PRE><<<grid, kFuWarps * 32, smem, st>>>(p, tiles, group_rows);
   return launch_status();
 }
 
-// The register variant for any number of rows up to kFuMaxRows.
+// The register variant for any number of rows up to kFuMaxRows; held: as registers_hold says.
 template <int PRO, int EPI>
-static int dispatch_registers(const FusedParams& p, int tiles, cudaStream_t st) {
+static int dispatch_registers(const FusedParams& p, int tiles, cudaStream_t st, bool held = false) {
+  if (held && p.K > 1536) return launch_fused<1, PRO, EPI, 8>(p, tiles, st);
+  if (held && p.K > 768)
+    return p.M <= 8 ? launch_fused<1, PRO, EPI, 6>(p, tiles, st)
+                    : launch_fused<2, PRO, EPI, 6>(p, tiles, st);
   if (p.M <= 8) return launch_fused<1, PRO, EPI>(p, tiles, st);
   if (p.M <= 16) return launch_fused<2, PRO, EPI>(p, tiles, st);
   if (p.M <= kFuMaxGroupRows) return launch_fused<4, PRO, EPI>(p, tiles, st);
@@ -101,7 +105,8 @@ static int dispatch_registers(const FusedParams& p, int tiles, cudaStream_t st) 
 
 // Matrices at least this wide, or this large, stream through shared memory
 // (decode_stream.cuh); narrow small ones are latency and do better without the copy unit.
-static int g_stream_min_k = 768;
+constexpr int kStreamMinK = 768;
+static int g_stream_min_k = kStreamMinK;
 static long long g_stream_min_bytes = 16LL << 20;
 // ... and up to this many tokens (beyond 16 as groups of 16 rows that each stream the matrix)
 static const int g_stream_max_rows = 64;
@@ -174,9 +179,29 @@ static int launch_stream(const FusedParams& whole, int tiles, cudaStream_t st) {
   return e == cudaSuccess ? launch_status() : (int)e;
 }
 
+// Matrices beyond kStreamMinK columns of which every CTA holds its whole tile in registers before the
+// wait: what is left behind it is x, the product and its reduction, without the ring's barriers and
+// without x behind the weights in the copy unit's queue.  One wave of tiles (a second tile's weights
+// come in one by one), and few rows: 135M's down product, microseconds a decode step streamed and held:
+// 432 and 401 alone, 610 and 566 at 16 rows, but 760 and 839 at 32; 360M (K = 960, with its norm)
+// 619 and 548 alone, 683 and 654 at 8 rows, 906 and 852 at 16, but 548 and 596 alone with its
+// gate|up's 320 tiles.  Beyond 5 MB the plain epilogue only pays for one or two rows (1.7B's o product,
+// 8.4 MB: 950 and 922 alone, but 1,016 and 1,049 at 3 rows and 1,202 and 1,252 at 8: the next product's
+// ring starts filling under it, in front of its x), the gated one always (a shared expert beside the
+// routed ones, whose CTAs a ring of 200 KB keeps off the SM: Pudorax m at 8 rows 1,348 and 1,250).
+template <int PRO, int EPI>
+static bool registers_hold(const FusedParams& p, int tiles, long long w_bytes) {
+  if (g_stream_min_k != kStreamMinK || p.M > 16 || p.K > (p.M <= 8 ? 2048 : 1536) || tiles > 2 * kSmCount)
+    return false;
+  const bool large = p.M <= 2 || (PRO == kProPlain && EPI == kEpiSilu);
+  return w_bytes <= (large ? 9LL << 20 : 5LL << 20);
+}
+
 template <int PRO, int EPI>
 static int dispatch_nt(const FusedParams& p, int tiles, cudaStream_t st) {
   const long long w_bytes = 2LL * tiles * kFuRows * p.K;
+  if (p.K >= kStreamMinK && registers_hold<PRO, EPI>(p, tiles, w_bytes))
+    return dispatch_registers<PRO, EPI>(p, tiles, st, true);
   if ((p.K >= g_stream_min_k || w_bytes >= g_stream_min_bytes) && p.M <= g_stream_max_rows) {
     if (p.M <= 8) return launch_stream<1, PRO, EPI>(p, tiles, st);
     return launch_stream<2, PRO, EPI>(p, tiles, st);      // groups of 16 rows beyond 16

@@ -538,17 +538,18 @@ __device__ __forceinline__ void norm_rows_to_cluster(const FusedParams& p, unsig
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-constexpr int kFuPre = 3;      // weight chunks per warp fetched ahead (covers K <= 768)
+// PRE: weight chunks of 32 columns that a warp asks for ahead of the wait and holds in registers: 3, 6 or
+// 8 (every chunk for K up to 768, 1,536 or 2,048; a wider K fetches the rest in its loop).
 
-template <int EPI>
+template <int EPI, int PRE>
 __device__ __forceinline__ void fetch_weights(const FusedParams& p, int tile, int warp, int r, int c,
-                                              int n_chunks, uint4 (&pa)[kFuPre], uint4 (&pb)[kFuPre]) {
+                                              int n_chunks, uint4 (&pa)[PRE], uint4 (&pb)[PRE]) {
   const int row_a = tile_row<EPI>(p, tile, r), row_b = tile_row<EPI>(p, tile, r + 8);
   const __nv_bfloat16* wa = p.W + (size_t)max(row_a, 0) * p.ldw + c * 8;
   const __nv_bfloat16* wb = p.W + (size_t)max(row_b, 0) * p.ldw + c * 8;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int i = 0; i < kFuPre; ++i) {
+  for (int i = 0; i < PRE; ++i) {
     const int ch = warp + kFuWarps * i;
     const bool in = ch < n_chunks && ch * 32 + c * 8 < p.K;
     pa[i] = in ? __ldg(reinterpret_cast<const uint4*>(wa + ch * 32)) : zero;
@@ -559,7 +560,7 @@ __device__ __forceinline__ void fetch_weights(const FusedParams& p, int tile, in
 // The body of the fused product for the CTA's share of tiles: tiles first_tile,
 // first_tile + tile_stride, ...  `pdl`: signal/await the neighbouring launches
 // (programmatic dependent launch).
-template <int NT, int PRO, int EPI>
+template <int NT, int PRO, int EPI, int PRE>
 __device__ __forceinline__ void skinny_fused_tiles(const FusedParams& p, int n_tiles,
                                                    unsigned char* fsmem, int first_tile,
                                                    int tile_stride, bool pdl) {
@@ -587,8 +588,8 @@ __device__ __forceinline__ void skinny_fused_tiles(const FusedParams& p, int n_t
   // The first tile's weights do not depend on anything computed before this kernel: ask for
   // them first, so that their latency runs under the prologue.
   int tile = first_tile;
-  uint4 pa[kFuPre], pb[kFuPre];
-  if (tile < n_tiles) fetch_weights<EPI>(p, tile, warp, r, c, n_chunks, pa, pb);
+  uint4 pa[PRE], pb[PRE];
+  if (tile < n_tiles) fetch_weights<EPI, PRE>(p, tile, warp, r, c, n_chunks, pa, pb);
   // Programmatic dependent launch: the kernel behind this one may start its own weight
   // fetch now, and this one goes on to read activations only when the kernel before it has
   // finished (a no-op when the launch was an ordinary one).
@@ -651,13 +652,31 @@ __device__ __forceinline__ void skinny_fused_tiles(const FusedParams& p, int n_t
         mma_16816(acc[t], a2, ux.z, ux.w);
       }
     };
+    if (PRO == kProPlain && NT == 1) {
+      // x of all these chunks is asked for at once, not a chunk at a time between the products
+      uint4 xr[PRE];
 #pragma unroll
-    for (int i = 0; i < kFuPre; ++i) consume(pa[i], pb[i], warp + kFuWarps * i);
-    if (n_chunks > kFuWarps * kFuPre) {
+      for (int i = 0; i < PRE; ++i) {
+        const int ch = warp + kFuWarps * i, k = ch * 32 + c * 8;
+        xr[i] = (ch < n_chunks && k < p.K && r < p.M)
+                    ? __ldcg(reinterpret_cast<const uint4*>(p.X + (size_t)r * p.ldx + k)) : zero;
+      }
+#pragma unroll
+      for (int i = 0; i < PRE; ++i) {
+        const uint32_t a1[4] = {pa[i].x, pb[i].x, pa[i].y, pb[i].y};
+        const uint32_t a2[4] = {pa[i].z, pb[i].z, pa[i].w, pb[i].w};
+        mma_16816(acc[0], a1, xr[i].x, xr[i].y);
+        mma_16816(acc[0], a2, xr[i].z, xr[i].w);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < PRE; ++i) consume(pa[i], pb[i], warp + kFuWarps * i);
+    }
+    if (n_chunks > kFuWarps * PRE) {
       const int row_a = tile_row<EPI>(p, tile, r), row_b = tile_row<EPI>(p, tile, r + 8);
       const __nv_bfloat16* wa = p.W + (size_t)max(row_a, 0) * p.ldw + c * 8;
       const __nv_bfloat16* wb = p.W + (size_t)max(row_b, 0) * p.ldw + c * 8;
-      for (int ch = warp + kFuWarps * kFuPre; ch < n_chunks; ch += 2 * kFuWarps) {
+      for (int ch = warp + kFuWarps * PRE; ch < n_chunks; ch += 2 * kFuWarps) {
         const int ch2 = ch + kFuWarps;
         const bool in1 = ch * 32 + c * 8 < p.K, in2 = ch2 < n_chunks && ch2 * 32 + c * 8 < p.K;
         const uint4 ua1 = in1 ? __ldg(reinterpret_cast<const uint4*>(wa + ch * 32)) : zero;
@@ -670,7 +689,7 @@ __device__ __forceinline__ void skinny_fused_tiles(const FusedParams& p, int n_t
     }
     // the next tile's weights travel while this tile is reduced and finished
     if (tile + tile_stride < n_tiles)
-      fetch_weights<EPI>(p, tile + tile_stride, warp, r, c, n_chunks, pa, pb);
+      fetch_weights<EPI, PRE>(p, tile + tile_stride, warp, r, c, n_chunks, pa, pb);
 
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -710,13 +729,13 @@ __host__ __device__ inline FusedParams rows_of(const FusedParams& p, int m0, int
 constexpr int kFuMaxGroupRows = 32;
 constexpr int kFuMaxRows = 128;
 
-template <int NT, int PRO, int EPI>
+template <int NT, int PRO, int EPI, int PRE>
 __global__ void __launch_bounds__(kFuWarps * 32, 2)
 skinny_fused_kernel(const FusedParams p, int n_tiles, int group_rows) {
   extern __shared__ __align__(16) unsigned char fsmem_k[];
   const int m0 = blockIdx.y * group_rows;            // one group: all rows from 0
   const FusedParams q = rows_of(p, m0, min(group_rows, p.M - m0));
-  skinny_fused_tiles<NT, PRO, EPI>(q, n_tiles, fsmem_k, blockIdx.x, gridDim.x, true);
+  skinny_fused_tiles<NT, PRO, EPI, PRE>(q, n_tiles, fsmem_k, blockIdx.x, gridDim.x, true);
 }
 
 inline size_t fused_smem(int nt, int pro, int M, int K) {

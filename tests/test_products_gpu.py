@@ -1,0 +1,32 @@
+"""The matrix products' further bodies against float64: weights held in registers for few rows, the
+float32 store through TMA, q|k|v with two CTAs on a tile."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, ToyCache, _norm_bf16, close, ops, rnd  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(48, 768), (40, 776), (576, 1536), (33, 1544), (130, 2048), (16, 2056),
+                                 # beyond one wave of tiles: the ring again
+                                 (4800, 960)])
+def test_held_in_registers(ops, M, N, K):  # noqa: F811
+    """Around every depth of the register body and the widths where it gives way to the ring.  Sums of K
+    exact products of bfloat16 in 32 bits: 1e-5 of the largest; normed rows are rounded once more."""
+    w = rnd(N, K, dtype=torch.bfloat16, seed=2)
+    x = rnd(M, K, dtype=torch.bfloat16, seed=4)
+    before = ops.variant_counts()
+    base = rnd(M, N, seed=5)
+    acc = base.clone()
+    ops.fused_linear_add(x, w, acc)
+    after = ops.variant_counts()
+    close(acc, base.double().cpu() + x.double().cpu() @ w.double().cpu().T, 1e-5)
+    held = K <= (2048 if M <= 8 else 1536) and N <= 296 * 16
+    assert (after["fused_registers"] > before["fused_registers"]) == held
+    assert (after["stream"] > before["stream"]) == (not held)
+    h, nw = rnd(M, K), rnd(K, seed=1) * 0.1 + 1
+    out = torch.empty(M, N, device=DEV)
+    ops.fused_norm_linear(h, nw, 1e-5, w, out)
+    close(out, _norm_bf16(h, nw, 1e-5) @ w.double().cpu().T, 3e-3)
