@@ -87,7 +87,7 @@ __host__ __device__ constexpr bool tc_is_store(int epi) {
 
 struct TcEpi {
   void* C; int ldc, accumulate;                            // store
-  int bulk;        // through TMA (map_c): the float32 add of kTcStore, the store of kTcSilu
+  int bulk;        // through TMA (map_c): the float32 add or store of kTcStore, the store of kTcSilu
   __nv_bfloat16* act; int I;                               // silu
   __nv_bfloat16* Q; int ldq;                               // rope
   const float* cos_t; const float* sin_t;
@@ -338,7 +338,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (i == 0) stamp(3);
       const uint32_t lane_acc = tmem_acc + (uint32_t)(buf * BN) + ((uint32_t)(quad * 32) << 16);
       if (kBulk && ep.bulk) {
-        // The tile is added into the float32 matrix by TMA: a row per thread would touch 32
+        // The tile is added into (or stored as) the float32 matrix by TMA: a row per thread would touch 32
         // different lines with every load and store, and the old values would pass through
         // the SM at all.  Each group of four warps (128 rows, half of the columns) writes a
         // slab of 32 columns into shared memory in the 128-byte swizzle (eight 16-byte stores
@@ -367,7 +367,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           tc::fence_proxy_async();
           asm volatile("bar.sync %0, 128;" ::"r"(1 + chalf) : "memory");
           if (elected) {                   // (a group for every slab, or the count above is off)
-            if (ok && n0 + c0 < N) tc::tma_reduce_add_2d(&map_c, slab, n0 + c0, m0);
+            if (ok && n0 + c0 < N) {
+              if (accumulate) tc::tma_reduce_add_2d(&map_c, slab, n0 + c0, m0);
+              else tc::tma_store_2d(&map_c, slab, n0 + c0, m0);
+            }
             tc::bulk_commit_group();
           }
         }
@@ -1080,13 +1083,25 @@ static int launch_tc(const void* A, const void* W, const TcEpi& ep_in, int M, in
   // 11.4, x 1,536 29.6 -> 20.6; 2,048 x 576 x 1,536 13.7 -> 12.0; 2,048 x 960 x 2,560 22.6 -> 17.2;
   // 2,048 x 2,048 x 2,048 28.2 -> 26.1; with K = 8,192 the stages it takes away cost more than
   // it saves (69.6 -> 94.2).
+  // The plain float32 store takes the same way where its slabs cost no CTA an SM its place (128-wide
+  // tiles with four epilogue warps would go from two CTAs to one: the Rigozen mix's prompt 3,514 ->
+  // 3,547).  Prompts, us a pass, before and after: Losorax m 5,272 -> 5,015, Pudorax m 8,651 -> 8,201,
+  // Mipurax m 3,993 -> 3,847, Gibipel s 1,470 -> 1,392, Virorax s 1,949 -> 1,886 (the input products
+  // into 32-bit rows and the experts' down products).
   ep.bulk = 0;
-  if (tc_is_store(EPI) && sizeof(TC) == 4 && ep.accumulate && K <= 4096 && g_tc_bulk_add && ep.ldc % 4 == 0 && ((uintptr_t)ep.C & 15) == 0 &&
+  if (tc_is_store(EPI) && sizeof(TC) == 4 && !ep.unary && !ep.mul && K <= 4096 && g_tc_bulk_add &&
+      ep.ldc % 4 == 0 && ((uintptr_t)ep.C & 15) == 0 &&
       make_box_map(&map_c, ep.C, M, N, ep.ldc, kTcBM, 32, true, true) == 0) {
-    ep.bulk = 1;
-    stages = TcSmem<BN>::stages_with_staging(stages, epi_warps / 2);
-    smem = TcSmem<BN>::total(stages, epi_warps / 2);
-    count_variant(kVarTcBulkAdd);
+    const int with = TcSmem<BN>::stages_with_staging(stages, epi_warps / 2);
+    const int plain = smem, before = residents(epi_warps);
+    smem = TcSmem<BN>::total(with, epi_warps / 2);
+    if (ep.accumulate || tiles <= sm_count || residents(epi_warps) == before) {
+      ep.bulk = 1;
+      stages = with;
+      count_variant(kVarTcBulkAdd);
+    } else {
+      smem = plain;
+    }
   }
   if (tc_is_gated(EPI) && epi_warps == 8 && BN == 256 && g_tc_bulk_add &&
       make_box_map(&map_c, ep.act, M, ep.I, ep.I, kTcBM, 64, true, false) == 0) {

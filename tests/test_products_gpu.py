@@ -30,3 +30,27 @@ def test_held_in_registers(ops, M, N, K):  # noqa: F811
     out = torch.empty(M, N, device=DEV)
     ops.fused_norm_linear(h, nw, 1e-5, w, out)
     close(out, _norm_bf16(h, nw, 1e-5) @ w.double().cpu().T, 3e-3)
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(300, 200, 72, 0), (129, 68, 136, 64), (70, 1000, 1544, 128),
+                                      (1000, 960, 576, 192), (2100, 2048, 264, 256), (20000, 520, 72, 256)])
+def test_float32_store_through_tma(ops, M, N, K, bn):  # noqa: F811
+    """Stored by the threads and through TMA: the same numbers, tails clipped, the padding beside the
+    matrix untouched; with a factor as well."""
+    x, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1)
+    want = x.double() @ w.double().T
+    ldc = -(-N // 8) * 8 + 8
+    got, took = [], []
+    for bulk in (False, True):
+        for alpha in (1.0, -0.7):
+            old = ops.set_tc_bulk_add(bulk)
+            before = ops.variant_counts()["tc_bulk_add"]
+            full = torch.full((M, ldc), 7.0, device=DEV)
+            ops.gemm_tc(x, w, full[:, :N], bn=bn, alpha=alpha)
+            ops.set_tc_bulk_add(old)
+            took.append(ops.variant_counts()["tc_bulk_add"] > before)
+            close(full[:, :N], alpha * want, 1e-5)
+            assert bool((full[:, N:] == 7.0).all())
+            got.append(full)
+    assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[3])
+    assert not any(took[:2]) and (all(took[2:]) or bn in (64, 128, 192))
