@@ -642,7 +642,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // both, and each ends up with its 128 rows of the accumulator in its own tensor memory: 64
 // bytes a cycle per SM.  The loads of both CTAs are counted on CTA 0's barriers; its commits
 // arrive on the barriers of both.  Epilogues: the float32 add and the SiLU store through
-// shared-memory slabs and TMA, as above.
+// shared-memory slabs and TMA, as above, and the rotary one, whose warps turn a head's columns into
+// whole lines in 4 KB of shared memory each.
 constexpr int kTpThreads = 320;         // producer, issuer, eight epilogue warps
 template <int kTpBN>                    // the tile's width: 256, or 192 for widths like 576 and 960
 struct TpSmem {
@@ -766,11 +767,124 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int tile = pair + i * n_pairs;
       const int mt = tile / n_n_tiles, nt = tile - mt * n_n_tiles;
       const int m0 = mt * 2 * kTcBM + (int)rank * kTcBM, n0 = nt * kTpBN;
+      // Rotary epilogue: where the row goes (position -> slot -> cache block) and its angles do not
+      // need the product: their loads run while it does.
+      const int hd = ep.hd, half = hd >> 1, units = EPI == kTcRope ? hd >> 6 : 0;
+      const int head0 = EPI == kTcRope ? n0 / hd : 0, m = m0 + row;
+      const bool row_ok = EPI == kTcRope && m < M;
+      int pos = 0, blk = -1;
+      float cs_r[EPI == kTcRope ? 32 : 1], sn_r[EPI == kTcRope ? 32 : 1];
+      auto load_angles = [&](int u) {
+        const float* cs = ep.cos_t + (size_t)pos * half + 32 * u;
+        const float* sn = ep.sin_t + (size_t)pos * half + 32 * u;
+#pragma unroll
+        for (int j = 0; j < (EPI == kTcRope ? 32 : 0); j += 8) {
+          float c8[8], s8[8];
+          load8(cs + j, c8);
+          load8(sn + j, s8);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { cs_r[j + e] = c8[e]; sn_r[j + e] = s8[e]; }
+        }
+      };
+      if (EPI == kTcRope) {
+        if (row_ok) {
+          pos = ep.tok_pos[m];
+          if (ep.write_cache && head0 + kTpBN / hd > ep.nh) {
+            blk = ep.table[(size_t)ep.seq_slot[ep.tok_seq[m]] * ep.table_stride + pos / ep.bt];
+            if (blk < 0) atomicOr(fault, kFaultBlockTable);
+          }
+        }
+        if (units == 1 && head0 < ep.nh + ep.nkv) load_angles(0);
+      }
       alive = tc::mbar_wait(&acc_full[buf], (uint32_t)((i >> 1) & 1), abort) && alive;
       const bool ok = alive;
       tc::tc_fence_after();
       const uint32_t lane_acc = tmem_acc + (uint32_t)(buf * kTpBN) + ((uint32_t)(quad * 32) << 16);
-      if (tc_is_store(EPI)) {
+      if (EPI == kTcRope) {
+        // 64 columns of a head at a time: rotated (or not), rounded, into this warp's 32 rows of
+        // shared memory (swizzled, conflict-free), and from there with eight lanes a row, so that
+        // a store writes whole 128-byte lines.
+        unsigned char* mine = staging + (warp - 2) * (32 * 128);
+        for (int hh = chalf; hh * hd < kTpBN; hh += 2) {
+          const int head = head0 + hh;
+          if (head >= ep.nh + 2 * ep.nkv) break;
+          const bool rotate = head < ep.nh + ep.nkv, query = head < ep.nh;
+          // where this lane's row of the head goes, in elements (-1: nowhere)
+          long long at = -1;
+          if (ok && row_ok) {
+            if (query) at = (long long)m * ep.ldq + (long long)head * hd;
+            else if (blk >= 0)
+              at = (((long long)blk * ep.nkv + (rotate ? head - ep.nh : head - ep.nh - ep.nkv)) * ep.bt +
+                    pos % ep.bt) * hd;
+          }
+          __nv_bfloat16* const base = query ? ep.Q : rotate ? ep.kc : ep.vc;
+          for (int u = 0; u < units; ++u) {
+            const bool split = rotate && ep.pairing == 0;
+            const int c_lo = split ? 32 * u : 64 * u, c_hi = split ? half + 32 * u : 64 * u + 32;
+            uint32_t lo[32], hi[32];
+            tc::tmem_load_32(lane_acc + (uint32_t)(hh * hd + c_lo), lo);
+            tc::tmem_load_32(lane_acc + (uint32_t)(hh * hd + c_hi), hi);
+            if (rotate && units > 1) load_angles(u);
+            tc::tmem_load_wait();
+            __syncwarp();                              // the rows before have been read
+            auto put = [&](int piece, const float (&v)[8]) {
+              store8(reinterpret_cast<__nv_bfloat16*>(mine + lane * 128 + ((piece ^ (lane & 7)) << 4)), v);
+            };
+            if (!rotate) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 8) {
+                float a[8], b[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { a[e] = __uint_as_float(lo[j + e]); b[e] = __uint_as_float(hi[j + e]); }
+                put(j >> 3, a);
+                put(4 + (j >> 3), b);
+              }
+            } else if (split) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 8) {
+                float y0[8], y1[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  const float x0 = round_bf16(__uint_as_float(lo[j + e]));
+                  const float x1 = round_bf16(__uint_as_float(hi[j + e]));
+                  y0[e] = x0 * cs_r[j + e] - x1 * sn_r[j + e];
+                  y1[e] = x0 * sn_r[j + e] + x1 * cs_r[j + e];
+                }
+                put(j >> 3, y0);
+                put(4 + (j >> 3), y1);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; j += 8) {
+                float a[8], b[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                  const float x0 = round_bf16(__uint_as_float(lo[j + e]));
+                  const float x1 = round_bf16(__uint_as_float(lo[j + e + 1]));
+                  const float z0 = round_bf16(__uint_as_float(hi[j + e]));
+                  const float z1 = round_bf16(__uint_as_float(hi[j + e + 1]));
+                  const int p0 = (j + e) >> 1, p1 = 16 + p0;
+                  a[e] = x0 * cs_r[p0] - x1 * sn_r[p0];
+                  a[e + 1] = x0 * sn_r[p0] + x1 * cs_r[p0];
+                  b[e] = z0 * cs_r[p1] - z1 * sn_r[p1];
+                  b[e + 1] = z0 * sn_r[p1] + z1 * cs_r[p1];
+                }
+                put(j >> 3, a);
+                put(4 + (j >> 3), b);
+              }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int r = it * 4 + (lane >> 3), piece = lane & 7;
+              const long long to = __shfl_sync(0xffffffffu, at, r);
+              const uint4 v = *reinterpret_cast<const uint4*>(mine + r * 128 + ((piece ^ (r & 7)) << 4));
+              if (to >= 0)
+                *reinterpret_cast<uint4*>(base + to + (piece < 4 ? c_lo + 8 * piece : c_hi + 8 * (piece - 4))) = v;
+            }
+          }
+        }
+      } else if (tc_is_store(EPI)) {
         unsigned char* mine = staging + chalf * 2 * L::kSlab;
         const bool elected = ((warp - 2) & 3) == 0 && lane == 0;
 #pragma unroll 1
@@ -959,8 +1073,9 @@ static int launch_tc_pair(const void* A, const void* W, TcEpi ep, int M, int N, 
   CUtensorMap map_a, map_w, map_c;
   if (make_tile_map_bf16(&map_a, A, M, K, lda, kTcBM)) return kBadArgument;
   if (make_tile_map_bf16(&map_w, W, N, K, ldw, kTpBN / 2)) return kBadArgument;
-  if (tc_is_store(EPI) ? make_box_map(&map_c, ep.C, M, N, ep.ldc, kTcBM, 32, true, true)
-                      : make_box_map(&map_c, ep.act, M, ep.I, ep.I, kTcBM, 64, true, false))
+  if (EPI == kTcRope) map_c = map_a;           // (not used: the epilogue's threads store)
+  else if (tc_is_store(EPI) ? make_box_map(&map_c, ep.C, M, N, ep.ldc, kTcBM, 32, true, true)
+                           : make_box_map(&map_c, ep.act, M, ep.I, ep.I, kTcBM, 64, true, false))
     return kBadArgument;
   static int sm_count = 0;
   if (!sm_count) {
@@ -1345,6 +1460,16 @@ extern "C" int cretif_gemm_tc_qkv_rope(const void* A, const void* Wqkv, void* Q,
   ep.kc = (__nv_bfloat16*)kc; ep.vc = (__nv_bfloat16*)vc; ep.bt = bt; ep.write_cache = write_cache;
   const int N = (nh + 2 * nkv) * hd;
   cudaStream_t st = (cudaStream_t)stream;
+  const long long wide_pairs = (long long)((N + 255) / 256) * ((M + 255) / 256);
+  // Two CTAs a tile: 128-wide tiles pull 32 KB through L2 for 2 MFLOP, which holds q|k|v to 560 to 720
+  // TFLOP/s however its epilogue goes; a pair's 256 x 256 pull half as much.  Prompts, us a pass, before
+  // and after: SmolLM2-1.7B (6,144 x 2,048) 8 x 1,024 26,970 -> 25,410, one of 1,024 4,980 -> 4,760;
+  // 360M (1,600 x 960) 16 of 256 to 2,048 13,560 -> 12,870, but two of 1,500 4,600 -> 4,640; 135M
+  // (960 x 576) 8 x 2,048 7,600 -> 7,670.  So: from one wave of pairs on where pairs pay anyhow, from four on
+  // for the smaller matrices from 1.5 M elements up.
+  if (g_tc_pair != 0 && (g_tc_pair > 0 || (pair_pays(N, K) ? wide_pairs >= 74
+                                                           : (long long)N * K >= 1500000 && wide_pairs >= 4 * 74)))
+    return launch_tc_pair<256, kTcRope>(A, Wqkv, ep, M, N, K, lda, ldw, fault, st);
   // A tile is a whole number of heads.  Small products want many narrow tiles; large ones
   // (two waves of 128-wide tiles and more) do more arithmetic per byte with wide ones.
   const long long m_tiles = (M + kTcBM - 1) / kTcBM;

@@ -54,3 +54,44 @@ def test_float32_store_through_tma(ops, M, N, K, bn):  # noqa: F811
             got.append(full)
     assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[3])
     assert not any(took[:2]) and (all(took[2:]) or bn in (64, 128, 192))
+
+
+@pytest.mark.parametrize("pairing", [0, 1])
+@pytest.mark.parametrize("nh,nkv,hd,K", [(9, 3, 64, 72), (2, 1, 128, 96), (15, 5, 64, 136), (6, 1, 128, 64)])
+def test_qkv_rope_with_two_ctas_on_a_tile(ops, pairing, nh, nkv, hd, K):  # noqa: F811
+    """Against the separate kernels: rows of several sequences in a tile, a chunk at a cached position,
+    the last tile's heads beyond the matrix, one step that may not write the cache."""
+    P, lens, news = 512, [200, 70, 333], [200, 70, 150]
+    j = torch.arange(hd // 2, dtype=torch.float64)
+    ang = torch.arange(P, dtype=torch.float64)[:, None] / 10000.0 ** (2 * j / hd)[None, :]
+    cos, sin = torch.cos(ang).float().to(DEV), torch.sin(ang).float().to(DEV)
+    qpos, qseq = [], []
+    for b, (n, m) in enumerate(zip(lens, news)):
+        qpos += list(range(n - m, n))
+        qseq += [b] * m
+    T = len(qpos)
+    pos_t = torch.tensor(qpos, dtype=torch.int32, device=DEV)
+    seq_t = torch.tensor(qseq, dtype=torch.int32, device=DEV)
+    x = rnd(T, K, dtype=torch.bfloat16)
+    w = rnd((nh + 2 * nkv) * hd, K, dtype=torch.bfloat16, seed=2, scale=0.3)
+    fault = ops.fault_word(DEV)
+    fault.zero_()
+    got = []
+    for pair in (0, 1):
+        cache = ToyCache(lens, nkv, hd, torch.bfloat16, seed=3)
+        q = torch.zeros(T, nh * hd, device=DEV, dtype=torch.bfloat16)
+        old = ops.set_tc_pair(pair)
+        before = ops.variant_counts()["tc_pair"]
+        ops.gemm_tc_qkv_rope(x, w, q, cos, sin, pairing, nh, nkv, hd, pos_t, seq_t, cache.seq_slot,
+                             cache.table, cache.k, cache.v, 64, True)
+        assert (ops.variant_counts()["tc_pair"] > before) == bool(pair)
+        kept = cache.k.clone(), cache.v.clone()
+        ops.gemm_tc_qkv_rope(x + 1, w, q.clone(), cos, sin, pairing, nh, nkv, hd, pos_t, seq_t,
+                             cache.seq_slot, cache.table, cache.k, cache.v, 64, False)
+        ops.set_tc_pair(old)
+        assert torch.equal(kept[0], cache.k) and torch.equal(kept[1], cache.v)
+        got.append((q, *kept))
+    assert fault.item() == 0
+    # the same products in the same order of sums, rounded at the same places
+    for a, b in zip(*got):
+        close(b, a, 1e-2)
