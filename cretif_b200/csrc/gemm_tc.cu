@@ -386,6 +386,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int j = 0; j < 8; ++j) cur[j] = oldv[j];
             if (c0 + 32 < c_first + kCols) fetch_old(c0 + 32);
           }
+          if (EPI == kTcStoreEx && ep.scaled) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(ep.alpha * __uint_as_float(r[j]));
+          }
+          if (EPI == kTcStoreEx && ep.unary) unary_activations(r, ep.unary - 1);
           if (m < M && n0 + c0 < N) {
             TC* out = C + (size_t)m * ldc + n0 + c0;
 #pragma unroll
@@ -393,14 +398,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               float v[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[j + e]);
-              if (EPI == kTcStoreEx && ep.scaled) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] *= ep.alpha;
-              }
-              if (EPI == kTcStoreEx && ep.unary) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = unary_activation(v[e], ep.unary - 1);
-              }
               const int n = n0 + c0 + j;
               if (EPI == kTcStoreEx && ep.mul && n < N) {          // (N is a multiple of 8 then)
                 const int id = ep.mul_ids[m];
