@@ -277,27 +277,52 @@ moe_group_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ of
   int* counts = sh;
   int* cursor = sh + E;
   int* start = sh + 2 * E;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = cursor[e] = 0;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
   __syncthreads();
   for (int p = threadIdx.x; p < P; p += blockDim.x)
     if (ids[p] < E) atomicAdd(&counts[ids[p]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0, n_tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      start[e] = at;
-      if (offsets) offsets[e] = at;
-      for (int r = 0; r < counts[e] && n_tiles < max_tiles; r += tile, ++n_tiles) {
-        tile_expert[n_tiles] = e;
-        if (tile_row0) tile_row0[n_tiles] = at + r;
+  // The first warp sums rows and tiles over the experts, 32 at a time, then every thread writes its
+  // experts' tiles (one thread doing both took most of the launch).
+  int* tile0 = cursor;                           // an expert's first tile, until the places are dealt
+  __shared__ int all_tiles;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int rows = 0, tiles = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, n = e < E ? counts[e] : 0, t = (n + tile - 1) / tile;
+      int r_sum = padded ? t * tile : n, t_sum = t;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int ro = __shfl_up_sync(0xffffffffu, r_sum, off);
+        const int to = __shfl_up_sync(0xffffffffu, t_sum, off);
+        if (lane >= off) { r_sum += ro; t_sum += to; }
       }
-      at += padded ? (counts[e] + tile - 1) / tile * tile : counts[e];
+      if (e < E) {
+        start[e + 1] = rows + r_sum;
+        tile0[e] = tiles + t_sum - t;
+      }
+      rows += __shfl_sync(0xffffffffu, r_sum, 31);
+      tiles += __shfl_sync(0xffffffffu, t_sum, 31);
     }
-    start[E] = at;
-    if (offsets) offsets[E] = at;
-    if (used) used[0] = n_tiles;
-    for (; n_tiles < max_tiles; ++n_tiles) tile_expert[n_tiles] = -1;
+    if (lane == 0) {
+      start[0] = 0;
+      all_tiles = tiles;
+    }
   }
+  __syncthreads();
+  const int n_tiles = min(all_tiles, max_tiles);
+  for (int e = threadIdx.x; e < E; e += blockDim.x)
+    for (int i = tile0[e], r = 0; r < counts[e] && i < max_tiles; ++i, r += tile) {
+      tile_expert[i] = e;
+      if (tile_row0) tile_row0[i] = start[e] + r;
+    }
+  for (int i = n_tiles + threadIdx.x; i < max_tiles; i += blockDim.x) tile_expert[i] = -1;
+  if (offsets)
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = start[e];
+  if (used && threadIdx.x == 0) used[0] = n_tiles;
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) cursor[e] = 0;
   __syncthreads();
   for (int p = threadIdx.x; p < P; p += blockDim.x) {
     const int e = ids[p];
