@@ -362,13 +362,14 @@ int cretif_attn_decode_mma_bias(const void* q, int ldq, void* out, int ldo, cons
                                 const float* bias_near, const float* bias_far, int n_far,
                                 int head_groups, const float* bias_slope, unsigned int* fault,
                                 void* stream);
-// ... and with pooled entries (see cretif_attn_simt_pooled; pool_blocks blocks of them).
+// ... and with pooled entries (see cretif_attn_simt_pooled; pool_blocks blocks of them).  seq_items:
+// head_groups where tok_pos and tok_seq have an entry a sequence, 1 where they have one an item.
 int cretif_attn_decode_mma_pooled(
     const void* q, int ldq, void* out, int ldo, const void* kc, const void* vc, long long n_blocks,
     const int* table, int table_stride, const int* tok_pos, const int* tok_seq, const int* seq_slot,
     int nh, int nkv, int hd, float scale, int window, int bt, int B, int n_splits, float* part_o,
     float* part_ml, int* counters, const float* sink, const float* bias_near, const float* bias_far,
-    int n_far, int head_groups, const float* bias_slope, const void* pool_k, const void* pool_v,
+    int n_far, int head_groups, int seq_items, const float* bias_slope, const void* pool_k, const void* pool_v,
     long long pool_blocks, const int* pool_table, int pool_stride, int pool, unsigned int* fault,
     void* stream);
 

@@ -124,7 +124,7 @@ extern "C" int cretif_attn_decode_mma_bias(const void* q, int ldq, void* out, in
   return cretif_attn_decode_mma_pooled(
       q, ldq, out, ldo, kc, vc, n_blocks, table, table_stride, tok_pos, tok_seq, seq_slot, nh, nkv,
       hd, scale, window, bt, B, n_splits, part_o, part_ml, counters, sink, bias_near, bias_far,
-      n_far, head_groups, bias_slope, nullptr, nullptr, 0, nullptr, 0, 0, fault, stream);
+      n_far, head_groups, 1, bias_slope, nullptr, nullptr, 0, nullptr, 0, 0, fault, stream);
 }
 
 // pool_k, pool_v (blocks like kc and vc, pool_blocks of them), pool_table [slots, pool_stride]: the
@@ -134,16 +134,17 @@ extern "C" int cretif_attn_decode_mma_pooled(
     const int* table, int table_stride, const int* tok_pos, const int* tok_seq, const int* seq_slot,
     int nh, int nkv, int hd, float scale, int window, int bt, int B, int n_splits, float* part_o,
     float* part_ml, int* counters, const float* sink, const float* bias_near, const float* bias_far,
-    int n_far, int head_groups, const float* bias_slope, const void* pool_k, const void* pool_v,
+    int n_far, int head_groups, int seq_items, const float* bias_slope, const void* pool_k, const void* pool_v,
     long long pool_blocks, const int* pool_table, int pool_stride, int pool, unsigned int* fault,
     void* stream) {
   if (B <= 0) return kOk;
   if (pool_table && (!pool_k || !pool_v || pool <= 0 || window <= 0 || pool_blocks <= 0))
     return kBadArgument;
   if ((bias_near != nullptr) != (bias_far != nullptr) || (bias_near && n_far < 1) ||
-      head_groups < 1 || B % head_groups || (bias_near && bias_slope))
+      head_groups < 1 || B % head_groups || (seq_items != 1 && seq_items != head_groups) ||
+      (bias_near && bias_slope))
     return kBadArgument;
-  const DistanceBias bias{bias_near, bias_far, n_far, head_groups, bias_slope};
+  const DistanceBias bias{bias_near, bias_far, n_far, head_groups, seq_items, bias_slope};
   if (nh <= 0 || nkv <= 0 || nh % nkv || nh / nkv > 8 || hd % 16 || hd < 16 || hd > 128 ||
       bt != kDmTile || n_splits <= 0 || n_splits > kDmTile || nkv > 65535 || B > 65535 ||
       ldq % 2)

@@ -99,12 +99,15 @@ __host__ __device__ constexpr size_t dm_mrg_floats() {
 // the scaled score of the key n positions back, near[h, n] for n < n_far, far[h] beyond.
 // head_groups = G > 1: the launch's items are (sequence, group of heads) pairs, item b serving
 // heads (b % G) * nh .. of a model with G * nh query heads on these key/value heads; the rows of
-// q, out, tok_pos and tok_seq are laid out by item, the sink's and the bias's rows by head.
+// q and out are laid out by item, the sink's and the bias's rows by head; entry b / seq_items of tok_pos
+// and tok_seq is item b's (seq_items: G where they have an entry a sequence, 1 where one an item).  Both
+// are read in front of the wait for the kernel before: they have to be the step's own arrays, as a copy
+// per item that a kernel of the same step makes is promised to be visible only behind that wait.
 struct DistanceBias {
   const float* near_;
   const float* far_;
   int n_far;
-  int head_groups;
+  int head_groups, seq_items;
   const float* slope_;      // [heads], times log2 e: n times it is taken off instead of a table
 };
 
@@ -127,7 +130,7 @@ __device__ __forceinline__ void attn_decode_mma_item(
     int ldo, int* __restrict__ counters, unsigned int* __restrict__ fault, int split,
     int n_splits, int kvh, int b, uint32_t& it_base, unsigned long long* stamps = nullptr,
     int n_stages = kDmStages, const float* sink = nullptr,
-    DistanceBias bias = DistanceBias{nullptr, nullptr, 0, 1, nullptr},
+    DistanceBias bias = DistanceBias{nullptr, nullptr, 0, 1, 1, nullptr},
     const PooledTiles<POOLED>* pool = nullptr) {
   if (bias.head_groups > 1) {           // this item's heads start at head0 of the model's
     const int head0 = (b % bias.head_groups) * nh;
@@ -180,8 +183,9 @@ __device__ __forceinline__ void attn_decode_mma_item(
   };
   const int nthreads = blockDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pos = tok_pos[b];
-  const int slot = seq_slot[tok_seq[b]];
+  const int item_seq = bias.seq_items > 1 ? b / bias.seq_items : b;
+  const int pos = tok_pos[item_seq];
+  const int slot = seq_slot[tok_seq[item_seq]];
   const int* tab = table + (size_t)slot * table_stride;
   const int first_key = first_visible_key(pos, window);
   const int first_tile = first_key / kDmTile;

@@ -1671,9 +1671,11 @@ def attn_decode(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv:
     ``bias_slope`` (float32 [heads], times log2 e; tensor-core kernel only, not with the
     table): the key n positions back has n times it taken off its scaled score.
     ``head_groups`` = G > 1 (tensor-core kernel only): more than eight query heads on a
-    key/value head in ONE launch; the rows of ``q``, ``out``, ``tok_pos`` and ``tok_seq`` are
-    (sequence, group of ``nh`` heads) items, G of them a sequence, while ``sink`` and the bias
-    keep a row per head of all G·nh.  ``sink`` (float32 [heads], optional; tensor-core kernel only): exp(sink_h) joins head h's
+    key/value head in ONE launch; the rows of ``q`` and ``out`` are (sequence, group of ``nh``
+    heads) items, G of them a sequence; ``tok_pos`` and ``tok_seq`` have an entry a sequence (or
+    an item), ``sink`` and the bias a row per head of all G·nh.  ``tok_pos``, ``tok_seq``, ``seq_slot``
+    and the tables are read ahead of the kernels launched before: nothing of the same step may
+    write them.  ``sink`` (float32 [heads], optional; tensor-core kernel only): exp(sink_h) joins head h's
     softmax denominator.  ``bias_near`` [heads, n_far] with ``bias_far`` [heads] (float32, times
     log2 e; tensor-core kernel only): what the key n positions back adds to its scaled score."""
     n_far = 0
@@ -1698,6 +1700,7 @@ def attn_decode(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv:
     if head_groups > 1 and (hd > 128 or _decode_simt_only or q.shape[0] % head_groups):
         raise KernelError("attn_decode: groups of heads need head_dim <= 128 and whole "
                           "sequences of items")
+    seq_items = head_groups if tok_pos.shape[0] * head_groups == q.shape[0] else 1
     _need(q, "q", torch.bfloat16, 2); _need(out, "out", torch.bfloat16, 2)
     _need(kc, "k cache", torch.bfloat16, 4); _need(vc, "v cache", torch.bfloat16, 4)
     B = q.shape[0]
@@ -1718,7 +1721,7 @@ def attn_decode(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv:
             ctypes.c_longlong(kc.shape[0]), _p(table), table.stride(0), _p(tok_pos), _p(tok_seq),
             _p(seq_slot), nh, nkv, hd, ctypes.c_float(scale), window, block_tokens, B, n_splits,
             None, None, None, _p(sink), _p(bias_near), _p(bias_far), n_far, head_groups,
-            _p(bias_slope), *_pool_args(pool, True), _p(fault), _stream()),
+            seq_items, _p(bias_slope), *_pool_args(pool, True), _p(fault), _stream()),
             "attn_decode_mma")
         return
     part_o = torch.empty((B, nh, n_splits, hd), dtype=torch.float32, device=q.device)
@@ -1730,7 +1733,7 @@ def attn_decode(q, out, kc, vc, table, tok_pos, tok_seq, seq_slot, nh: int, nkv:
             ctypes.c_longlong(kc.shape[0]), _p(table), table.stride(0), _p(tok_pos), _p(tok_seq),
             _p(seq_slot), nh, nkv, hd, ctypes.c_float(scale), window, block_tokens, B, n_splits,
             _p(part_o), _p(part_ml), _p(counters), _p(sink), _p(bias_near), _p(bias_far), n_far,
-            head_groups, _p(bias_slope), *_pool_args(pool, True), _p(fault), _stream()),
+            head_groups, seq_items, _p(bias_slope), *_pool_args(pool, True), _p(fault), _stream()),
             "attn_decode_mma")
         return
     _check(lib().cretif_attn_decode(

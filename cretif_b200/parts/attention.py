@@ -140,15 +140,9 @@ def run_attention(q, o, ctx, kv, nh, nkv, hd, scale, window, dtype, sink=None, v
             G = nh // 8
             if (nh // nkv > 8 and nh % 8 == 0 and hd <= 128 and q.stride(0) == nh * hd
                     and o.stride(0) == nh * hd and ops.attn_decode_supported(hd, kv.block_tokens, 8)):
-                key = ("decode_head_groups", G)
-                if key not in ctx.extras:       # once a step, for every layer that asks
-                    # (materialised: a stride-0 view of one sequence's entry is no array)
-                    ctx.extras[key] = tuple(t.repeat_interleave(G).contiguous()
-                                            for t in (ctx.tok_pos, ctx.tok_seq))
-                pos_g, seq_g = ctx.extras[key]
                 splits, cluster = ops.decode_plan(ctx.B * G, 1, context, q.device, hd)
                 ops.attn_decode(q.view(ctx.B * G, 8 * hd), o.view(ctx.B * G, 8 * hd), kv.k, kv.v,
-                                kv.table, pos_g, seq_g, ctx.seq_slot, 8, 1, hd, scale, window,
+                                kv.table, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, 8, 1, hd, scale, window,
                                 kv.block_tokens, splits, ctx.fault, cluster, sink=sink,
                                 bias_near=near, bias_far=far, head_groups=G, bias_slope=tilt,
                                 pool=pool)
