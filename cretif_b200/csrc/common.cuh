@@ -193,6 +193,7 @@ enum Variant : int {
   kVarF32Tile32,            // ... 32 x 32 tiles, the slabs dealt to four warps
   kVarDeltaSlices32,        // chunks of a delta rule, 32 columns a CTA
   kVarDeltaSlices16,        // ... 16
+  kVarFusedHeld,            // fused projection, a CTA's whole tile of weights held in registers
   kVarCount
 };
 void count_variant(int v);

@@ -83,13 +83,16 @@ static int launch_fused(const FusedParams& p, int tiles, cudaStream_t st, int gr
   return launch_status();
 }
 
-// The register variant for any number of rows up to kFuMaxRows; held: as registers_hold says.
+// The register variant for any number of rows up to kFuMaxRows; held (see registers_hold): a body of
+// more than three chunks, whatever the width, as only those start the kernel behind late.
 template <int PRO, int EPI>
 static int dispatch_registers(const FusedParams& p, int tiles, cudaStream_t st, bool held = false) {
-  if (held && p.K > 1536) return launch_fused<1, PRO, EPI, 8>(p, tiles, st);
-  if (held && p.K > 768)
+  if (held) {
+    count_variant(kVarFusedHeld);
+    if (p.K > 1536) return launch_fused<1, PRO, EPI, 8>(p, tiles, st);
     return p.M <= 8 ? launch_fused<1, PRO, EPI, 6>(p, tiles, st)
                     : launch_fused<2, PRO, EPI, 6>(p, tiles, st);
+  }
   if (p.M <= 8) return launch_fused<1, PRO, EPI>(p, tiles, st);
   if (p.M <= 16) return launch_fused<2, PRO, EPI>(p, tiles, st);
   if (p.M <= kFuMaxGroupRows) return launch_fused<4, PRO, EPI>(p, tiles, st);

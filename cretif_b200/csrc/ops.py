@@ -52,7 +52,7 @@ _VARIANTS = ("fused_registers", "fused_row_groups", "fused_cluster2", "fused_clu
              "stream_row_groups", "decode_cluster", "decode_split", "prefill_attn", "tc64",
              "tc128", "tc256", "tc_several_tiles", "tc192", "prefill_attn_pair",
              "prefill_attn_split", "tc_bulk_add", "tc_pair", "delta_prepare_rows", "f32_few",
-             "f32_tile64", "f32_tile32", "delta_slices32", "delta_slices16")
+             "f32_tile64", "f32_tile32", "delta_slices32", "delta_slices16", "fused_held")
 
 
 def variant_counts() -> dict:

@@ -32,6 +32,21 @@ def test_held_in_registers(ops, M, N, K):  # noqa: F811
     close(out, _norm_bf16(h, nw, 1e-5) @ w.double().cpu().T, 3e-3)
 
 
+@pytest.mark.parametrize("M", [1, 8, 16])
+def test_the_narrowest_held_product(ops, M):  # noqa: F811
+    """K = 768, where held products begin, takes a held body (which starts the kernel behind late) and not
+    the three-chunk one, which covers as many columns but starts it early."""
+    took = {}
+    for K in (760, 768, 776):
+        w, x = rnd(48, K, dtype=torch.bfloat16, seed=2), rnd(M, K, dtype=torch.bfloat16, seed=4)
+        base = rnd(M, 48, seed=5)
+        acc, before = base.clone(), ops.variant_counts()["fused_held"]
+        ops.fused_linear_add(x, w, acc)
+        took[K] = ops.variant_counts()["fused_held"] - before
+        close(acc, base.double().cpu() + x.double().cpu() @ w.double().cpu().T, 1e-5)
+    assert took == {760: 0, 768: 1, 776: 1}
+
+
 @pytest.mark.parametrize("M,N,K,bn", [(300, 200, 72, 0), (129, 68, 136, 64), (70, 1000, 1544, 128),
                                       (1000, 960, 576, 192), (2100, 2048, 264, 256), (20000, 520, 72, 256)])
 def test_float32_store_through_tma(ops, M, N, K, bn):  # noqa: F811
