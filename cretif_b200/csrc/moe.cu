@@ -273,7 +273,7 @@ moe_group_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ of
                  int* __restrict__ place, int* __restrict__ order, int* __restrict__ tile_expert,
                  int* __restrict__ tile_row0, int max_tiles, int tile, int padded,
                  int* __restrict__ used) {
-  extern __shared__ int sh[];                    // counts [E], cursor [E], start [E + 1]
+  extern __shared__ int sh[];                    // counts [E], cursor [E], start [E + 1], tiles in use
   int* counts = sh;
   int* cursor = sh + E;
   int* start = sh + 2 * E;
@@ -285,7 +285,7 @@ moe_group_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ of
   // The first warp sums rows and tiles over the experts, 32 at a time, then every thread writes its
   // experts' tiles (one thread doing both took most of the launch).
   int* tile0 = cursor;                           // an expert's first tile, until the places are dealt
-  __shared__ int all_tiles;
+  int* all_tiles = sh + 3 * E + 1;               // (a static array would cost the last expert of 48 KB)
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     int rows = 0, tiles = 0;
@@ -307,11 +307,11 @@ moe_group_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ of
     }
     if (lane == 0) {
       start[0] = 0;
-      all_tiles = tiles;
+      *all_tiles = tiles;
     }
   }
   __syncthreads();
-  const int n_tiles = min(all_tiles, max_tiles);
+  const int n_tiles = min(*all_tiles, max_tiles);
   for (int e = threadIdx.x; e < E; e += blockDim.x)
     for (int i = tile0[e], r = 0; r < counts[e] && i < max_tiles; ++i, r += tile) {
       tile_expert[i] = e;
@@ -777,7 +777,7 @@ extern "C" int cretif_moe_group(const int* ids, int P, int E, int* offsets, int*
                                 int* tile_expert, int* tile_row0, int max_tiles, void* stream) {
   if (P <= 0) return kOk;
   if (E <= 0 || E > 4096 || max_tiles < (P + kTile - 1) / kTile + E) return kBadArgument;
-  moe_group_kernel<<<1, 1024, sizeof(int) * (3 * E + 1), (cudaStream_t)stream>>>(
+  moe_group_kernel<<<1, 1024, sizeof(int) * (3 * E + 2), (cudaStream_t)stream>>>(
       ids, P, E, offsets, place, order, tile_expert, tile_row0, max_tiles, kTile, 0, nullptr);
   return launch_status();
 }
@@ -789,7 +789,7 @@ extern "C" int cretif_moe_group_padded(const int* ids, int P, int E, int tile, i
   if (P <= 0) return kOk;
   if (E <= 0 || E > 4096 || tile <= 0 || max_tiles < (P + tile - 1) / tile + E || !used)
     return kBadArgument;
-  moe_group_kernel<<<1, 1024, sizeof(int) * (3 * E + 1), (cudaStream_t)stream>>>(
+  moe_group_kernel<<<1, 1024, sizeof(int) * (3 * E + 2), (cudaStream_t)stream>>>(
       ids, P, E, nullptr, place, nullptr, tile_expert, nullptr, max_tiles, tile, 1, used);
   return launch_status();
 }

@@ -46,3 +46,16 @@ def test_the_sorted_order(ops, P, E, n, tile, padded):  # noqa: F811
                                                    for i in range(int(n_tiles[e]))]
         kept = order.cpu().long()[:int(counts.sum())]
         assert at[kept].tolist() == list(range(int(counts.sum())))
+
+
+def test_the_most_experts(ops):  # noqa: F811
+    """4,095 experts: the order's counts, places and starts fill the 48 KB a launch has without asking."""
+    E, P = 4095, 700
+    ids = torch.randint(0, E, (P, 1), generator=torch.Generator().manual_seed(1)).int().to(DEV)
+    place, used = torch.full((P,), -7, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    tile_expert = torch.full((ops.moe_tc_tiles(P, E),), -7, dtype=torch.int32, device=DEV)
+    ops.moe_group_padded(ids, E, place, tile_expert, used)
+    want = sorted(set(ids.flatten().tolist()))           # (700 pairs: a tile of 128 rows each)
+    assert used.item() == len(want) and tile_expert.tolist()[:len(want)] == want
+    assert bool((tile_expert[len(want):] == -1).all())
+    assert all(want[p // 128] == e for p, e in zip(place.tolist(), ids.flatten().tolist()))
