@@ -1554,10 +1554,14 @@ _FAULT = {}
 
 
 def fault_word(device) -> torch.Tensor:
-    """The int32 status word of a device that kernels OR their fault bits into."""
-    key = str(torch.device(device))
+    """The int32 status word of a device that kernels OR their fault bits into: one a device, however it
+    is named ("cuda" is the current one)."""
+    dev = torch.device(device)
+    if dev.type == "cuda" and dev.index is None:
+        dev = torch.device("cuda", torch.cuda.current_device())
+    key = str(dev)
     if key not in _FAULT:
-        _FAULT[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        _FAULT[key] = torch.zeros(1, dtype=torch.int32, device=dev)
     return _FAULT[key]
 
 

@@ -67,3 +67,14 @@ def test_a_token_outside_the_vocabulary_in_a_decode_step(model_dirs, plain_model
     got = eng.generate(prompts, max_tokens=4, stop_ids=[], use_graph=use_graph)
     for p, r in zip(prompts, got):
         assert r.tokens == pl.greedy(cfg, w, p, 4)
+
+
+def test_the_products_word_is_the_engines(model_dirs):
+    """A product writes the word of its tensors' device; an engine made for "cuda" reads that one."""
+    from cretif_b200.csrc import ops
+    from cretif_b200.engine import Engine, StepError
+    eng = Engine(model_dirs["A"], dtype="bfloat16", max_tokens=512)
+    ops.wait_that_expires(100, ops.fault_word(torch.zeros(1, device="cuda").device))
+    with pytest.raises(StepError, match="bounded wait"):
+        eng.check_fault()
+    eng.check_fault()
