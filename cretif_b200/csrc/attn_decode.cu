@@ -238,6 +238,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq,
         }
       }
     }
+    // (the stage is refilled by the async proxy: every thread's reads of it end before that)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();                    // the stage's tiles and ps are free again
     if (tid == 0 && tile + 2 < t_end) issue(tile + 2, stage);
   }

@@ -364,8 +364,7 @@ __device__ __forceinline__ void attn_decode_mma_item(
           o[2 * np + 1][0] = c1[0]; o[2 * np + 1][1] = c1[1];
         }
       }
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&empty[s]);
+      tc::release_stage(&empty[s], lane);
       if (++s == n_stages) { s = 0; ++turn; }
     }
     (void)ok;

@@ -281,8 +281,7 @@ skinny_stream_kernel(const FusedParams whole, const __grid_constant__ CUtensorMa
             mma_16816(acc[t], a2, ux.z, ux.w);
           }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&empty[s]);
+        tc::release_stage(&empty[s], lane);
         if (++s == n_stages) { s = 0; ++turn; }
       }
 #pragma unroll

@@ -37,6 +37,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Gives a stage of a TMA ring back that the warp has read with ordinary loads of shared memory: the
+// copies that follow are made by the async proxy, which an arrival orders nothing against that the loads
+// have not finished by themselves.  Without the fence a warp whose loads were queued behind another CTA's
+// read the next turn's contents (a ring of eight stages beside a CTA that asks for 64 KB of weights).
+__device__ __forceinline__ void release_stage(uint64_t* empty, int lane) {
+  fence_proxy_async();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(empty);
+}
 
 // Wait for the phase with the given parity; false when it gave up after `limit` polls (and
 // raised *abort).

@@ -110,3 +110,27 @@ def test_qkv_rope_with_two_ctas_on_a_tile(ops, pairing, nh, nkv, hd, K):  # noqa
     # the same products in the same order of sums, rounded at the same places
     for a, b in zip(*got):
         close(b, a, 1e-2)
+
+
+def test_the_ring_beside_another_streams_loads(ops):  # noqa: F811
+    """A ring that turns more than once (16 steps in eight stages), while products on another stream ask
+    for whole tiles of weights on the same SMs: a stage may be refilled only when its reads are done."""
+    w, x = rnd(2048, 8192, dtype=torch.bfloat16, seed=1), rnd(1, 8192, dtype=torch.bfloat16, seed=2)
+    v, y = rnd(2176, 2048, dtype=torch.bfloat16, seed=3), rnd(1, 2048, dtype=torch.bfloat16, seed=4)
+    want = torch.zeros(1, 2048, device=DEV)
+    before = ops.variant_counts()
+    ops.fused_linear_add(x, w, want)
+    ops.fused_linear_add(y, v, torch.zeros(1, 2176, device=DEV))
+    after = ops.variant_counts()
+    assert after["stream"] > before["stream"] and after["fused_held"] > before["fused_held"]
+    close(want, x.double().cpu() @ w.double().cpu().T, 1e-5)
+    got, beside = torch.zeros(300, 2048, device=DEV), torch.zeros(1, 2176, device=DEV)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for i in range(len(got)):
+        with torch.cuda.stream(other):
+            for _ in range(2):
+                ops.fused_linear_add(y, v, beside)
+        ops.fused_linear_add(x, w, got[i:i + 1])
+    torch.cuda.synchronize()
+    assert bool((got == want).all())
