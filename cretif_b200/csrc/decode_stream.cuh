@@ -46,6 +46,8 @@ __host__ __device__ inline size_t stream_smem(int nt, int pro, int M, int K, int
 int make_box_map_bf16(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows,
                       int box_cols, bool swizzle);
 
+__device__ __forceinline__ uint32_t bits_of(const uint4& v) { return v.x ^ v.y ^ v.z ^ v.w; }
+
 // The two groups of eight consecutive weight rows that tile `tile` is made of.
 template <int EPI>
 __device__ __forceinline__ void tile_groups(const FusedParams& p, int tile, int& row_a, int& row_b,
@@ -237,6 +239,7 @@ skinny_stream_kernel(const FusedParams whole, const __grid_constant__ CUtensorMa
       asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     int s = 0, turn = 0;                         // the ring's stage and how often it has turned
+    int refills = total - n_stages;              // uses of a stage that a refill waits for: the first ones
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
       if (!have_ahead) epi_prefetch<NT, EPI>(p, tile, ahead);
       have_ahead = false;
@@ -252,36 +255,54 @@ skinny_stream_kernel(const FusedParams whole, const __grid_constant__ CUtensorMa
       for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
-      for (int step = 0; step < n_steps; ++step) {
+      for (int step = 0; step < n_steps; ++step, --refills) {
         const int k0 = step * kStK;
         tc::mbar_wait(&full[s], (uint32_t)(turn & 1), abort);   // bounded; see abort
         const unsigned char* ws = wst + (size_t)s * kStW;
+        constexpr int kChunks = kStK / (32 * kFuWarps);      // chunks of 32 columns, two per warp
+        uint4 ua[kChunks], ub[kChunks], ux[kChunks][NT];
 #pragma unroll
-        for (int j = 0; j < kStK / (32 * kFuWarps); ++j) {   // chunks of 32 columns, two per warp
+        for (int j = 0; j < kChunks; ++j) {
           const int kl = (warp + j * kFuWarps) * 32 + c * 8, k = k0 + kl;
           const int box = kl / kStBoxK, cb = (kl % kStBoxK) * 2;
           const bool in = k < p.K;
-          const uint4 ua = in ? *reinterpret_cast<const uint4*>(ws + off_a + box * kStGroup + cb) : zero;
-          const uint4 ub = in ? *reinterpret_cast<const uint4*>(ws + off_b + box * kStGroup + cb) : zero;
-          const uint32_t a1[4] = {ua.x, ub.x, ua.y, ub.y};
-          const uint32_t a2[4] = {ua.z, ub.z, ua.w, ub.w};
+          ua[j] = in ? *reinterpret_cast<const uint4*>(ws + off_a + box * kStGroup + cb) : zero;
+          ub[j] = in ? *reinterpret_cast<const uint4*>(ws + off_b + box * kStGroup + cb) : zero;
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
             const int m = t * 8 + r;
-            uint4 ux = zero;
+            ux[j][t] = zero;
             if (in) {
               if (pro_is_norm(PRO)) {
-                if (m < p.M) ux = *reinterpret_cast<const uint4*>(xs + (size_t)m * xs_stride + (size_t)k * 2);
+                if (m < p.M)
+                  ux[j][t] = *reinterpret_cast<const uint4*>(xs + (size_t)m * xs_stride + (size_t)k * 2);
               } else {                 // rows beyond M arrived as zeros
-                ux = *reinterpret_cast<const uint4*>(xs + (size_t)s * kXStage +
-                                                     (size_t)box * NT * kStGroup + m * kStRowB + cb);
+                ux[j][t] = *reinterpret_cast<const uint4*>(xs + (size_t)s * kXStage +
+                                                           (size_t)box * NT * kStGroup + m * kStRowB + cb);
               }
             }
-            mma_16816(acc[t], a1, ux.x, ux.y);
-            mma_16816(acc[t], a2, ux.z, ux.w);
           }
         }
-        tc::release_stage(&empty[s], lane);
+#pragma unroll
+        for (int j = 0; j < kChunks; ++j) {
+          const uint32_t a1[4] = {ua[j].x, ub[j].x, ua[j].y, ub[j].y};
+          const uint32_t a2[4] = {ua[j].z, ub[j].z, ua[j].w, ub[j].w};
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            mma_16816(acc[t], a1, ux[j][t].x, ux[j][t].y);
+            mma_16816(acc[t], a2, ux[j][t].z, ux[j][t].w);
+          }
+        }
+        if (refills > 0) {             // the producer waits for this use of the stage
+          uint32_t taken = 0;
+#pragma unroll
+          for (int j = 0; j < kChunks; ++j) {
+            taken ^= bits_of(ua[j]) ^ bits_of(ub[j]);
+#pragma unroll
+            for (int t = 0; PRO == kProPlain && t < NT; ++t) taken ^= bits_of(ux[j][t]);
+          }
+          tc::release_stage_read(&empty[s], lane, taken);
+        }
         if (++s == n_stages) { s = 0; ++turn; }
       }
 #pragma unroll

@@ -47,11 +47,14 @@ def test_the_narrowest_held_product(ops, M):  # noqa: F811
     assert took == {760: 0, 768: 1, 776: 1}
 
 
-@pytest.mark.parametrize("M,N,K,bn", [(300, 200, 72, 0), (129, 68, 136, 64), (70, 1000, 1544, 128),
-                                      (1000, 960, 576, 192), (2100, 2048, 264, 256), (20000, 520, 72, 256)])
-def test_float32_store_through_tma(ops, M, N, K, bn):  # noqa: F811
+@pytest.mark.parametrize("M,N,K,bn,taken", [(300, 200, 72, 0, True), (129, 68, 136, 64, True),
+                                            (70, 1000, 1544, 128, True), (1000, 960, 576, 192, True),
+                                            (2100, 2048, 264, 256, True), (20000, 520, 72, 256, True),
+                                            # the slabs would take the second CTA its place on the SM
+                                            (4000, 1000, 1544, 128, False)])
+def test_float32_store_through_tma(ops, M, N, K, bn, taken):  # noqa: F811
     """Stored by the threads and through TMA: the same numbers, tails clipped, the padding beside the
-    matrix untouched; with a factor as well."""
+    matrix untouched; with a factor as well.  A launch of at most one tile an SM always goes through TMA."""
     x, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1)
     want = x.double() @ w.double().T
     ldc = -(-N // 8) * 8 + 8
@@ -59,22 +62,25 @@ def test_float32_store_through_tma(ops, M, N, K, bn):  # noqa: F811
     for bulk in (False, True):
         for alpha in (1.0, -0.7):
             old = ops.set_tc_bulk_add(bulk)
-            before = ops.variant_counts()["tc_bulk_add"]
-            full = torch.full((M, ldc), 7.0, device=DEV)
-            ops.gemm_tc(x, w, full[:, :N], bn=bn, alpha=alpha)
-            ops.set_tc_bulk_add(old)
-            took.append(ops.variant_counts()["tc_bulk_add"] > before)
+            try:
+                before = ops.variant_counts()["tc_bulk_add"]
+                full = torch.full((M, ldc), 7.0, device=DEV)
+                ops.gemm_tc(x, w, full[:, :N], bn=bn, alpha=alpha)
+                took.append(ops.variant_counts()["tc_bulk_add"] > before)
+            finally:
+                ops.set_tc_bulk_add(old)
             close(full[:, :N], alpha * want, 1e-5)
             assert bool((full[:, N:] == 7.0).all())
             got.append(full)
     assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[3])
-    assert not any(took[:2]) and (all(took[2:]) or bn in (64, 128, 192))
+    assert took == [False, False, taken, taken]
 
 
 @pytest.mark.parametrize("pairing", [0, 1])
 @pytest.mark.parametrize("nh,nkv,hd,K", [(9, 3, 64, 72), (2, 1, 128, 96), (15, 5, 64, 136), (6, 1, 128, 64)])
 def test_qkv_rope_with_two_ctas_on_a_tile(ops, pairing, nh, nkv, hd, K):  # noqa: F811
-    """Against the separate kernels: rows of several sequences in a tile, a chunk at a cached position,
+    """Against the body with one CTA on a tile, which sums in the same order and rounds at the same places,
+    and its queries against float64: rows of several sequences in a tile, a chunk at a cached position,
     the last tile's heads beyond the matrix, one step that may not write the cache."""
     P, lens, news = 512, [200, 70, 333], [200, 70, 150]
     j = torch.arange(hd // 2, dtype=torch.float64)
@@ -96,20 +102,28 @@ def test_qkv_rope_with_two_ctas_on_a_tile(ops, pairing, nh, nkv, hd, K):  # noqa
         cache = ToyCache(lens, nkv, hd, torch.bfloat16, seed=3)
         q = torch.zeros(T, nh * hd, device=DEV, dtype=torch.bfloat16)
         old = ops.set_tc_pair(pair)
-        before = ops.variant_counts()["tc_pair"]
-        ops.gemm_tc_qkv_rope(x, w, q, cos, sin, pairing, nh, nkv, hd, pos_t, seq_t, cache.seq_slot,
-                             cache.table, cache.k, cache.v, 64, True)
-        assert (ops.variant_counts()["tc_pair"] > before) == bool(pair)
-        kept = cache.k.clone(), cache.v.clone()
-        ops.gemm_tc_qkv_rope(x + 1, w, q.clone(), cos, sin, pairing, nh, nkv, hd, pos_t, seq_t,
-                             cache.seq_slot, cache.table, cache.k, cache.v, 64, False)
-        ops.set_tc_pair(old)
+        try:
+            before = ops.variant_counts()["tc_pair"]
+            ops.gemm_tc_qkv_rope(x, w, q, cos, sin, pairing, nh, nkv, hd, pos_t, seq_t, cache.seq_slot,
+                                 cache.table, cache.k, cache.v, 64, True)
+            assert (ops.variant_counts()["tc_pair"] > before) == bool(pair)
+            kept = cache.k.clone(), cache.v.clone()
+            ops.gemm_tc_qkv_rope(x + 1, w, q.clone(), cos, sin, pairing, nh, nkv, hd, pos_t, seq_t,
+                                 cache.seq_slot, cache.table, cache.k, cache.v, 64, False)
+        finally:
+            ops.set_tc_pair(old)
         assert torch.equal(kept[0], cache.k) and torch.equal(kept[1], cache.v)
         got.append((q, *kept))
     assert fault.item() == 0
-    # the same products in the same order of sums, rounded at the same places
     for a, b in zip(*got):
-        close(b, a, 1e-2)
+        assert torch.equal(b, a)
+    # rounded before and behind the rotation: 2^-9 of each of the two channels and of the result
+    u = (x.double() @ w.double().T)[:, :nh * hd].view(T, nh, hd).cpu()
+    c, s = torch.cos(ang)[qpos][:, None], torch.sin(ang)[qpos][:, None]
+    even, odd = (slice(0, hd, 2), slice(1, hd, 2)) if pairing else (slice(0, hd // 2), slice(hd // 2, hd))
+    turned = torch.empty_like(u)
+    turned[..., even], turned[..., odd] = u[..., even] * c - u[..., odd] * s, u[..., odd] * c + u[..., even] * s
+    close(got[1][0], turned.view(T, nh * hd), 3 * 2.0 ** -9)
 
 
 def test_the_ring_beside_another_streams_loads(ops):  # noqa: F811
