@@ -83,15 +83,20 @@ static int launch_fused(const FusedParams& p, int tiles, cudaStream_t st, int gr
   return launch_status();
 }
 
-// The register variant for any number of rows up to kFuMaxRows; held (see registers_hold): a body of
-// more than three chunks, whatever the width, as only those start the kernel behind late.
+// The register variant for any number of rows up to kFuMaxRows; held (see registers_hold): a body that
+// holds every chunk.  The kernel behind a held product starts in front of its wait, but for one token and
+// more than 1,024 columns of the six-chunk body, where its early start gets in the way (decode steps of one
+// sequence, us, early and late: 135M's down product, K = 1,536, 421 and 399; 360M, K = 960, 548 and 564 to
+// 604; 1.7B, K = 2,048, 938 and 978).
 template <int PRO, int EPI>
 static int dispatch_registers(const FusedParams& p, int tiles, cudaStream_t st, bool held = false) {
   if (held) {
     count_variant(kVarFusedHeld);
     if (p.K > 1536) return launch_fused<1, PRO, EPI, 8>(p, tiles, st);
-    return p.M <= 8 ? launch_fused<1, PRO, EPI, 6>(p, tiles, st)
-                    : launch_fused<2, PRO, EPI, 6>(p, tiles, st);
+    FusedParams q = p;
+    q.late = p.M == 1 && p.K > 1024;
+    return p.M <= 8 ? launch_fused<1, PRO, EPI, 6>(q, tiles, st)
+                    : launch_fused<2, PRO, EPI, 6>(q, tiles, st);
   }
   if (p.M <= 8) return launch_fused<1, PRO, EPI>(p, tiles, st);
   if (p.M <= 16) return launch_fused<2, PRO, EPI>(p, tiles, st);
@@ -182,21 +187,22 @@ static int launch_stream(const FusedParams& whole, int tiles, cudaStream_t st) {
   return e == cudaSuccess ? launch_status() : (int)e;
 }
 
-// Matrices beyond kStreamMinK columns of which every CTA holds its whole tile in registers before the
+// Matrices from kStreamMinK columns on of which every CTA holds its whole tile in registers before the
 // wait: what is left behind it is x, the product and its reduction, without the ring's barriers and
 // without x behind the weights in the copy unit's queue.  One wave of tiles (a second tile's weights
-// come in one by one), and few rows: 135M's down product, microseconds a decode step streamed and held:
-// 432 and 401 alone, 610 and 566 at 16 rows, but 760 and 839 at 32; 360M (K = 960, with its norm)
-// 619 and 548 alone, 683 and 654 at 8 rows, 906 and 852 at 16, but 548 and 596 alone with its
-// gate|up's 320 tiles.  Beyond 5 MB the plain epilogue only pays for one or two rows (1.7B's o product,
-// 8.4 MB: 950 and 922 alone, but 1,016 and 1,049 at 3 rows and 1,202 and 1,252 at 8: the next product's
-// ring starts filling under it, in front of its x), the gated one always (a shared expert beside the
-// routed ones, whose CTAs a ring of 200 KB keeps off the SM: Pudorax m at 8 rows 1,348 and 1,250).
+// come in one by one), and few rows.  Microseconds a decode step, everything streamed and with this rule:
+// 135M (down product) 446 and 399 alone, 418 and 398 at 2 rows, 427 and 404 at 4, 455 and 429 at 8 (527
+// and 508 at contexts of 2,048), 562 and 536 at 9, 604 and 570 at 16, but 760 and 839 at 32; 360M (q|k|v, o)
+// 604 and 548 alone, 604 and 576 at 2, 630 and 606 at 4, 670 and 647 at 8, 917 and 871 at 16, but 548 and
+// 596 alone with its gate|up's 320 tiles.  Beyond 5 MB the plain epilogue only pays for one row (1.7B's o
+// product, 8.4 MB: 958 and 939 alone, 959 and 992 at 2 rows, 1,016 and 1,049 at 3: the next product's ring
+// starts filling under it, in front of its x), the gated one always (a shared expert beside the routed
+// ones, whose CTAs a ring of 200 KB keeps off the SM: Pudorax m at 8 rows 1,375 and 1,289).
 template <int PRO, int EPI>
 static bool registers_hold(const FusedParams& p, int tiles, long long w_bytes) {
   if (g_stream_min_k != kStreamMinK || p.M > 16 || p.K > (p.M <= 8 ? 2048 : 1536) || tiles > 2 * kSmCount)
     return false;
-  const bool large = p.M <= 2 || (PRO == kProPlain && EPI == kEpiSilu);
+  const bool large = p.M == 1 || (PRO == kProPlain && EPI == kEpiSilu);
   return w_bytes <= (large ? 9LL << 20 : 5LL << 20);
 }
 

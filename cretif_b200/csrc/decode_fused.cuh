@@ -103,6 +103,7 @@ struct FusedParams {
   // set by the launcher from the above
   FastDiv gu_div, tph_div;  // by gu_block; by tiles per head (hd / 16)
   int bt_shift;             // log2 of bt (a power of two)
+  int late;                 // held bodies: the kernel behind starts after the wait (set by the launcher)
 };
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
@@ -606,14 +607,10 @@ __device__ __forceinline__ void skinny_fused_tiles(const FusedParams& p, int n_t
     epi_prefetch<NT, EPI>(p, tile, ahead);
     have_ahead = true;
   }
-  // Held tiles (PRE > 3) let the kernel behind start only after the wait: with the trigger in front of it,
-  // kernels two and three launches on began while the ones before this one still ran, and a Rigozen m
-  // step's logits were 0.005 to 0.02 off the ordered ones (error against 64 bits 0.0122 -> 0.0146).
-  // What ran ahead has not been found; behind the wait all its logits are bit for bit those of the ring.
   if (pdl) {
-    if (PRE <= 3) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (PRE <= 3 || !p.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (PRE > 3) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (PRE > 3 && p.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
   if (pro_is_norm(PRO)) {
