@@ -352,8 +352,8 @@ inline size_t ssm_carry_smem(int n, int ec, int nbuf) {
 // The pieces tid, tid + kScThreads, ... of a [rows][n4] block without a division a piece.
 struct SsmWalk {
   int row, col, n4, dr, dc;
-  __device__ SsmWalk(int tid, int n4_, int threads = kScThreads)
-      : row(tid / n4_), col(tid % n4_), n4(n4_), dr(threads / n4_), dc(threads % n4_) {}
+  __device__ SsmWalk(int tid, int n4_)
+      : row(tid / n4_), col(tid % n4_), n4(n4_), dr(kScThreads / n4_), dc(kScThreads % n4_) {}
   __device__ void next() {
     row += dr;
     col += dc;
@@ -522,13 +522,13 @@ ssm_intra_kernel(const SsmArgs a, int heads) {
 
 // Two buffers for C, B and x where they fit (nbuf = 2): a chunk's copies are under way while the chunk
 // before is computed.
-template <int EC, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+template <int EC>
+__global__ void __launch_bounds__(kScThreads)
 ssm_carry_kernel(const SsmArgs a, int nbuf) {
   extern __shared__ __align__(16) float smem[];
   constexpr int C = kScTokens;
   constexpr int CG = EC / 4;               // groups of four columns
-  constexpr int NR = THREADS / CG;      // threads along the rows
+  constexpr int NR = kScThreads / CG;      // threads along the rows
   constexpr int RT = C / NR;               // read-out rows a thread
   const int tid = threadIdx.x, H = a.H, N = a.N, e = a.e;
   // the grid: heads, slices of columns, sequences (the slowest)
@@ -547,7 +547,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
   const int grp = h / (H / a.G);
   const int cb = a.inner() + grp * N, cc = cb + a.G * N, cx = h * e + col0;
   float* M = a.S(b, h) + col0;
-  for (int idx = tid; idx < N * CG; idx += THREADS) {
+  for (int idx = tid; idx < N * CG; idx += kScThreads) {
     const int i = idx / CG, jg = idx - i * CG;
     *reinterpret_cast<float4*>(sS + i * EC + 4 * jg) =
         *reinterpret_cast<const float4*>(M + (size_t)i * e + 4 * jg);
@@ -561,7 +561,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
   auto stage = [&](int c0, int which) {
     const int nt = min(C, t1 - c0);
     float* buf = bufs + which * buf_floats;
-    for (SsmWalk w(tid, n4, THREADS); w.row < nt; w.next()) {
+    for (SsmWalk w(tid, n4); w.row < nt; w.next()) {
       const float* row = a.xbc + (size_t)(c0 + w.row) * a.ldx + 4 * w.col;
       float* to = buf + w.row * ldq + 4 * w.col;
       ssm_cp16(to, row + cc);
@@ -571,7 +571,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
       ssm_cp_one(sums + which * C + tid, F + c0 + tid);
       ssm_cp_one(steps + which * C + tid, dts + c0 + tid);
     }
-    for (int idx = tid; idx < nt * CG; idx += THREADS) {
+    for (int idx = tid; idx < nt * CG; idx += kScThreads) {
       const int tt = idx / CG, jg = idx - tt * CG;
       ssm_cp16(buf + 2 * C * ldq + tt * EC + 4 * jg,
                a.xbc + (size_t)(c0 + tt) * a.ldx + cx + 4 * jg);
@@ -632,7 +632,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
     }
     if (last && !a.write_state) break;     // nobody reads the state after the last chunk
     // x takes the weight it has in the state's update (the read-out does not use x)
-    for (int idx = tid; idx < nt * CG; idx += THREADS) {
+    for (int idx = tid; idx < nt * CG; idx += kScThreads) {
       const int tt = idx / CG, jg = idx - tt * CG;
       float4 v4 = *reinterpret_cast<float4*>(sX + tt * EC + 4 * jg);
       scale4(v4, expf((float)(Fn - sF[tt])) * sD[tt]);
@@ -688,7 +688,7 @@ ssm_carry_kernel(const SsmArgs a, int nbuf) {
   }
   if (a.write_state) {
     __syncthreads();
-    for (int idx = tid; idx < N * CG; idx += THREADS) {
+    for (int idx = tid; idx < N * CG; idx += kScThreads) {
       const int i = idx / CG, jg = idx - i * CG;
       *reinterpret_cast<float4*>(M + (size_t)i * e + 4 * jg) =
           *reinterpret_cast<const float4*>(sS + i * EC + 4 * jg);
@@ -700,11 +700,7 @@ template <int EC>
 int launch_ssm_carry(const SsmArgs& a, cudaStream_t st) {
   const int nbuf = ssm_carry_smem(a.N, EC, 2) <= 220 * 1024 ? 2 : 1;
   const size_t smem = ssm_carry_smem(a.N, EC, nbuf);
-  // 64 columns a CTA: one CTA fits an SM, and the products of a chunk wait on shared memory, which 16 warps
-  // hide better than 8 (prompts, with 256 and 512 threads, microseconds: Pudorax s, four of 200 to 700 tokens,
-  // 2,378 and 2,232; m, two, 5,171 and 5,018; eight 8,232 and 8,096, with the experts' order beside it).
-  constexpr int kThreads = EC == 64 ? 512 : kScThreads;
-  auto kern = ssm_carry_kernel<EC, kThreads>;
+  auto kern = ssm_carry_kernel<EC>;
   if (smem > 48 * 1024) {
     cudaError_t err =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -712,7 +708,7 @@ int launch_ssm_carry(const SsmArgs& a, cudaStream_t st) {
   }
   const long long ctas = (long long)a.B * a.H * (a.e / EC);
   if (ctas > 0x7fffffffLL) return kBadArgument;
-  kern<<<(unsigned)ctas, kThreads, smem, st>>>(a, nbuf);
+  kern<<<(unsigned)ctas, kScThreads, smem, st>>>(a, nbuf);
   return launch_status();
 }
 
