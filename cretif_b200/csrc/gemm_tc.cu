@@ -640,7 +640,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // bytes a cycle per SM.  The loads of both CTAs are counted on CTA 0's barriers; its commits
 // arrive on the barriers of both.  Epilogues: the float32 add and the SiLU store through
 // shared-memory slabs and TMA, as above, and the rotary one, whose warps turn a head's columns into
-// whole lines in 4 KB of shared memory each.
+// whole lines in 4 KB of shared memory each (it spills: 168 registers, 92 bytes stored, for the angles that it
+// holds through the wait for the product).
 constexpr int kTpThreads = 320;         // producer, issuer, eight epilogue warps
 template <int kTpBN>                    // the tile's width: 256, or 192 for widths like 576 and 960
 struct TpSmem {
@@ -1463,7 +1464,12 @@ extern "C" int cretif_gemm_tc_qkv_rope(const void* A, const void* Wqkv, void* Q,
   // and after: SmolLM2-1.7B (6,144 x 2,048) 8 x 1,024 26,970 -> 25,410, one of 1,024 4,980 -> 4,760;
   // 360M (1,600 x 960) 16 of 256 to 2,048 13,560 -> 12,870, but two of 1,500 4,600 -> 4,640; 135M
   // (960 x 576) 8 x 2,048 7,600 -> 7,670.  So: from one wave of pairs on where pairs pay anyhow, from four on
-  // for the smaller matrices from 1.5 M elements up.
+  // for the smaller matrices from 1.5 M elements up.  The kernel alone between those sizes, us, one CTA and
+  // two at 3,000, 4,096 and 8,192 rows: 1,280 x 768 (1.0 M) 23.4 / 21.4, 28.6 / 29.0, 43.0 / 37.4; 1,152 x 896
+  // 22.5 / 22.5, 26.6 / 28.7, 36.9 / 38.9 (and 73.7 / 54.7 at 16,384); 1,280 x 1,024 26.6 / 22.5, 30.7 / 30.7,
+  // 48.6 / 41.8; 1,600 x 960 28.1 / 30.7, 30.1 / 31.2, 54.2 / 45.5; 2,048 x 1,024 31.1 / 32.2, 37.7 / 32.7,
+  // 63.5 / 49.2; 2,560 x 1,280 39.9 / 33.7, 56.8 / 42.5, 94.7 / 59.4: pairs pay from some 150 of them on from 1 M
+  // elements up, which the rule leaves to the next size.
   if (g_tc_pair != 0 && (g_tc_pair > 0 || (pair_pays(N, K) ? wide_pairs >= 74
                                                            : (long long)N * K >= 1500000 && wide_pairs >= 4 * 74)))
     return launch_tc_pair<256, kTcRope>(A, Wqkv, ep, M, N, K, lda, ldw, fault, st);

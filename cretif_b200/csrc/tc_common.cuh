@@ -41,7 +41,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // that refill it are made by the async proxy; an arrival alone did not hold them back until the loads had
 // finished: a warp whose loads were queued behind another CTA's (64 KB of weights asked for at once) read
 // the next turn's contents.
-// Behind a proxy fence:
+// Behind a proxy fence (the decode attention: 64 sequences of 2,048 tokens, 360M, 2,174 us a step without it,
+// 2,337 with it, 2,368 with the form below; eight sequences the same as before):
 __device__ __forceinline__ void release_stage(uint64_t* empty, int lane) {
   fence_proxy_async();
   __syncwarp();
